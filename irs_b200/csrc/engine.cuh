@@ -612,10 +612,10 @@ class MapMaker {
           launch_f32<VERT, false, false>(grid, sp, lp, pix, pmin, psad, verts);
       }
     } else {
-      if (par)
-        shoot_f64<VERT, true><<<grid, kShootThreads, 0, stream_>>>(sp, lp, tiles_.total, pix, pmin, psad, verts);
-      else
-        shoot_f64<VERT, false><<<grid, kShootThreads, 0, stream_>>>(sp, lp, tiles_.total, pix, pmin, psad, verts);
+      const bool gen = prm.rectangular || !prm.approx;
+      auto kernel = par ? (gen ? shoot_f64<VERT, !VERT, true> : shoot_f64<VERT, !VERT, false>)
+                        : (gen ? shoot_f64<VERT, false, true> : shoot_f64<VERT, false, false>);
+      kernel<<<grid, kShootThreads, 0, stream_>>>(sp, lp, tiles_.total, pix, pmin, psad, verts);
     }
     IRSB_LAUNCH_CK("shoot");
     IRSB_CKR(cudaEventRecord(ev_lat1_, stream_));

@@ -7,10 +7,9 @@
 // evaluation of the leaf's local expansion and alpha_smooth the smooth sheet.
 //
 // Two arithmetic forms:
-//   * shoot_f64 -- the plain uniform FP64 form. Global coordinates and the
-//     reference's operation order for the ray position, the far-field Horner
-//     loop and the source-to-pixel conversion (point_to_pixel,
-//     array_functions.cuh:70-75).
+//   * shoot_f64 -- the plain uniform FP64 form. Global coordinates, the
+//     reference's ray positions and, for rays, its source-to-pixel conversion
+//     (point_to_pixel, array_functions.cuh:70-75).
 //   * shoot_f32 -- the FP32 form. Coordinates are taken relative to the leaf
 //     centre; the near-field sum runs in FP32 with blocked two-sum
 //     compensation (naive partial sums of 16 stars folded into a compensated
@@ -41,7 +40,6 @@
 namespace irsb {
 
 constexpr int kShootThreads = 256;
-constexpr int kRaysPerThread = kTileY / (kShootThreads / kTileX);  // 4
 
 struct ShootParams {
   double kappa, gamma, kstar, theta2, inv_pi;
@@ -207,97 +205,152 @@ __device__ __forceinline__ void irs_deposit(double px, double py, int npx, int n
 }
 
 // ----------------------------------------------------------------- FP64 form
-template <bool VERT, bool PAR>
-__global__ void __launch_bounds__(kShootThreads) shoot_f64(ShootParams sp, LeafPtrs lp, long long total_tiles,
+// 1 / d for a normal d: the hardware's FP64 reciprocal approximation (PTX
+// rcp.approx.ftz.f64, about 2^-20) and one third-order (Halley-type) step
+// r (1 + e + e^2), e = 1 - d r, whose truncation 2^-60 is below the rounding:
+// three FMAs and about an ulp, without the range checks and the slow path of a
+// general division. A zero or subnormal d gives NaN, where 1 / d gives inf;
+// both leave the ray without an image.
+__device__ __forceinline__ double rcp_f64(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// P lattice points per thread at a time (rows ty + r * 8), sharing each staged
+// star and coefficient. Bound by the FP64 pipe (8 operations per star and
+// point, 4 per order) and, before points were taken together, by its latency:
+// one point at a time with general divisions the lattice of 4.1e7 corners
+// (15 near stars, order 11) took 2.60 ms and 1.03e8 rays with parities
+// 6.36 ms (B200); now 0.76 and 2.60 ms. The divisions by the leaf's half length (32
+// columns, 32 rows) are made once per tile.
+//
+// GEN: the smooth sheet is not the circular approximation; its general form
+// then runs in a function of its own, which keeps its registers out of the
+// star loop (inlined for every point the kernel took 196 registers).
+__device__ __noinline__ cplx<double> alpha_smooth_call(cplx<double> z, const ShootParams& sp) {
+  return alpha_smooth_(z, sp.kstar, sp.rect, mk(sp.corner_re, sp.corner_im), sp.approx, sp.taylor_smooth, sp.inv_pi);
+}
+__device__ __noinline__ cplx<double> d_alpha_smooth_dzbar_call(cplx<double> z, const ShootParams& sp) {
+  return d_alpha_smooth_dzbar_(z, sp.kstar, sp.rect, mk(sp.corner_re, sp.corner_im), sp.approx, sp.taylor_smooth,
+                               sp.inv_pi);
+}
+
+template <bool VERT, bool PAR, bool GEN>
+__global__ void __launch_bounds__(kShootThreads, PAR || GEN ? 2 : 3) shoot_f64(ShootParams sp, LeafPtrs lp, long long total_tiles,
                                                            int* __restrict__ pix, int* __restrict__ pmin,
                                                            int* __restrict__ psad, double2* __restrict__ verts) {
+  constexpr int P = 2, RS = kShootThreads / kTileX;
   __shared__ double4 s_near[kMaxStarsDirect];
   __shared__ double2 s_coef[kMaxOrder];
+  __shared__ double s_y[kTileY], s_dzi[kTileY];
   const int tx = threadIdx.x & (kTileX - 1), ty = threadIdx.x / kTileX;
   const cplx<double> corner = mk(sp.corner_re, sp.corner_im);
+  const double scx = sp.npx / (2.0 * sp.hly_re), scy = sp.npy / (2.0 * sp.hly_im);
   for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
     TileInfo ti = tile_info(lp, t);
     const int nn = lp.nnear[ti.leaf];
+    const double lcx = lp.cx[ti.leaf], lcy = lp.cy[ti.leaf], lhl = lp.hl[ti.leaf];
     if (threadIdx.x < kMaxStarsDirect) s_near[threadIdx.x] = lp.near64[(size_t)ti.leaf * kMaxStarsDirect + threadIdx.x];
     if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxOrder)
       s_coef[threadIdx.x - 64] = lp.coef64[(size_t)ti.leaf * kMaxOrder + threadIdx.x - 64];
-    const double lcx = lp.cx[ti.leaf], lcy = lp.cy[ti.leaf], lhl = lp.hl[ti.leaf];
+    if (threadIdx.x >= 128 && threadIdx.x < 128 + kTileY) {
+      const int jj = threadIdx.x - 128;
+      const double y = sp.base_y + 2.0 * (sp.rhs_y * double((long long)ti.j0 + jj));
+      s_y[jj] = y;
+      s_dzi[jj] = (y - lcy) / lhl;
+    }
+    const long long i = ti.i0 + tx;
+    const double x = sp.base_x + 2.0 * (sp.rhs_x * double(i));
+    const double dzr = (x - lcx) / lhl, loc_scale = sp.theta2 / lhl;
     __syncthreads();
     if (tx < ti.ni) {
-      const long long i = ti.i0 + tx;
-      const double x = sp.base_x + 2.0 * (sp.rhs_x * double(i));
-#pragma unroll 1
-      for (int r = 0; r < kRaysPerThread; r++) {
-        int jj = ty + r * (kShootThreads / kTileX);
-        if (jj >= ti.nj) break;
-        const long long j = ti.j0 + jj;
-        const double y = sp.base_y + 2.0 * (sp.rhs_y * double(j));
+      for (int jj0 = ty; jj0 < ti.nj; jj0 += P * RS) {
+        double y[P], dzi[P];
+#pragma unroll
+        for (int q = 0; q < P; q++) {  // a row past the tile's last repeats it and is not written
+          const int jj = min(jj0 + q * RS, ti.nj - 1);
+          y[q] = s_y[jj];
+          dzi[q] = s_dzi[jj];
+        }
         // near field: sum m / (z - z_i)
-        double ar = 0.0, ai = 0.0, dr = 0.0, di = 0.0;
+        double ar[P], ai[P], dr[P], di[P];
+#pragma unroll
+        for (int q = 0; q < P; q++) ar[q] = ai[q] = dr[q] = di[q] = 0.0;
+#pragma unroll 2
         for (int s = 0; s < nn; s++) {
-          double4 st = s_near[s];
-          double ex = x - st.x, ey = y - st.y;
-          double inv = 1.0 / (ex * ex + ey * ey);
-          double q = st.z * inv;
-          ar += q * ex;
-          ai -= q * ey;
-          if (PAR) {  // m / (z - z_i)^2 = m conj(d)^2 / |d|^4
-            double t2 = q * inv;
-            dr += t2 * (ex * ex - ey * ey);
-            di -= t2 * (2.0 * ex * ey);
+          const double4 st = s_near[s];
+          const double ex = x - st.x, ex2 = ex * ex;
+#pragma unroll
+          for (int q = 0; q < P; q++) {
+            const double ey = y[q] - st.y;
+            const double inv = rcp_f64(fma(ey, ey, ex2));
+            const double w = st.z * inv;
+            ar[q] = fma(w, ex, ar[q]);
+            ai[q] = fma(-w, ey, ai[q]);
+            if (PAR) {  // m / (z - z_i)^2 = m conj(d)^2 / |d|^4
+              const double t2 = w * inv;
+              dr[q] = fma(t2, fma(-ey, ey, ex2), dr[q]);
+              di[q] = fma(-t2, 2.0 * ex * ey, di[q]);
+            }
           }
         }
-        cplx<double> a_star = mk(ar * sp.theta2, -(ai * sp.theta2));
         // far field: Horner in dz = (z - c) / hl
-        cplx<double> dz = mk((x - lcx) / lhl, (y - lcy) / lhl);
-        cplx<double> A = mk(0.0, 0.0), Ad = mk(0.0, 0.0);
+        double Ar[P], Ai[P], Dr[P], Di[P];
+#pragma unroll
+        for (int q = 0; q < P; q++) Ar[q] = Ai[q] = Dr[q] = Di[q] = 0.0;
         for (int k = sp.p; k >= 1; k--) {
-          if (PAR && k >= 2) {
-            Ad = cmul(Ad, dz);
-            double2 c = s_coef[k - 1];
-            Ad = cadd(Ad, mk(c.x * (k - 1), c.y * (k - 1)));
+          const double2 c = s_coef[k - 1];
+#pragma unroll
+          for (int q = 0; q < P; q++) {
+            if (PAR && k >= 2) {
+              const double u = fma(Dr[q], dzr, fma(-Di[q], dzi[q], c.x * (k - 1)));
+              Di[q] = fma(Dr[q], dzi[q], fma(Di[q], dzr, c.y * (k - 1)));
+              Dr[q] = u;
+            }
+            const double u = fma(Ar[q], dzr, fma(-Ai[q], dzi[q], c.x));
+            Ai[q] = fma(Ar[q], dzi[q], fma(Ai[q], dzr, c.y));
+            Ar[q] = u;
           }
-          A = cmul(A, dz);
-          double2 c = s_coef[k - 1];
-          A = cadd(A, mk(c.x, c.y));
         }
-        A = cscale(A, sp.theta2);
-        A = cdivr(A, lhl);
-        cplx<double> a_local = cconj(A);
-        cplx<double> z = mk(x, y);
-        cplx<double> a_sm = alpha_smooth_(z, sp.kstar, sp.rect, corner, sp.approx, sp.taylor_smooth, sp.inv_pi);
-        cplx<double> w = cadd(cscale(z, 1.0 - sp.kappa), cscale(cconj(z), sp.gamma));
-        w = csub(csub(csub(w, a_star), a_local), a_sm);
-        if (VERT) {
-          w.re -= sp.cy_re;
-          w.im -= sp.cy_im;
-          double px = (w.re + sp.hly_re) * sp.npx / (2.0 * sp.hly_re);
-          double py = (w.im + sp.hly_im) * sp.npy / (2.0 * sp.hly_im);
-          verts[(size_t)(j - sp.jbase) * (sp.nx) + i] = make_double2(px, double(sp.npy) - py);
-        } else {
-          if (isnan(w.re) || isnan(w.im)) continue;
-          w.re -= sp.cy_re;
-          w.im -= sp.cy_im;
-          if (w.re < -sp.hly_re || w.re > sp.hly_re || w.im < -sp.hly_im || w.im > sp.hly_im) continue;
-          double px = (w.re + sp.hly_re) * sp.npx / (2.0 * sp.hly_re);
-          double py = (w.im + sp.hly_im) * sp.npy / (2.0 * sp.hly_im);
-          bool pmin_ = false;
-          if (PAR) {
-            // mu = 1 / ((dw/dz)^2 - |dw/dzbar|^2)   (irs_functions.cuh:66-81)
-            cplx<double> dstar = mk(-(dr * sp.theta2), (di * sp.theta2));  // -theta^2 conj(sum m/d^2)
-            Ad = cscale(Ad, sp.theta2);
-            Ad = cdivr(Ad, lhl * lhl);
-            cplx<double> dloc = cconj(Ad);
-            double dsz = d_alpha_smooth_dz_(z, sp.kstar, sp.rect, corner, sp.approx);
-            cplx<double> dszb =
-                d_alpha_smooth_dzbar_(z, sp.kstar, sp.rect, corner, sp.approx, sp.taylor_smooth, sp.inv_pi);
-            double dwdz = (1.0 - sp.kappa) - dsz;
-            cplx<double> dwdzb = csub(csub(csub(mk(sp.gamma, 0.0), dstar), dloc), dszb);
-            double a = cabs_(dwdzb);
-            double mu = 1.0 / (dwdz * dwdz - a * a);
-            pmin_ = mu >= 0;
+#pragma unroll
+        for (int q = 0; q < P; q++) {
+          if (jj0 + q * RS >= ti.nj) break;
+          const long long j = (long long)ti.j0 + jj0 + q * RS;
+          const cplx<double> a_star = mk(ar[q] * sp.theta2, -(ai[q] * sp.theta2));
+          const cplx<double> a_local = mk(Ar[q] * loc_scale, -(Ai[q] * loc_scale));
+          const cplx<double> z = mk(x, y[q]);
+          const cplx<double> a_sm = GEN ? alpha_smooth_call(z, sp) : mk(-sp.kstar * z.re, -sp.kstar * z.im);
+          cplx<double> w = cadd(cscale(z, 1.0 - sp.kappa), cscale(cconj(z), sp.gamma));
+          w = csub(csub(csub(w, a_star), a_local), a_sm);
+          if (VERT) {
+            const double px = ((w.re - sp.cy_re) + sp.hly_re) * scx;
+            const double py = ((w.im - sp.cy_im) + sp.hly_im) * scy;
+            verts[(size_t)(j - sp.jbase) * (sp.nx) + i] = make_double2(px, double(sp.npy) - py);
+          } else {
+            if (isnan(w.re) || isnan(w.im)) continue;
+            w.re -= sp.cy_re;
+            w.im -= sp.cy_im;
+            if (w.re < -sp.hly_re || w.re > sp.hly_re || w.im < -sp.hly_im || w.im > sp.hly_im) continue;
+            double px = (w.re + sp.hly_re) * sp.npx / (2.0 * sp.hly_re);
+            double py = (w.im + sp.hly_im) * sp.npy / (2.0 * sp.hly_im);
+            bool pmin_ = false;
+            if (PAR) {
+              // mu = 1 / ((dw/dz)^2 - |dw/dzbar|^2)   (irs_functions.cuh:66-81)
+              const cplx<double> dstar = mk(-(dr[q] * sp.theta2), (di[q] * sp.theta2));  // -theta^2 conj(sum m/d^2)
+              const double s2 = sp.theta2 / (lhl * lhl);
+              const cplx<double> dloc = mk(Dr[q] * s2, -(Di[q] * s2));
+              const double dsz = d_alpha_smooth_dz_(z, sp.kstar, sp.rect, corner, sp.approx);
+              const cplx<double> dszb = GEN ? d_alpha_smooth_dzbar_call(z, sp) : mk(0.0, 0.0);
+              const double dwdz = (1.0 - sp.kappa) - dsz;
+              const cplx<double> dwdzb = csub(csub(csub(mk(sp.gamma, 0.0), dstar), dloc), dszb);
+              const double a = cabs_(dwdzb);
+              const double mu = 1.0 / (dwdz * dwdz - a * a);
+              pmin_ = mu >= 0;
+            }
+            irs_deposit(px, py, sp.npx, sp.npy, pix, pmin, psad, pmin_, PAR);
           }
-          irs_deposit(px, py, sp.npx, sp.npy, pix, pmin, psad, pmin_, PAR);
         }
       }
     }
