@@ -27,7 +27,8 @@
 //     the lens-equation kernels (near64, coef64 = k c_k); a point outside the
 //     root box takes the direct sum over all stars, as get_nearest_node
 //     returns the root there (tree_node.cuh:535-539);
-//   * a final root costs its warp one load and one store.
+//   * one cooperative launch follows all chains, with a grid barrier per update
+//     that also counts the roots still moving: a step ends with its last root.
 #pragma once
 #include "leaves.cuh"
 #include "shoot.cuh"  // LeafPtrs
@@ -148,7 +149,7 @@ __device__ __forceinline__ cplx<double> recip(cplx<double> d) {
 // sum over k = lane, lane + 32, ... < n, k != skip, of 1 / (z - p[k]): four
 // independent accumulators (four reciprocals in flight per lane), added in a
 // fixed order.
-__device__ __forceinline__ cplx<double> lane_recip_sum(const double2* __restrict__ p, int n, cplx<double> z,
+__device__ __forceinline__ cplx<double> lane_recip_sum(const double2* p, int n, cplx<double> z,
                                                        int skip, int lane) {
   cplx<double> acc[4];
 #pragma unroll
@@ -218,70 +219,125 @@ __device__ __forceinline__ CcfField ccf_field_warp(const CcfParams& P, const Lea
   return f;
 }
 
-// One Jacobi step for chains [0, nchains): chain ch is branch ch / sides,
-// side (ch % sides) (0: phi decreasing, 1: increasing; sides = 1 at j = 0,
-// where both sides start from the branch centre). Positions are read from
-// `src` (rows of the root array, or the chain's scratch row) and written to
-// `dst`; fin[ch][a] marks final roots, which are copied. One warp per root:
-// the lanes split the sums over all stars (their positions `spos`, in tree
-// order) and over the chain's other roots (strided, so a warp reads 32
-// consecutive positions at a time; both arrays stay in L1) and reduce them in
-// a fixed order.
+// cos and sin of phi at every step of every chain, entry (ch, j) at
+// [ch * (half + 1) + j]: the phases of the root finding, evaluated once.
+__global__ void ccf_phases(CcfParams P, double2* __restrict__ cs) {
+  const int half = P.nphi / (2 * P.nbranches), n = 2 * P.nbranches * (half + 1);
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int ch = q / (half + 1), j = q - ch * (half + 1);
+    const double phi = ccf_phi(P, ch / 2, ch % 2 == 0 ? -j : j);
+    cs[q] = make_double2(cos(phi), sin(phi));
+  }
+}
+
+// The Jacobi update of one root by one warp: z <- z - f0 / (f1 + f0 (...)) with
+// the chain's roots `src` (root a is z itself), phase cs = (cos, sin) phi. The
+// lanes split the sums over all stars (their positions `spos`, in tree order)
+// and over the chain's other roots (strided, so a warp reads 32 consecutive
+// positions at a time; both arrays stay in L1) and reduce them in a fixed
+// order. Returns whether the root is final; zn (lane 0) is its new position.
 template <typename T>
-__global__ void __launch_bounds__(kCcfThreads) ccf_iterate(CcfParams P, LeafPtrs lp, DescentPtrs<T> dp,
-                                                           const StarRec<T>* __restrict__ stars,
-                                                           const double2* __restrict__ spos, int j, int sides,
-                                                           int from_scratch, double2* __restrict__ roots,
-                                                           double2* __restrict__ scratch,
-                                                           unsigned char* __restrict__ fin) {
-  const int lane = threadIdx.x & 31;
-  const int ch = blockIdx.y;
-  const int c = ch / sides, side = ch % sides;
-  const int sj = side == 0 ? -j : j;
-  const int a = blockIdx.x * (kCcfThreads / 32) + (threadIdx.x >> 5);  // root of this warp
-  if (a >= P.nroots) return;                                           // whole warps only
-  const double2* src = from_scratch ? scratch + (size_t)ch * P.nroots : roots + (size_t)ccf_row(P, c, sj) * P.nroots;
-  double2* dst = from_scratch ? roots + (size_t)ccf_row(P, c, sj) * P.nroots : scratch + (size_t)ch * P.nroots;
-  unsigned char* fn = fin + (size_t)ch * P.nroots;
+__device__ __forceinline__ bool ccf_update(const CcfParams& P, const LeafPtrs& lp, const DescentPtrs<T>& dp,
+                                           const StarRec<T>* __restrict__ stars, const double2* __restrict__ spos,
+                                           const double2* src, int a, double2 cs, int lane, double2& out) {
   const double2 z2 = src[a];
   const cplx<double> z = mk(z2.x, z2.y);
-  if (fn[a]) {
-    if (lane == 0) dst[a] = z2;
-    return;
-  }
+  out = z2;
   const CcfField f = ccf_field_warp(P, lp, dp, stars, z, lane);
   const CcfDerivs d = ccf_derivs(P, f, z);
-  const cplx<double> f0 = ccf_f0(d, ccf_phi(P, c, sj));
-  if (ccf_inv_mu_bound(cabs_(f0), d.dwdz) < 1e-9) {  // already a root to the precision sought: final
-    __syncwarp();
-    if (lane == 0) {
-      fn[a] = 1;
-      dst[a] = z2;
-    }
-    return;
-  }
+  const cplx<double> f0 = csub(cconj(d.dwdzb), mk(d.dwdz * cs.x, -d.dwdz * cs.y));  // ccf_f0
+  if (ccf_inv_mu_bound(cabs_(f0), d.dwdz) < 1e-9) return true;  // already a root to the precision sought
   const cplx<double> f1 = cconj(d.d2wdzb2);  // d f0 / dz
   cplx<double> ps = warp_sum(lane_recip_sum(spos, P.nstars, z, -1, lane));
   cplx<double> rs = warp_sum(lane_recip_sum(src, P.nroots, z, a, lane));
-  if (lane != 0) return;
   if (!P.rect && !P.approx) ps = cadd(ps, recip(z));
   ps = cscale(ps, 2.0);
   const cplx<double> den = cadd(f1, cmul(f0, csub(ps, rs)));
   const cplx<double> zn = csub(z, cdiv(f0, den));
-  if (cabs_(csub(zn, z)) / sqrt(P.theta2) < 1e-9) fn[a] = 1;
-  dst[a] = make_double2(zn.re, zn.im);
+  out = make_double2(zn.re, zn.im);
+  return cabs_(csub(zn, z)) / sqrt(P.theta2) < 1e-9;
 }
 
-// Step j of every chain starts from step j - 1 (ccf_functions.cuh:268-301);
-// the final flags are reset.
-__global__ void ccf_prepare(CcfParams P, int j, double2* __restrict__ roots, unsigned char* __restrict__ fin) {
-  const int nch = 2 * P.nbranches;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (long long)nch * P.nroots;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int ch = int(q / P.nroots), a = int(q - (long long)ch * P.nroots);
-    const int c = ch / 2, sgn = (ch % 2) ? 1 : -1;
-    roots[(size_t)ccf_row(P, c, sgn * j) * P.nroots + a] = roots[(size_t)ccf_row(P, c, sgn * (j - 1)) * P.nroots + a];
-    fin[q] = 0;
+// Reads of a barrier word (about a microsecond each) after which a CTA gives
+// up: seconds, and far more than the other CTAs' share of one update takes.
+__host__ __device__ __forceinline__ long long ccf_spins(const CcfParams& P) {
+  return (1LL << 24) + (long long)(2.0 * P.nbranches * P.nroots * (double(P.nstars) + P.nroots) * 1e-4);
+}
+
+// All roots of all chains from the branch centres to the last phi step: up to
+// it0 updates at the centres, then per step j up to it1 updates starting from
+// step j - 1 (ccf_functions.cuh:268-301), both sides of every branch at once
+// (chain ch is side ch % 2 of branch ch / 2, 0: phi decreasing; at the
+// centres, where both sides start, chain c is branch c). One cooperative
+// launch, one warp per (chain, root), a grid barrier per update; the updates
+// alternate between the buffers s0 and s1 ([chain][root]), and a root reaches
+// its row of `roots` when the next step starts from it. A step ends as soon as
+// the barrier reports that no root is left to move: a final root is never
+// moved again, so the updates left out change nothing.
+//
+// Bound by latency: a chain of dependent updates, each a tree descent, a Horner
+// evaluation and two sums, with 2 chains x 274 roots for the default field;
+// from 1000 stars on by the FP64 reciprocals (2 N^2 per update and chain).
+// As ~1000 graph-captured launches, most of which found every root final, the
+// root finding of 137 / 1000 stars took 4.6 / 13.0 ms (B200) besides 3 - 5 ms
+// to capture and instantiate the graphs; now 2.5 / 12.4 ms.
+template <typename T>
+__global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs lp, DescentPtrs<T> dp,
+                                                          const StarRec<T>* __restrict__ stars,
+                                                          const double2* __restrict__ spos,
+                                                          const double2* __restrict__ cs, int it0, int it1,
+                                                          double2* roots, double2* s0, double2* s1,
+                                                          unsigned char* fin, unsigned long long* words, int* err,
+                                                          int centres, double2** last) {
+  const int lane = threadIdx.x & 31;
+  const int nwarps = gridDim.x * (kCcfThreads / 32);
+  const int warp = blockIdx.x * (kCcfThreads / 32) + (threadIdx.x >> 5);
+  const int half = P.nphi / (2 * P.nbranches);
+  double2* cur = centres ? s0 : *last;
+  double2* nxt = cur == s0 ? s1 : s0;
+  if (!cur) return;  // the centres were given up
+  unsigned long long* word = words;
+  const long long spins = ccf_spins(P);
+  for (int j = centres ? 0 : 1; j <= (centres ? 0 : half); j++) {
+    const int sides = j == 0 ? 1 : 2, nitems = sides * P.nbranches * P.nroots, iters = j == 0 ? it0 : it1;
+    for (int i = 0; i < iters; i++) {
+      int left = 0;  // roots of this warp that are not final yet
+      for (int q = warp; q < nitems; q += nwarps) {
+        const int ch = q / P.nroots, a = q - ch * P.nroots, c = ch / sides;
+        const unsigned char state = i == 0 ? 0 : fin[q];  // 1: became final in the last update, 2: in both buffers
+        if (state == 2) continue;
+        const double2* src = cur + (size_t)(i == 0 && j == 1 ? c : ch) * P.nroots;
+        double2 z = src[a];
+        // the step's start is the result of the step before it
+        if (i == 0 && j > 0 && lane == 0) {
+          const int sj = ch % 2 == 0 ? -(j - 1) : j - 1;
+          roots[(size_t)ccf_row(P, c, sj) * P.nroots + a] = z;
+        }
+        bool done = true;
+        if (state == 0)
+          done = ccf_update<T>(P, lp, dp, stars, spos, src, a, cs[(j == 0 ? 2 * c : ch) * (half + 1) + j], lane, z);
+        done = __shfl_sync(0xffffffffu, int(done), 0) != 0;
+        if (lane == 0) {
+          nxt[(size_t)ch * P.nroots + a] = z;
+          fin[q] = state == 1 ? 2 : (done ? 1 : 0);
+        }
+        left += done ? 0 : 1;
+      }
+      const int moving = grid_barrier_sum(word++, left, err, spins);
+      if (moving < 0) return;
+      double2* t = cur;
+      cur = nxt;
+      nxt = t;
+      if (moving == 0) break;
+    }
+  }
+  if (centres) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *last = cur;
+    return;
+  }
+  for (int q = warp * 32 + lane; q < 2 * P.nbranches * P.nroots; q += nwarps * 32) {  // the last step
+    const int ch = q / P.nroots, a = q - ch * P.nroots;
+    roots[(size_t)ccf_row(P, ch / 2, ch % 2 == 0 ? -half : half) * P.nroots + a] = cur[q];
   }
 }
 

@@ -8,7 +8,6 @@
 #include "stars.cuh"
 
 #include <chrono>
-#include <functional>
 #include <fstream>
 #include <iostream>
 
@@ -183,10 +182,9 @@ class CCF {
     // ---- initial roots at each branch centre: star +/- 1, the rest on the
     // circle of radius |corner| (include/ccf.cuh:706-726)
     const int rows = num_phi + num_branches;
-    std::vector<double2> init((size_t)rows * num_roots, make_double2(0, 0));
-    const CcfParams P = params();
+    std::vector<double2> init((size_t)num_branches * num_roots);
     for (int c = 0; c < num_branches; c++) {
-      double2* r = init.data() + (size_t)ccf_row(P, c, 0) * num_roots;
+      double2* r = init.data() + (size_t)c * num_roots;
       for (int i = 0; i < n; i++) {
         r[i] = make_double2(double(field[i].x) + 1.0, double(field[i].y));
         r[i + n] = make_double2(double(field[i].x) - 1.0, double(field[i].y));
@@ -225,61 +223,53 @@ class CCF {
     // ---- roots
     const CcfParams Q = params();
     const int nch = 2 * num_branches;
-    if (!d_roots_.alloc_exact(init.size()) || !d_scratch_.alloc_exact((size_t)nch * num_roots) ||
-        !d_fin_.alloc_exact((size_t)nch * num_roots) || !d_stat_.alloc_exact(2))
+    const int it0 = num_iters_init + (num_iters_init & 1), it1 = num_iters_step + (num_iters_step & 1);
+    const int half = num_phi / (2 * num_branches);
+    const size_t nwords = size_t(it0) + size_t(half) * it1;  // a grid barrier per update
+    if (!d_roots_.alloc_exact((size_t)rows * num_roots) || !d_scratch_.alloc_exact(2 * (size_t)nch * num_roots) ||
+        !d_fin_.alloc_exact((size_t)nch * num_roots) || !d_stat_.alloc_exact(2) || !d_words_.alloc_exact(nwords + 2) ||
+        !d_phase_.alloc_exact((size_t)nch * (half + 1)))
       return false;
-    IRSB_CKR(cudaMemcpyAsync(d_roots_.p, init.data(), init.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
-    IRSB_CKR(cudaMemsetAsync(d_fin_.p, 0, (size_t)nch * num_roots, s));
+    double2 *b0 = d_scratch_.p, *b1 = d_scratch_.p + (size_t)nch * num_roots;
+    unsigned long long* words = d_words_.p;  // then an error flag and the buffer that holds the centres
+    int* err = reinterpret_cast<int*>(words + nwords);
+    double2** last = reinterpret_cast<double2**>(words + nwords + 1);
+    IRSB_CKR(cudaMemcpyAsync(b0, init.data(), init.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
+    IRSB_CKR(cudaMemsetAsync(words, 0, (nwords + 2) * sizeof(unsigned long long), s));
     const LeafPtrs lp = leaf_ptrs();
     const DescentPtrs<T> dp{tree_.cx.p, tree_.cy.p, tree_.child0.p, leaves_.pos.p, nullptr};
-    const int rpb = kCcfThreads / 32;  // roots per CTA (a warp each)
-    const dim3 g0(ceil_div(num_roots, rpb), num_branches), g1(ceil_div(num_roots, rpb), nch);
-    const int it0 = num_iters_init + (num_iters_init & 1), it1 = num_iters_step + (num_iters_step & 1);
-    // The root finding is ~1000 short launches: each part is captured as a
-    // CUDA graph and replayed, so the launches cost no host round trips.
-    const int half = num_phi / (2 * num_branches);
-    const int gp = std::max(1, std::min(ceil_div(nch * num_roots, 256), 148 * 8));
-    cudaGraphExec_t centres = nullptr, steps = nullptr;
-    auto capture = [&](cudaGraphExec_t& exec, const std::function<void()>& launches) -> bool {
-      cudaGraph_t g = nullptr;
-      IRSB_CKR(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      launches();
-      const cudaError_t le = cudaGetLastError();
-      const cudaError_t ce = cudaStreamEndCapture(s, &g);
-      if (le != cudaSuccess || ce != cudaSuccess) {
-        std::cerr << "Error. Capturing the root finding failed: " << cudaGetErrorString(le != cudaSuccess ? le : ce)
-                  << "\n";
-        if (g) cudaGraphDestroy(g);
+    ccf_phases<<<std::max(1, std::min(ceil_div((long long)nch * (half + 1), 64), 148)), 64, 0, s>>>(Q, d_phase_.p);
+    IRSB_LAUNCH_CK("ccf_phases");
+    // a warp per root, as many CTAs as can be resident together (the grid
+    // waits for one another at every update)
+    auto follow = [&](int centres, int chains, unsigned long long* w) -> bool {
+      int grid = 0;
+      if (!cooperative_grid(ccf_follow<T>, kCcfThreads, ceil_div((long long)chains * num_roots, kCcfThreads / 32), &grid))
         return false;
-      }
-      const cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
-      cudaGraphDestroy(g);
-      return IRSB_CK(ie);
+      CcfParams q = Q;
+      LeafPtrs l = lp;
+      DescentPtrs<T> d = dp;
+      const StarRec<T>* st = d_stars_.p;
+      const double2 *sp = d_spos_.p, *ph = d_phase_.p;
+      int i0 = it0, i1 = it1;
+      double2 *ro = d_roots_.p, *s0 = b0, *s1 = b1;
+      unsigned char* fi = d_fin_.p;
+      void* args[] = {&q, &l, &d, &st, &sp, &ph, &i0, &i1, &ro, &s0, &s1, &fi, &w, &err, &centres, &last};
+      return IRSB_CK(cudaLaunchCooperativeKernel((const void*)ccf_follow<T>, dim3(grid), dim3(kCcfThreads), args, 0, s));
     };
-    const bool ok_graphs =
-        capture(centres,
-                [&] {
-                  for (int i = 0; i < it0; i++)  // branch centres (include/ccf.cuh:906-977)
-                    ccf_iterate<T><<<g0, kCcfThreads, 0, s>>>(Q, lp, dp, d_stars_.p, d_spos_.p, 0, 1, i & 1,
-                                                              d_roots_.p, d_scratch_.p, d_fin_.p);
-                }) &&
-        capture(steps, [&] {
-          for (int j = 1; j <= half; j++) {  // steps away from the centres (include/ccf.cuh:979-1037)
-            ccf_prepare<<<gp, 256, 0, s>>>(Q, j, d_roots_.p, d_fin_.p);
-            for (int i = 0; i < it1; i++)
-              ccf_iterate<T><<<g1, kCcfThreads, 0, s>>>(Q, lp, dp, d_stars_.p, d_spos_.p, j, 2, i & 1, d_roots_.p,
-                                                        d_scratch_.p, d_fin_.p);
-          }
-        });
-    bool ok_run = ok_graphs;
-    if (ok_run) {
-      ok_run = IRSB_CK(cudaEventRecord(e0_, s)) && IRSB_CK(cudaGraphLaunch(centres, s)) &&
-               IRSB_CK(cudaEventRecord(e1_, s)) && IRSB_CK(cudaGraphLaunch(steps, s)) &&
-               IRSB_CK(cudaEventRecord(e2_, s)) && IRSB_CK(cudaStreamSynchronize(s));
+    // branch centres (include/ccf.cuh:906-977), then the steps away from them (:979-1037)
+    IRSB_CKR(cudaEventRecord(e0_, s));
+    if (!follow(1, num_branches, words)) return false;
+    IRSB_CKR(cudaEventRecord(e1_, s));
+    if (!follow(0, nch, words + it0)) return false;
+    IRSB_CKR(cudaEventRecord(e2_, s));
+    int gave_up = 0;
+    IRSB_CKR(cudaMemcpyAsync(&gave_up, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    IRSB_CKR(cudaStreamSynchronize(s));
+    if (gave_up) {
+      std::cerr << "Error. The root finding did not finish.\n";
+      return false;
     }
-    if (centres) cudaGraphExecDestroy(centres);
-    if (steps) cudaGraphExecDestroy(steps);
-    if (!ok_run) return false;
     // ---- error bound in 1/mu over every root (include/ccf.cuh:1044-1069)
     IRSB_CKR(cudaMemsetAsync(d_stat_.p, 0, 2 * sizeof(unsigned long long), s));
     const long long total = (long long)rows * num_roots;
@@ -412,10 +402,10 @@ class CCF {
   TreeDev<T> tree_;
   FmmDev fmm_;
   LeafSet leaves_;
-  DevVec<double2> d_roots_, d_scratch_, d_ccs_, d_caus_, d_spos_;
+  DevVec<double2> d_roots_, d_scratch_, d_ccs_, d_caus_, d_spos_, d_phase_;
   DevVec<double> d_mu_;
   DevVec<unsigned char> d_fin_;
-  DevVec<unsigned long long> d_stat_;
+  DevVec<unsigned long long> d_stat_, d_words_;
 
   // Corner of a circular field of num_stars stars (include/ccf.cuh:427-432).
   cplx<T> scaled_circle(cplx<T> c, T mm) const {

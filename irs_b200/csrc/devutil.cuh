@@ -84,6 +84,54 @@ struct HostVec {
   }
 };
 
+// ---------------------------------------------------------------- grid barrier
+// Barrier of a cooperative grid, one 64-bit word per barrier (zeroed before
+// the launch): every CTA adds 1 + 2^32 * value, value the sum of its threads'
+// `value` given on the first lane of each warp (>= 0, below 2^31 in all), and
+// leaves with the sum over the grid once all have arrived. Writes before the
+// barrier are visible after it to plain loads (not to the read-only path). The
+// wait is bounded: after `spins` reads of the word (about a microsecond each;
+// a cooperative grid is resident as a whole, so it is never reached) or when
+// another CTA gave up, *err is set and the sum returned is -1.
+__device__ __forceinline__ int grid_barrier_sum(unsigned long long* word, int value, int* err, long long spins) {
+  __shared__ int s_value, s_sum;
+  if (threadIdx.x == 0) s_value = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0 && value) atomicAdd(&s_value, value);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // this CTA's writes before its arrival
+    atomicAdd(word, 1ull + ((unsigned long long)s_value << 32));
+    int sum = -1;
+    for (long long n = 0; n < spins; n++) {
+      unsigned long long v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+      if ((v & 0xffffffffull) == gridDim.x) {
+        sum = int(v >> 32);
+        break;
+      }
+      if ((n & 1023) == 1023 && *(volatile int*)err) break;
+    }
+    if (sum < 0) atomicExch(err, 1);
+    __threadfence();
+    s_sum = sum;
+  }
+  __syncthreads();
+  return s_sum;
+}
+
+// CTAs of a cooperative grid: `want`, at most what is resident at once.
+template <typename K>
+bool cooperative_grid(K kernel, int threads, long long want, int* grid) {
+  int dev = 0, sms = 0, per_sm = 0;
+  IRSB_CKR(cudaGetDevice(&dev));
+  IRSB_CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  IRSB_CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+  const long long most = (long long)sms * per_sm;
+  *grid = int(want < 1 ? 1 : (want > most ? most : want));
+  return true;
+}
+
 // ---------------------------------------------------------------- scan
 // Exclusive prefix sum of n values (int or long long input), written as long
 // long. Three passes: per-block totals, a single-block scan of the totals, and

@@ -46,3 +46,30 @@ def test_ray_bands_with_parities_add_up(gpu, dbl):
     for a, w in zip(acc, whole):
         np.testing.assert_array_equal(a, w)
     m.close()
+
+
+@pytest.mark.parametrize("n,nphi,nb", [(1, 4, 1), (2, 12, 3), (3, 8, 4), (33, 8, 2)])
+def test_critical_curves_of_few_stars_match_oracle(gpu, tmp_path, n, nphi, nb):
+    """Fields of fewer roots than a CTA has warps, one phi step per side, many
+    branches: the sets of critical-curve points at every phi agree with the
+    oracle's to its expansion error."""
+    from scipy.optimize import linear_sum_assignment
+
+    from oracle import ccf_ref
+    from tests.test_gpu_ccf import as_complex, star_field, write_stars
+    stars, rad = star_field(n, kstar=0.3, seed=40 + n)
+    write_stars(str(tmp_path / "s.bin"), stars, rad)
+    c = irs_b200.CCF(kappa_tot=0.45, shear=0.25, starfile=str(tmp_path / "s.bin"), num_phi=nphi, num_branches=nb)
+    c.run()
+    assert c.value("max_error") < 1e-8
+    L = ccf_ref.Lens(stars, 0.45, 0.25, c.kappa_star, 1.0, 1, rad)
+    z = ccf_ref.critical_curves(L, ccf_ref.initial_roots(stars, c.num_roots, nphi, nb, rad), nphi, nb)
+    ref, got = ccf_ref.outputs(L, z, nb)[0], as_complex(c.critical_curves)
+    assert ref.shape == got.shape
+    for b in range(nb):
+        rows = np.arange(b, ref.shape[0], nb)
+        for k in range(ref.shape[1]):
+            d = np.abs(ref[rows, k][:, None] - got[rows, k][None, :])
+            i, j = linear_sum_assignment(d)
+            assert d[i, j].max() < 1e-7
+    c.close()
