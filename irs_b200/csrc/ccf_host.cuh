@@ -165,8 +165,8 @@ class CCF {
     if (starfile.empty()) {
       while (random_seed == 0) random_seed = int(std::chrono::system_clock::now().time_since_epoch().count());
       const int blocks = std::max(1, std::min(ceil_div(n, 256), 148 * 16));
-      generate_stars_kernel<T><<<blocks, 256, 0, s>>>(d_stars_.p, n, random_seed, rectangular, corner, mf,
-                                                       m_lower_run, m_upper_run, m_solar);
+      generate_stars_kernel<T><<<blocks, 256, 0, s>>>(
+          d_stars_.p, n, StarDraw<T>{random_seed, rectangular, mf, corner, m_lower_run, m_upper_run, m_solar});
       IRSB_LAUNCH_CK("generate_stars_kernel");
       field.resize(n);
       IRSB_CKR(cudaMemcpyAsync(field.data(), d_stars_.p, size_t(n) * sizeof(StarRec<T>), cudaMemcpyDeviceToHost, s));

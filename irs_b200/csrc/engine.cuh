@@ -226,8 +226,9 @@ class MapMaker {
       while (p.random_seed == 0)
         p.random_seed = int(std::chrono::system_clock::now().time_since_epoch().count());
       int blocks = std::max(1, std::min(ceil_div(n, 256), 148 * 16));
-      generate_stars_kernel<T><<<blocks, 256, 0, stream_>>>(d_stars_.p, n, p.random_seed, p.rectangular, p.corner,
-                                                            p.mf_kind, p.m_lower, p.m_upper, p.m_solar);
+      generate_stars_kernel<T><<<blocks, 256, 0, stream_>>>(
+          d_stars_.p, n,
+          StarDraw<T>{p.random_seed, p.rectangular, p.mf_kind, p.corner, p.m_lower, p.m_upper, p.m_solar});
       IRSB_LAUNCH_CK("generate_stars_kernel");
       stars_out.resize(n);
       IRSB_CKR(cudaMemcpyAsync(stars_out.data(), d_stars_.p, size_t(n) * sizeof(StarRec<T>), cudaMemcpyDeviceToHost,

@@ -16,29 +16,59 @@
 
 namespace irsb {
 
+// What star i of a field is drawn with.
 template <typename T>
-__global__ void __launch_bounds__(256) generate_stars_kernel(StarRec<T>* __restrict__ stars, int n, int seed,
-                                                             int rectangular, cplx<T> corner, int mf_kind,
-                                                             T m_lower, T m_upper, T m_solar) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    curandState st;
-    curand_init((unsigned long long)seed, (unsigned long long)i, 0ULL, &st);
-    T x1, x2;
-    if (rectangular) {
-      x1 = T(curand_uniform_double(&st) * 2 * corner.re - corner.re);
-      x2 = T(curand_uniform_double(&st) * 2 * corner.im - corner.im);
-    } else {
-      T a = T(curand_uniform_double(&st) * 2 * kPi<T>);
-      T r = T(sqrt(curand_uniform_double(&st)) * cabs_(corner));
-      x1 = r * xcos(a);
-      x2 = r * xsin(a);
+struct StarDraw {
+  int seed, rectangular, mf_kind;
+  cplx<T> corner;
+  T m_lower, m_upper, m_solar;
+};
+
+template <typename T>
+__device__ __forceinline__ StarRec<T> draw_star(const StarDraw<T>& d, int i) {
+  curandState st;
+  curand_init((unsigned long long)d.seed, (unsigned long long)i, 0ULL, &st);
+  T x1, x2;
+  if (d.rectangular) {
+    x1 = T(curand_uniform_double(&st) * 2 * d.corner.re - d.corner.re);
+    x2 = T(curand_uniform_double(&st) * 2 * d.corner.im - d.corner.im);
+  } else {
+    T a = T(curand_uniform_double(&st) * 2 * kPi<T>);
+    T r = T(sqrt(curand_uniform_double(&st)) * cabs_(d.corner));
+    x1 = r * xcos(a);
+    x2 = r * xsin(a);
+  }
+  T p = T(curand_uniform_double(&st));
+  StarRec<T> s;
+  s.x = x1;
+  s.y = x2;
+  s.m = mf_mass<T>(d.mf_kind, p, d.m_lower, d.m_upper, d.m_solar);
+  return s;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) generate_stars_kernel(StarRec<T>* __restrict__ stars, int n, StarDraw<T> d) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) stars[i] = draw_star(d, i);
+}
+
+// The fields of R realizations in one launch: realization r owns the stars
+// [off[r], off[r + 1]). Bound by curand_init's skip-ahead, a long dependent
+// chain per star that one field of 8e4 stars leaves mostly exposed: a launch
+// per field took 5.5 ms for 24 fields of 1.9e6 stars in all (B200), this one
+// 3.4 ms.
+template <typename T>
+__global__ void __launch_bounds__(256) generate_stars_batch(StarRec<T>* __restrict__ stars, int R,
+                                                            const long long* __restrict__ off,
+                                                            const StarDraw<T>* __restrict__ draw) {
+  const long long n = off[R];
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    int lo = 0, hi = R - 1;  // last realization with off[r] <= q
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (off[mid] <= q) lo = mid;
+      else hi = mid - 1;
     }
-    T p = T(curand_uniform_double(&st));
-    StarRec<T> s;
-    s.x = x1;
-    s.y = x2;
-    s.m = mf_mass<T>(mf_kind, p, m_lower, m_upper, m_solar);
-    stars[i] = s;
+    stars[q] = draw_star(draw[lo], int(q - off[lo]));
   }
 }
 

@@ -48,9 +48,9 @@ def test_ray_bands_with_parities_add_up(gpu, dbl):
     m.close()
 
 
-@pytest.mark.parametrize("n,nphi,nb", [(1, 4, 1), (2, 12, 3), (3, 8, 4), (33, 8, 2)])
+@pytest.mark.parametrize("n,nphi,nb", [(1, 40, 2), (2, 12, 3), (3, 8, 4), (33, 8, 2)])
 def test_critical_curves_of_few_stars_match_oracle(gpu, tmp_path, n, nphi, nb):
-    """Fields of fewer roots than a CTA has warps, one phi step per side, many
+    """Fields of fewer roots than a CTA has warps, one phi step per side, several
     branches: the sets of critical-curve points at every phi agree with the
     oracle's to its expansion error."""
     from scipy.optimize import linear_sum_assignment
@@ -73,3 +73,21 @@ def test_critical_curves_of_few_stars_match_oracle(gpu, tmp_path, n, nphi, nb):
             i, j = linear_sum_assignment(d)
             assert d[i, j].max() < 1e-7
     c.close()
+
+
+@pytest.mark.parametrize("index", [11, 17])
+def test_batch_mass_sums_of_large_fields(gpu, index):
+    """Kroupa fields of 3.8e5 and 7.6e5 float masses: the sums of m are exact in
+    any order; the sum of m^2 of the larger one passes the last bit of its
+    smallest terms on the way and is finished star by star. The corner, hence
+    the map, is the single run's bit for bit."""
+    from irs_b200.batch import random_realizations
+    kw = random_realizations(24, num_pixels=32, half_length=12.0)[0][index]
+    b = irs_b200.BatchIPM([kw], expansion_order=10)
+    b.run()
+    s = irs_b200.IPM(**kw, expansion_order=10)
+    s.run()
+    assert int(b.value("num_stars", 0)) == s.num_stars > 3e5
+    np.testing.assert_array_equal(b.maps[0], s.magnifications)
+    b.close()
+    s.close()
