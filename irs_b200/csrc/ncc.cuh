@@ -23,7 +23,9 @@
 //     in explicitly rounded FP64 (the reference evaluates the same quantity
 //     through logarithms and exponentials, :62-98), so a host
 //     restatement with the same operations gives the same map bit for bit;
-//   * the block maximum is one pass over the fine map.
+//   * up to over_sample 3 the fine map is never stored: one warp per output
+//     row sums the differences of its fine rows side by side and keeps the
+//     block maxima (ncc_rows_pool).
 #pragma once
 #include "common.cuh"
 
@@ -71,10 +73,11 @@ __device__ __forceinline__ void ncc_correct(double& x, double& y, double xo, dou
 }
 
 // One thread per segment (row i, points j and j + 1) of the caustics.
-// diff: [npy][npx + 1] row differences of the fine map; err counts crossings
-// that would land outside the map (the reference prints an error for them).
-__global__ void ncc_segments(const double2* __restrict__ caus, int nrows, int ncols, NccGeom g, int* __restrict__ diff,
-                             int* __restrict__ err) {
+// diff: row differences of the fine map (rows ld values apart); err counts
+// crossings that would land outside the map (the reference prints an error
+// for them).
+__global__ void ncc_segments(const double2* __restrict__ caus, int nrows, int ncols, NccGeom g, long long ld,
+                             int* __restrict__ diff, int* __restrict__ err) {
   const long long nseg = (long long)nrows * (ncols - 1);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nseg; q += (long long)gridDim.x * blockDim.x) {
     const long long i = q / (ncols - 1), j = q - i * (ncols - 1);
@@ -112,20 +115,112 @@ __global__ void ncc_segments(const double2* __restrict__ caus, int nrows, int nc
         atomicAdd(err, 1);
         continue;
       }
-      int* d = diff + (long long)row * (g.npx + 1);
+      int* d = diff + (long long)row * ld;
       atomicAdd(d, v);
       atomicAdd(d + col + 1, -v);
     }
   }
 }
 
-// Fine map from the row differences: one warp per row, 32 columns per step
-// with a carried running sum.
-__global__ void ncc_rows(const int* __restrict__ diff, int npx, int npy, int* __restrict__ fine) {
+// Row stride of the differences: npx + 1 values, a multiple of 4 so that every
+// row starts on 16 bytes.
+__host__ __device__ __forceinline__ long long ncc_row_stride(int npx) { return ((long long)npx + 4) & ~3LL; }
+
+// Smallest and largest value of the lanes into range[0], range[1].
+__device__ __forceinline__ void ncc_range(int lo, int hi, int* range) {
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0 && lo <= hi) {
+    atomicMin(&range[0], lo);
+    atomicMax(&range[1], hi);
+  }
+}
+
+// Output rows straight from the differences, B = 1, 2, 4 or 8 fine rows and
+// columns per output pixel: one warp per output row walks its B fine rows side
+// by side, 128 columns a step, lane q columns 4q .. 4q + 3 of the step. Each
+// row's prefix sum carries over the steps; the maximum over the B rows and over
+// the columns of an output pixel is taken in registers (for B = 8 with the
+// neighbouring lane). The next step's differences are loaded ahead. Also the
+// range of the output.
+// Bound by reading the differences (4 B per fine pixel); with the fine map
+// written and read back, and its range and histogram taken on the host, the
+// two passes took 80 us of a 3.4 ms run for 1000^2 pixels at over_sample 2
+// (B200); now 24 us and 0.68 ms.
+template <int B>
+__global__ void __launch_bounds__(128) ncc_rows_pool(const int* __restrict__ diff, long long ld, int npx, int npy,
+                                                     int* __restrict__ out, int* __restrict__ range) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const long long fx = (long long)npx * B;
+  int lo = 0x7fffffff, hi = int(0x80000000);
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < npy; r += warps) {
+    const int* d = diff + (long long)r * B * ld;
+    int* o = out + (long long)r * npx;
+    int carry[B];
+    int4 next[B];
+    auto load = [&](long long c) {
+#pragma unroll
+      for (int b = 0; b < B; b++)  // ld is a multiple of 4: a whole quad or none
+        next[b] = c < ld ? *reinterpret_cast<const int4*>(d + b * ld + c) : make_int4(0, 0, 0, 0);
+    };
+#pragma unroll
+    for (int b = 0; b < B; b++) carry[b] = 0;
+    load(4 * lane);
+    for (long long c0 = 0; c0 < fx; c0 += 128) {
+      const long long c = c0 + 4 * lane;
+      int4 v[B];
+#pragma unroll
+      for (int b = 0; b < B; b++) v[b] = next[b];
+      load(c + 128);
+      int m[4];
+#pragma unroll
+      for (int b = 0; b < B; b++) {
+        v[b].y += v[b].x;
+        v[b].z += v[b].y;
+        v[b].w += v[b].z;
+        int incl = v[b].w;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, incl, s);
+          if (lane >= s) incl += u;
+        }
+        const int base = carry[b] + incl - v[b].w;
+        const int x[4] = {base + v[b].x, base + v[b].y, base + v[b].z, base + v[b].w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) m[i] = b == 0 ? x[i] : max(m[i], x[i]);
+        carry[b] += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      auto put = [&](long long p, int val) {
+        if (p < npx) {
+          o[p] = val;
+          lo = min(lo, val);
+          hi = max(hi, val);
+        }
+      };
+      if (B == 1) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) put(c + i, m[i]);
+      } else if (B == 2) {
+        put(c / 2, max(m[0], m[1]));
+        put(c / 2 + 1, max(m[2], m[3]));
+      } else {
+        int mm = max(max(m[0], m[1]), max(m[2], m[3]));
+        if (B == 8) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, 1));
+        if (B == 4 || (lane & 1) == 0) put(c / B, mm);
+      }
+    }
+  }
+  ncc_range(lo, hi, range);
+}
+
+// Fine map from the row differences (larger B): one warp per row, 32 columns
+// per step with a carried running sum.
+__global__ void ncc_rows(const int* __restrict__ diff, long long ld, int npx, int npy, int* __restrict__ fine) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < npy; r += warps) {
-    const int* d = diff + (long long)r * (npx + 1);
+    const int* d = diff + (long long)r * ld;
     int* out = fine + (long long)r * npx;
     int carry = 0;
     for (int c0 = 0; c0 < npx; c0 += 32) {
@@ -143,15 +238,20 @@ __global__ void ncc_rows(const int* __restrict__ diff, int npx, int npy, int* __
 }
 
 // Output pixel = maximum over its B x B block of the fine map (B = 2^over_sample).
-__global__ void ncc_pool(const int* __restrict__ fine, int npx, int npy, int B, int* __restrict__ out) {
+__global__ void ncc_pool(const int* __restrict__ fine, int npx, int npy, int B, int* __restrict__ out,
+                         int* __restrict__ range) {
   const long long n = (long long)npx * npy;
+  int lo = 0x7fffffff, hi = int(0x80000000);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     const int r = int(q / npx), c = int(q - (long long)r * npx);
     int m = fine[(long long)r * B * npx * B + (long long)c * B];
     for (int dy = 0; dy < B; dy++)
       for (int dx = 0; dx < B; dx++) m = max(m, fine[((long long)r * B + dy) * npx * B + (long long)c * B + dx]);
     out[q] = m;
+    lo = min(lo, m);
+    hi = max(hi, m);
   }
+  ncc_range(lo, hi, range);
 }
 
 }  // namespace irsb

@@ -4,6 +4,7 @@
 // Declarations and the extensions are in include/lib_ncc.h.
 #include "ncc_host.cuh"
 
+#include <cstring>
 #include <limits>
 
 using dtype = double;
@@ -50,9 +51,8 @@ void destroy(Obj* self) { delete self; }
 void set_caustics(Obj* self, const double* vals, int nrows, int ncols) {
   self->host_rows = vals && nrows > 0 && ncols > 0 ? nrows : 0;
   self->host_cols = self->host_rows ? ncols : 0;
-  self->host_caustics.assign(size_t(self->host_rows) * self->host_cols, make_double2(0, 0));
-  for (size_t k = 0; k < self->host_caustics.size(); k++)
-    self->host_caustics[k] = make_double2(vals[2 * k], vals[2 * k + 1]);
+  self->host_caustics.resize(size_t(self->host_rows) * self->host_cols);
+  if (self->host_rows) std::memcpy(self->host_caustics.data(), vals, self->host_caustics.size() * sizeof(double2));
 }
 double get_value(Obj* self, const char* name) {
   const std::string n = name ? name : "";

@@ -36,7 +36,8 @@ class NCC {
   // ---- results ----
   double t_ncc = 0, t_reduce = 0;
   int num_rows = 0, num_cols = 0, min_num = 0, max_num = 0, errors = 0;
-  std::vector<int> map, histogram;
+  std::vector<int> histogram;
+  HostVec<int> map;  // pinned: the transfer's own target
 
   ~NCC() {
     for (cudaEvent_t* e : {&e0_, &e1_, &e2_})
@@ -44,7 +45,7 @@ class NCC {
     if (stream_) cudaStreamDestroy(stream_);
   }
 
-  int* num_crossings() { return map.empty() ? nullptr : map.data(); }
+  int* num_crossings() { return map.p; }
 
   // include/ncc.cuh:131-171
   bool check_input_params() const {
@@ -70,14 +71,14 @@ class NCC {
       for (cudaEvent_t* e : {&e0_, &e1_, &e2_}) IRSB_CKR(cudaEventCreate(e));
     }
     cudaStream_t s = stream_;
-    std::vector<double2> caus;
+    std::vector<double2> file_caustics;
     if (host_rows > 0) {
-      caus = host_caustics;
       num_rows = host_rows;
       num_cols = host_cols;
-    } else if (!read_caustics(infile_prefix + "ccf_caustics.bin", caus)) {
+    } else if (!read_caustics(infile_prefix + "ccf_caustics.bin", file_caustics)) {
       return false;
     }
+    const std::vector<double2>& caus = host_rows > 0 ? host_caustics : file_caustics;
     if (num_rows < 1 || num_cols < 2) {
       std::cerr << "Error. Need at least 1 row and 2 columns of caustic positions.\n";
       return false;
@@ -88,48 +89,73 @@ class NCC {
       std::cerr << "Error. The oversampled map is too large.\n";
       return false;
     }
-    const long long nfine = fx * fy, ndiff = fy * (fx + 1), nout = (long long)num_pixels_y.re * num_pixels_y.im;
-    if (!d_caus_.alloc_exact(caus.size()) || !d_diff_.alloc_exact(ndiff) || !d_fine_.alloc_exact(nfine) ||
-        !d_out_.alloc_exact(nout) || !d_err_.alloc_exact(1))
+    const long long ld = ncc_row_stride(int(fx)), ndiff = fy * ld;
+    const long long nout = (long long)num_pixels_y.re * num_pixels_y.im;
+    const bool pooled = B <= 8;  // the fine map is not stored
+    if (!d_caus_.alloc_exact(caus.size()) || !d_diff_.alloc_exact(ndiff) ||
+        (!pooled && !d_fine_.alloc_exact(fx * fy)) || !d_out_.alloc_exact(nout) || !d_stat_.alloc_exact(3) ||
+        !h_stat_.alloc(3) || !map.alloc(nout))
       return false;
-    IRSB_CKR(cudaMemcpyAsync(d_caus_.p, caus.data(), caus.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
     IRSB_CKR(cudaMemsetAsync(d_diff_.p, 0, ndiff * sizeof(int), s));
-    IRSB_CKR(cudaMemsetAsync(d_err_.p, 0, sizeof(int), s));
+    h_stat_.p[0] = 0;  // errors, smallest, largest value
+    h_stat_.p[1] = std::numeric_limits<int>::max();
+    h_stat_.p[2] = std::numeric_limits<int>::min();
+    IRSB_CKR(cudaMemcpyAsync(d_stat_.p, h_stat_.p, 3 * sizeof(int), cudaMemcpyHostToDevice, s));
+    IRSB_CKR(cudaMemcpyAsync(d_caus_.p, caus.data(), caus.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
     const NccGeom g{double(center_y.re), double(center_y.im), double(half_length_y.re), double(half_length_y.im),
                     int(fx), int(fy)};
     const long long nseg = (long long)num_rows * (num_cols - 1);
+    const int npx = num_pixels_y.re, npy = num_pixels_y.im;
     IRSB_CKR(cudaEventRecord(e0_, s));
     ncc_segments<<<int(std::max<long long>(1, std::min<long long>(ceil_div(nseg, 256LL), 148LL * 16))), 256, 0, s>>>(
-        d_caus_.p, num_rows, num_cols, g, d_diff_.p, d_err_.p);
+        d_caus_.p, num_rows, num_cols, g, ld, d_diff_.p, d_stat_.p);
     IRSB_LAUNCH_CK("ncc_segments");
-    ncc_rows<<<int(std::max<long long>(1, std::min<long long>(ceil_div(fy * 32, 256LL), 148LL * 16))), 256, 0, s>>>(
-        d_diff_.p, int(fx), int(fy), d_fine_.p);
-    IRSB_LAUNCH_CK("ncc_rows");
-    IRSB_CKR(cudaEventRecord(e1_, s));
-    ncc_pool<<<int(std::max<long long>(1, std::min<long long>(ceil_div(nout, 256LL), 148LL * 16))), 256, 0, s>>>(
-        d_fine_.p, num_pixels_y.re, num_pixels_y.im, B, d_out_.p);
-    IRSB_LAUNCH_CK("ncc_pool");
+    if (pooled) {
+      IRSB_CKR(cudaEventRecord(e1_, s));
+      auto kernel = B == 1 ? ncc_rows_pool<1> : (B == 2 ? ncc_rows_pool<2> : (B == 4 ? ncc_rows_pool<4> : ncc_rows_pool<8>));
+      kernel<<<std::max(1, std::min(ceil_div(npy, 4LL), 148 * 16)), 128, 0, s>>>(d_diff_.p, ld, npx, npy, d_out_.p,
+                                                                              d_stat_.p + 1);
+      IRSB_LAUNCH_CK("ncc_rows_pool");
+    } else {
+      ncc_rows<<<int(std::max<long long>(1, std::min<long long>(ceil_div(fy * 32, 256LL), 148LL * 16))), 256, 0, s>>>(
+          d_diff_.p, ld, int(fx), int(fy), d_fine_.p);
+      IRSB_LAUNCH_CK("ncc_rows");
+      IRSB_CKR(cudaEventRecord(e1_, s));
+      ncc_pool<<<int(std::max<long long>(1, std::min<long long>(ceil_div(nout, 256LL), 148LL * 16))), 256, 0, s>>>(
+          d_fine_.p, npx, npy, B, d_out_.p, d_stat_.p + 1);
+      IRSB_LAUNCH_CK("ncc_pool");
+    }
     IRSB_CKR(cudaEventRecord(e2_, s));
-    map.resize(nout);
-    IRSB_CKR(cudaMemcpyAsync(map.data(), d_out_.p, nout * sizeof(int), cudaMemcpyDeviceToHost, s));
-    IRSB_CKR(cudaMemcpyAsync(&errors, d_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    IRSB_CKR(cudaMemcpyAsync(h_stat_.p, d_stat_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
     IRSB_CKR(cudaStreamSynchronize(s));
     float m01 = 0, m12 = 0;
     IRSB_CKR(cudaEventElapsedTime(&m01, e0_, e1_));
     IRSB_CKR(cudaEventElapsedTime(&m12, e1_, e2_));
     t_ncc = m01 * 1e-3;
     t_reduce = m12 * 1e-3;
+    errors = h_stat_.p[0];
+    min_num = h_stat_.p[1];
+    max_num = h_stat_.p[2];
     if (errors) std::cerr << "Error. Caustic crossing takes place outside the desired region.\n";
-    min_num = *std::min_element(map.begin(), map.end());
-    max_num = *std::max_element(map.begin(), map.end());
+    IRSB_CKR(cudaMemcpyAsync(map.p, d_out_.p, nout * sizeof(int), cudaMemcpyDeviceToHost, s));
+    histogram.clear();
+    if (write_histograms && min_num >= 0) {  // include/ncc.cuh:330-355
+      const int len = max_num - min_num + 1;
+      if (!d_hist_.alloc_exact(len)) return false;
+      IRSB_CKR(cudaMemsetAsync(d_hist_.p, 0, size_t(len) * sizeof(int), s));
+      const int gh = int(std::max<long long>(1, std::min<long long>(ceil_div(nout, 1024LL), 148LL)));
+      if (len <= kHistSmemBins)
+        histogram_map_smem<int><<<gh, 1024, size_t(len) * sizeof(int), s>>>(d_out_.p, nout, min_num, len, 1, 0, d_hist_.p);
+      else
+        histogram_map<int><<<gh, 1024, 0, s>>>(d_out_.p, nout, min_num, len, 1, 0, d_hist_.p);
+      IRSB_LAUNCH_CK("histogram_map");
+      histogram.resize(len);
+      IRSB_CKR(cudaMemcpyAsync(histogram.data(), d_hist_.p, size_t(len) * sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
+    IRSB_CKR(cudaStreamSynchronize(s));
     if (min_num < 0) {
       std::cerr << "Error. Number of caustic crossings should be >= 0\n";
       return false;
-    }
-    histogram.clear();
-    if (write_histograms) {  // include/ncc.cuh:330-355
-      histogram.assign(max_num - min_num + 1, 0);
-      for (int v : map) histogram[v - min_num]++;
     }
     if (verbose >= 1)
       std::cout << "ncc: " << num_rows << " x " << num_cols << " caustic points, map " << num_pixels_y.re << " x "
@@ -140,7 +166,7 @@ class NCC {
 
   // include/ncc.cuh:357-440
   bool save(int verbose) {
-    if (map.empty()) {
+    if (!map.p) {
       std::cerr << "Error. save() needs a completed run().\n";
       return false;
     }
@@ -174,7 +200,7 @@ class NCC {
       const int nr = num_pixels_y.im, nc = num_pixels_y.re;
       m.write(reinterpret_cast<const char*>(&nr), sizeof(int));
       m.write(reinterpret_cast<const char*>(&nc), sizeof(int));
-      m.write(reinterpret_cast<const char*>(map.data()), map.size() * sizeof(int));
+      m.write(reinterpret_cast<const char*>(map.p), map.n * sizeof(int));
       if (!m) return false;
     }
     if (verbose >= 1) std::cout << "Done writing NCC files with prefix " << outfile_prefix << "\n";
@@ -185,7 +211,8 @@ class NCC {
   cudaStream_t stream_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr, e2_ = nullptr;
   DevVec<double2> d_caus_;
-  DevVec<int> d_diff_, d_fine_, d_out_, d_err_;
+  DevVec<int> d_diff_, d_fine_, d_out_, d_stat_, d_hist_;
+  HostVec<int> h_stat_;
 
   // read_complex_array (include/array_functions.cuh:172-268): int nrows, int
   // ncols, then complex values in T, float or double (by the file size).

@@ -91,3 +91,26 @@ def test_batch_mass_sums_of_large_fields(gpu, index):
     np.testing.assert_array_equal(b.maps[0], s.magnifications)
     b.close()
     s.close()
+
+
+@pytest.mark.parametrize("over", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("npix", [(1, 1), (3, 2), (32, 31), (33, 5), (127, 9), (128, 8), (129, 7)])
+def test_crossing_maps_around_the_column_step(gpu, npix, over):
+    """Maps whose rows end inside, at and past a step of 128 fine columns, in
+    every oversampling the pooled kernel takes (0 to 3) and one it does not,
+    against the oracle's counts."""
+    from oracle import pyoracle as po
+    rng = np.random.default_rng(npix[0] + 7 * over)
+    t = -np.linspace(0, 2 * np.pi, 41)
+    c = (rng.normal(0, 1, (60, 1)) + 1j * rng.normal(0, 1, (60, 1))
+         + rng.uniform(0.1, 1, (60, 1)) * (np.cos(t) ** 3 + 1j * np.sin(t) ** 3))
+    c[:, -1] = c[:, 0]
+    n = irs_b200.NCC(half_length_y1=1.5, half_length_y2=1.2, num_pixels_y1=npix[0], num_pixels_y2=npix[1],
+                     over_sample=over)
+    n.set_caustics(c)
+    n.run()
+    ref, err = po.ncc(c, (0, 0), (1.5, 1.2), npix, over)
+    assert err == n.value("errors")
+    np.testing.assert_array_equal(n.num_caustic_crossings, ref)
+    assert (n.value("min_num"), n.value("max_num")) == (ref.min(), ref.max())
+    n.close()
