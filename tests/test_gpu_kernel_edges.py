@@ -114,3 +114,56 @@ def test_crossing_maps_around_the_column_step(gpu, npix, over):
     np.testing.assert_array_equal(n.num_caustic_crossings, ref)
     assert (n.value("min_num"), n.value("max_num")) == (ref.min(), ref.max())
     n.close()
+
+
+def _corner_lattice(kind, rng):
+    j, i = np.meshgrid(np.arange(31.0), np.arange(41.0), indexing="ij")
+    x, y = (i - 20) * 1.1, (j - 15) * 1.1
+    if kind == "horizontal":  # edges along rows, many of them on pixel lines
+        return np.stack([x * 0.7, np.floor(y * 3) / 3], -1)
+    if kind == "slivers":  # nearly vertical edges, rows snapped to lines
+        yy = np.where(rng.random(y.shape) < 0.3, np.floor(y), y)
+        return np.stack([x * 0.01 + rng.normal(0, 1e-7, x.shape), yy], -1)
+    if kind == "just_past_lines":
+        yy = np.floor(y) + np.where(rng.random(y.shape) < 0.5, 1e-9, 0.0)
+        return np.stack([np.floor(x) + np.where(rng.random(x.shape) < 0.3, -1e-12, 0.0), yy], -1)
+    if kind == "point_lens":  # cells stretched over many pixels around a lens
+        r2 = x * x + y * y + 0.01
+        return np.stack([x - 30 * x / r2, y - 30 * y / r2], -1)
+    if kind == "far":  # beyond the range of int, not finite
+        v = np.stack([x, y], -1)
+        pick = rng.random(x.shape)
+        for k, val in enumerate([3.0e9, -3.0e9, 5.0e9, 1e18, -1e300, np.inf, -np.inf, np.nan, 2147483648.0, -2147483649.0]):
+            v[(pick >= 0.01 * k) & (pick < 0.01 * (k + 1)), k % 2] = val
+        return v
+    if kind == "fine":  # most triangles inside one pixel
+        return np.stack([x * 0.04 + 0.013 * y, y * 0.05 - 0.01 * x], -1)
+    return np.stack([x, y], -1) + rng.normal(0, 3.0, x.shape + (2,))  # "tangled"
+
+
+@pytest.mark.parametrize("dbl", [False, True])
+@pytest.mark.parametrize("kind", ["horizontal", "slivers", "just_past_lines", "point_lens", "far", "fine", "tangled"])
+def test_deposition_of_awkward_cells(gpu, dbl, kind):
+    """Fixed-point maps bit for bit against the oracle's."""
+    import ctypes
+
+    import torch
+
+    import irs_b200._lib as L
+    from oracle import pyoracle as po
+    T, tdt = (ctypes.c_double, torch.float64) if dbl else (ctypes.c_float, torch.float32)
+    f = L.load("ipm", dbl).ipm_deposit_noalloc
+    f.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_longlong, T, ctypes.c_int, ctypes.c_int,
+                  ctypes.c_void_p, ctypes.c_void_p]
+    f.restype = ctypes.c_int
+    npx, npy, factor = 37, 29, 0.61
+    v = np.ascontiguousarray(_corner_lattice(kind, np.random.default_rng(11)) + np.array([npx / 2, npy / 2]))
+    d_v = torch.from_numpy(v).to("cuda")
+    d_map = torch.full((npy, npx), -1.0, dtype=tdt, device="cuda")
+    assert f(d_v.data_ptr(), v.shape[1] - 1, v.shape[0] - 1, factor, npx, npy, d_map.data_ptr(),
+             torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    q = po.ipm_deposit_fixed(v, factor if dbl else np.float32(factor), (npx, npy), single=not dbl)
+    got = d_map.cpu().numpy()
+    np.testing.assert_array_equal(got, (q.astype(np.float64) * 2.0 ** -32).astype(got.dtype))
+    assert q.any()
