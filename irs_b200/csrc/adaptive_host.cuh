@@ -442,9 +442,11 @@ class AdaptiveIPM {
     sps.nx = nxs;
     sps.ny = nys;
     sps.jbase = 0;
-    if (!build_lattice_tiles<T>(rtiles_, base.leaves_, base.tree_, sps.base_x, sps.base_y, sps.rhs_x, sps.rhs_y, nxs,
-                                nys, jlo, jhi, s))
+    if (!lattice_rects<T>(rtiles_, base.leaves_, base.tree_, base.leaves_.n, sps.base_x, sps.base_y, sps.rhs_x,
+                          sps.rhs_y, nxs, nys, jlo, jhi, s))
       return false;
+    IRSB_CKR(cudaStreamSynchronize(s));
+    if (!lattice_table<T>(rtiles_, base.leaves_, base.tree_, s)) return false;
     LeafPtrs lp = base.leaf_ptrs();
     lp.rect = rtiles_.rect.p;
     lp.tile_off = rtiles_.tile_off.p;

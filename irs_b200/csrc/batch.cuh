@@ -6,11 +6,10 @@
 //     one CTA per realization sums its masses in star order (the host
 //     summation of star_field_moments, so the corner and the tree root are
 //     those of a single run); the host recomputes the corners;
-//   * tree: one level-synchronous build over all roots (level l of every
-//     realization in the same launches), level sizes kept on the device, a
-//     fixed number of levels and fixed capacities checked on the device, so
-//     that no host synchronisation is needed and the whole build is captured;
-//   * expansions: the per-level FMM kernels over all realizations' nodes;
+//   * tree: one cooperative build over all roots (level l of every realization
+//     at the same time), fixed capacities checked on the device, so that no
+//     host synchronisation is needed and the whole build is captured;
+//   * expansions: the two FMM launches over all realizations' nodes;
 //   * leaves: one record set for all realizations (theta per realization);
 //   * shooting: passes over a bounded corner buffer; a pass holds row bands of
 //     one or more realizations, its tile list covers the leaves of all of them
@@ -168,57 +167,16 @@ __global__ void __launch_bounds__(kMomentThreads) batch_star_moments(const StarR
   }
 }
 
-// Roots of all realizations (level 0), level bookkeeping and flags reset.
-template <typename T>
-__global__ void batch_tree_roots(int R, const T* __restrict__ root_hl, const long long* __restrict__ star_off,
-                                 T* cx, T* cy, T* hl, int* level, int* parent, int* child0, int* sbeg, int* scnt,
-                                 int* rid, int* n_nbr, int* n_sil, int* n_dil, double* lox, double* hix, double* loy,
-                                 double* hiy, int* off, int* lvl_n, int nlev, int* stop, int* dstat,
-                                 int* levels_r) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    cx[r] = T(0);
-    cy[r] = T(0);
-    hl[r] = root_hl[r];
-    level[r] = 0;
-    parent[r] = -1;
-    child0[r] = -1;
-    sbeg[r] = int(star_off[r]);
-    scnt[r] = int(star_off[r + 1] - star_off[r]);
-    rid[r] = r;
-    n_nbr[r] = n_sil[r] = n_dil[r] = 0;
-    lox[r] = -INFINITY;
-    hix[r] = INFINITY;
-    loy[r] = -INFINITY;
-    hiy[r] = INFINITY;
-    levels_r[r] = 0;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    off[0] = 0;
-    off[1] = R;
-    for (int l = 2; l <= nlev + 1; l++) off[l] = R;
-    lvl_n[0] = R;
-    for (int l = 1; l <= nlev; l++) lvl_n[l] = 0;
-    *stop = 0;
-    dstat[0] = dstat[1] = 0;
-  }
-}
-
-__global__ void batch_levels(const int* __restrict__ off, int nlev, const int* __restrict__ level,
+// Tree levels of each realization (levels_r zeroed before).
+__global__ void batch_levels(const int* __restrict__ nodes, const int* __restrict__ level,
                              const int* __restrict__ rid, int* levels_r) {
-  const int n = off[nlev];
+  const int n = *nodes;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     // a level no deeper than one already seen (a stale read only costs the
     // atomic): without the test a node each queues on one word per
     // realization (1.6e6 nodes, 24 realizations, B200: 1.01 ms, now 0.27)
     if (*(volatile const int*)&levels_r[rid[k]] < level[k]) atomicMax(&levels_r[rid[k]], level[k]);
   }
-}
-
-__global__ void batch_set_count(const long long* __restrict__ sum, int* __restrict__ n) { *n = int(*sum); }
-
-__global__ void batch_tile_end(const int* __restrict__ nleaves, const long long* __restrict__ sum,
-                               long long* __restrict__ tile_off) {
-  tile_off[*nleaves] = *sum;
 }
 
 // ---------------------------------------------------------------- host driver
@@ -360,11 +318,11 @@ class BatchMaker {
   DevVec<StarDraw<T>> d_draw_;
   DevVec<T> d_mlo_, d_mhi_, d_root_hl_;
   DevVec<double> d_theta_;
-  DevVec<int> d_off_, d_lvl_n_, d_stop_, d_levels_;
+  DevVec<int> d_levels_;
   TreeDev<T> tree_;
   FmmDev fmm_;
   LeafSet leaves_;
-  DevVec<int> d_leaf_rid_, d_nleaves_;
+  DevVec<int> d_leaf_rid_;
   LatticeTiles tiles_;
   DevVec<ShootParams> d_sps_;
   DevVec<LatticeGeom> d_geom_;
@@ -610,25 +568,14 @@ class BatchMaker {
 
   bool plan_buffers() {
     const int R = size();
-    const long long ncoef = node_cap_ * (order + 1);
-    if (!tree_reserve(tree_, int(node_cap_), stream_) || !tree_.tmp_stars.reserve(total_stars, stream_) ||
-        !tree_.dstat.reserve(2, stream_) || !tree_.split.reserve(node_cap_, stream_) ||
-        !tree_.rank.reserve(node_cap_ + 1, stream_) || !scan_reserve(tree_.scan, node_cap_, stream_))
+    if (!tree_build_reserve(tree_, int(total_stars), int(node_cap_), stream_) || !d_levels_.alloc_exact(R) ||
+        !fmm_reserve(fmm_, node_cap_, order, stream_))
       return false;
-    if (!d_off_.alloc_exact(kMaxLevels + 2) || !d_lvl_n_.alloc_exact(kMaxLevels + 1) || !d_stop_.alloc_exact(1) ||
-        !d_levels_.alloc_exact(R))
-      return false;
-    if (!fmm_.mult.alloc_exact(ncoef) || !fmm_.loc.alloc_exact(ncoef)) return false;
-    fmm_.p = order;
-    std::vector<double> bt = binomial_table(2 * kMaxOrder);
-    if (!fmm_.btab.alloc_exact(bt.size())) return false;
-    IRSB_CKR(cudaMemcpyAsync(fmm_.btab.p, bt.data(), bt.size() * sizeof(double), cudaMemcpyHostToDevice, stream_));
     LeafSet& L = leaves_;
-    if (!L.flag.alloc_exact(node_cap_) || !L.pos.alloc_exact(node_cap_ + 1) || !L.node.alloc_exact(node_cap_) ||
+    if (!L.pos.alloc_exact(node_cap_) || !L.node.alloc_exact(node_cap_) ||
         !L.cx.alloc_exact(node_cap_) || !L.cy.alloc_exact(node_cap_) || !L.hl.alloc_exact(node_cap_) ||
         !L.nnear.alloc_exact(node_cap_) || !L.near32.alloc_exact(node_cap_ * kMaxStarsDirect) ||
-        !L.coef32.alloc_exact(node_cap_ * kMaxOrder) || !d_leaf_rid_.alloc_exact(node_cap_) ||
-        !d_nleaves_.alloc_exact(1) || !scan_reserve(L.scan, node_cap_, stream_))
+        !L.coef32.alloc_exact(node_cap_ * kMaxOrder) || !d_leaf_rid_.alloc_exact(node_cap_))
       return false;
     LatticeTiles& W = tiles_;
     if (!W.rect.alloc_exact(node_cap_) || !W.tiles.alloc_exact(node_cap_) || !W.tile_off.alloc_exact(node_cap_ + 1) ||
@@ -664,65 +611,20 @@ class BatchMaker {
     const int R = size();
     cudaStream_t s = stream_;
     TreeDev<T>& t = tree_;
-    const int G = 148 * 8;  // grid of the level kernels (grid-stride)
-    const int ncap = int(node_cap_);
-    int* dstat = t.dstat.p;
-    batch_tree_roots<T><<<ceil_div(R, 128), 128, 0, s>>>(
-        R, d_root_hl_.p, d_star_off_.p, t.cx.p, t.cy.p, t.hl.p, t.level.p, t.parent.p, t.child0.p, t.sbeg.p,
-        t.scnt.p, t.rid.p, t.n_nbr.p, t.n_sil.p, t.n_dil.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p, d_off_.p, d_lvl_n_.p,
-        nlev, d_stop_.p, dstat, d_levels_.p);
-    IRSB_LAUNCH_CK("batch_tree_roots");
-    for (int l = 0; l < nlev; l++) {
-      const LevelRange lr{d_off_.p, l};
-      tree_near_count<<<G, 256, 0, s>>>(0, 0, lr, t.scnt.p, t.nbr.p, t.n_nbr.p, t.split.p, dstat);
-      if (!exclusive_scan_dev<int>(t.split.p, d_lvl_n_.p + l, node_cap_, t.rank.p, t.scan, s)) return false;
-      tree_advance_level<<<1, 1, 0, s>>>(l, nlev, d_off_.p, d_lvl_n_.p, t.scan.sum.p, ncap, d_stop_.p, dstat);
-      tree_make_children<T><<<G, 256, 0, s>>>(0, 0, 0, lr, d_stop_.p, t.split.p, t.rank.p, t.cx.p, t.cy.p, t.hl.p,
-                                              t.level.p, t.parent.p, t.child0.p, t.sbeg.p, t.scnt.p, t.rid.p,
-                                              t.n_nbr.p, t.n_sil.p, t.n_dil.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p);
-      if (l + 1 < nlev) {
-        if (l < 2)  // a few nodes per realization, many stars each
-          tree_partition_stars<T, 1024><<<G, 1024, 0, s>>>(0, 0, lr, d_stop_.p, t.split.p, t.cx.p, t.cy.p,
-                                                            t.child0.p, t.sbeg.p, t.scnt.p, d_stars_.p,
-                                                            t.tmp_stars.p);
-        else
-          tree_partition_stars<T><<<G, 256, 0, s>>>(0, 0, lr, d_stop_.p, t.split.p, t.cx.p, t.cy.p, t.child0.p,
-                                                    t.sbeg.p, t.scnt.p, d_stars_.p, t.tmp_stars.p);
-        tree_set_neighbors<T><<<G, 256, 0, s>>>(0, 0, LevelRange{d_off_.p, l + 1}, t.cx.p, t.cy.p, t.hl.p,
-                                                t.parent.p, t.child0.p, t.scnt.p, t.nbr.p, t.n_nbr.p, t.sil.p,
-                                                t.n_sil.p, t.dil.p, t.n_dil.p, dstat);
-      }
-      IRSB_LAUNCH_CK("batch tree level");
-    }
-    batch_levels<<<G, 256, 0, s>>>(d_off_.p, nlev, t.level.p, t.rid.p, d_levels_.p);
-    // expansions
-    const long long ncoef = node_cap_ * (order + 1);
-    IRSB_CKR(cudaMemsetAsync(fmm_.mult.p, 0, ncoef * sizeof(double2), s));
-    IRSB_CKR(cudaMemsetAsync(fmm_.loc.p, 0, ncoef * sizeof(double2), s));
-    const int GF = 148 * 16;
-    for (int l = nlev - 1; l >= 0; l--) {
-      const LevelRange lr{d_off_.p, l};
-      fmm_p2m<T><<<GF, 256, 0, s>>>(0, 0, lr, order, t.cx.p, t.cy.p, t.hl.p, t.child0.p, t.sbeg.p, t.scnt.p,
-                                     d_stars_.p, fmm_.mult.p);
-      fmm_m2m<T><<<GF, 256, 0, s>>>(0, 0, lr, order, t.cx.p, t.cy.p, t.hl.p, t.child0.p, fmm_.btab.p, fmm_.mult.p);
-    }
-    for (int l = 2; l < nlev; l++) {
-      fmm_local<T><<<GF, 256, 0, s>>>(0, 0, LevelRange{d_off_.p, l}, order, t.cx.p, t.cy.p, t.hl.p, t.parent.p,
-                                       t.sbeg.p, t.scnt.p, t.sil.p, t.n_sil.p, t.dil.p, t.n_dil.p, d_stars_.p,
-                                       fmm_.btab.p, fmm_.mult.p, fmm_.loc.p);
-    }
-    IRSB_LAUNCH_CK("batch fmm");
-    // leaves
+    const int G = 148 * 8, GF = 148 * 16;  // grids of the grid-stride kernels
+    if (!launch_tree_build<T>(t, d_stars_.p, int(total_stars), R, T(0), d_root_hl_.p, d_star_off_.p, int(node_cap_),
+                              nlev, leaves_.pos.p, leaves_.node.p, s))
+      return false;
+    int* status = t.status.p;
+    const int *dnodes = status + kTreeOff + kMaxLevels + 1, *dleaves = status + kTreeLeaves;
+    IRSB_CKR(cudaMemsetAsync(d_levels_.p, 0, R * sizeof(int), s));
+    batch_levels<<<G, 256, 0, s>>>(dnodes, t.level.p, t.rid.p, d_levels_.p);
+    if (!compute_fmm<T>(fmm_, t, d_stars_.p, node_cap_, 0, s)) return false;  // a warp per node on every level
     LeafSet& L = leaves_;
-    const int* dnodes = d_off_.p + nlev;
-    leaf_flags<<<G, 256, 0, s>>>(0, dnodes, t.child0.p, L.flag.p);
-    if (!exclusive_scan_dev<int>(L.flag.p, dnodes, node_cap_, L.pos.p, L.scan, s)) return false;
-    batch_set_count<<<1, 1, 0, s>>>(L.scan.sum.p, d_nleaves_.p);
-    leaf_compact<<<G, 256, 0, s>>>(0, dnodes, L.flag.p, L.pos.p, L.node.p);
-    leaf_build<T><<<GF, 256, 0, s>>>(0, d_nleaves_.p, order, 1.0, d_theta_.p, t.rid.p, L.node.p, t.cx.p, t.cy.p,
-                                     t.hl.p, t.sbeg.p, t.scnt.p, t.nbr.p, t.n_nbr.p, d_stars_.p, fmm_.loc.p, L.cx.p,
-                                     L.cy.p, L.hl.p, L.nnear.p, nullptr, L.near32.p, nullptr, L.coef32.p,
-                                     d_leaf_rid_.p, dstat + 1);
+    leaf_build<T><<<GF, 256, 0, s>>>(0, dleaves, order, 1.0, d_theta_.p, t.rid.p, L.node.p, t.cx.p, t.cy.p, t.hl.p,
+                                     t.sbeg.p, t.scnt.p, t.nbr.p, t.n_nbr.p, d_stars_.p, fmm_.loc.p, L.cx.p, L.cy.p,
+                                     L.hl.p, L.nnear.p, nullptr, L.near32.p, nullptr, L.coef32.p, d_leaf_rid_.p,
+                                     status + kTreeNear);
     IRSB_LAUNCH_CK("batch leaves");
     // maps
     const long long npix = (long long)npx_ * npy_, ndiff = (long long)npy_ * (npx_ + 1);
@@ -732,15 +634,14 @@ class BatchMaker {
     LatticeTiles& W = tiles_;
     const LeafPtrs lp = leaf_ptrs();
     for (int c = 0; c < passes; c++) {
-      leaf_rects_batch<<<G, 256, 0, s>>>(d_nleaves_.p, L.node.p, t.rid.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p,
+      leaf_rects_batch<<<G, 256, 0, s>>>(dleaves, L.node.p, t.rid.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p,
                                          d_geom_.p, d_jlo_.p + (long long)c * R, d_jhi_.p + (long long)c * R, kTileX,
                                          kTileY, W.rect.p, W.tiles.p);
-      if (!exclusive_scan_dev<long long>(W.tiles.p, d_nleaves_.p, node_cap_, W.tile_off.p, W.scan, s)) return false;
-      batch_tile_end<<<1, 1, 0, s>>>(d_nleaves_.p, W.scan.sum.p, W.tile_off.p);
-      leaf_tile_table<<<G, 256, 0, s>>>(0, d_nleaves_.p, W.rect.p, W.tile_off.p, kTileX, kTileY, W.table.p,
-                                        table_cap_, dstat + 1);
+      if (!exclusive_scan_dev<long long>(W.tiles.p, dleaves, node_cap_, W.tile_off.p, W.scan, s)) return false;
+      leaf_tile_table<<<G, 256, 0, s>>>(0, dleaves, W.rect.p, W.tile_off.p, W.scan.sum.p, kTileX, kTileY, W.table.p,
+                                        table_cap_, status + kTreeTable);
       BatchShoot bs{d_sps_.p, d_leaf_rid_.p, d_jlo_.p + (long long)c * R, d_voff_.p + (long long)c * R,
-                    W.scan.sum.p, table_cap_, dstat + 1};
+                    W.scan.sum.p, table_cap_, status + kTreeTable};
       if (generic_)
         shoot_f32_batch<true><<<148 * 64, kShootBatchThreads, 0, s>>>(bs, lp, d_verts_.p);
       else
@@ -788,12 +689,18 @@ class BatchMaker {
   }
 
   bool check(int* st) {
-    int h[2] = {0, 0};
-    IRSB_CKR(cudaMemcpyAsync(h, tree_.dstat.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    int* h = tree_.h_status.p;
+    IRSB_CKR(cudaMemcpyAsync(h, tree_.status.p, kTreeOff * sizeof(int), cudaMemcpyDeviceToHost, stream_));
     IRSB_CKR(cudaStreamSynchronize(stream_));
-    *st = h[1];
-    if (h[1] & (kErrNeighborOverflow | kErrSameLevelOverflow | kErrDiffLevelOverflow | kErrNearOverflow)) {
-      std::cerr << "Error. Tree list overflow in the batch (code " << h[1] << ").\n";
+    if (h[kTreeBarrier]) {
+      std::cerr << "Error. The batch's tree build or expansions did not finish.\n";
+      return false;
+    }
+    *st = h[kTreeErr] | h[kTreeTable];
+    // an unfinished build leaves leaves with too many stars: the batch is built again
+    if (!(*st & (kErrNodeOverflow | kErrLevelOverflow))) *st |= h[kTreeNear];
+    if (*st & (kErrNeighborOverflow | kErrSameLevelOverflow | kErrDiffLevelOverflow | kErrNearOverflow)) {
+      std::cerr << "Error. Tree list overflow in the batch (code " << *st << ").\n";
       return false;
     }
     return true;

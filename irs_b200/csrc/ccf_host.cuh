@@ -197,7 +197,9 @@ class CCF {
     }
     // ---- tree and expansions (include/ccf.cuh:732-904)
     root_half_length = T((rectangular ? std::max(corner.re, corner.im) : cabs_(corner)) * 1.1);
-    if (!build_tree<T>(tree_, d_stars_.p, n, root_half_length, s)) return false;
+    if (!build_tree<T>(tree_, d_stars_.p, n, root_half_length, leaves_.pos, leaves_.node, s,
+                       [](long long) { return true; }))
+      return false;
     tree_levels = tree_.levels;
     expansion_order = static_cast<int>(std::ceil(2 * std::log2(theta_star) + tree_levels -
                                                  std::log2(root_half_length) - std::log2(alpha_error)));
@@ -209,12 +211,16 @@ class CCF {
       std::cerr << "Error. Maximum allowed expansion order is " << kMaxOrder << "\n";
       return false;
     }
-    if (!compute_fmm<T>(fmm_, tree_, d_stars_.p, expansion_order, s)) return false;
+    if (!fmm_reserve(fmm_, tree_.num_nodes, expansion_order, s) ||
+        !compute_fmm<T>(fmm_, tree_, d_stars_.p, tree_.num_nodes, kFmmBlockNodes, s))
+      return false;
     if (!build_leaves<T>(leaves_, tree_, fmm_, d_stars_.p, double(theta_star), s)) return false;
     stars_out.resize(n);
     IRSB_CKR(cudaMemcpyAsync(stars_out.data(), d_stars_.p, size_t(n) * sizeof(StarRec<T>), cudaMemcpyDeviceToHost,
                              s));
+    if (!fetch_leaf_status(tree_, s)) return false;
     IRSB_CKR(cudaStreamSynchronize(s));
+    if (!leaves_ok(tree_)) return false;
     std::vector<double2> pos(n);  // star positions in tree order, for the sums over all stars
     for (int i = 0; i < n; i++) pos[i] = make_double2(double(stars_out[i].x), double(stars_out[i].y));
     if (!d_spos_.alloc_exact(n)) return false;

@@ -238,29 +238,16 @@ struct ScanScratch {
   DevVec<long long> sum;
 };
 
-// out[i] = sum_{j<i} in[j]; *d_sum (device) receives the grand total.
+// out[i] = sum_{j<i} in[j] over the *dn (read on the device, at most n_cap)
+// values of `in`; *sum (device; sc.sum when not given) receives the grand
+// total. The scratch must already hold the blocks for n_cap (scan_reserve).
 template <typename In>
-bool exclusive_scan(const In* in, long long n, long long* out, ScanScratch& sc, cudaStream_t s) {
-  long long nb = (n + kScanTile - 1) / kScanTile;
-  if (nb < 1) nb = 1;
-  if (!sc.totals.reserve(size_t(nb), s)) return false;
-  if (!sc.sum.reserve(1, s)) return false;
-  scan_block_totals<In><<<unsigned(nb), kScanBlock, 0, s>>>(in, n, nullptr, sc.totals.p);
-  scan_totals_single<<<1, kScanBlock, 0, s>>>(sc.totals.p, nb, sc.sum.p);
-  scan_block_apply<In><<<unsigned(nb), kScanBlock, 0, s>>>(in, n, nullptr, sc.totals.p, out);
-  return IRSB_CK(cudaGetLastError());
-}
-
-// The same with the element count read on the device from *dn (at most
-// n_cap), for work whose size the host does not know (graph-captured
-// pipelines). The scratch must already hold the blocks for n_cap.
-template <typename In>
-bool exclusive_scan_dev(const In* in, const int* dn, long long n_cap, long long* out, ScanScratch& sc,
-                        cudaStream_t s) {
+bool exclusive_scan_dev(const In* in, const int* dn, long long n_cap, long long* out, ScanScratch& sc, cudaStream_t s,
+                        long long* sum = nullptr) {
   long long nb = (n_cap + kScanTile - 1) / kScanTile;
   if (nb < 1) nb = 1;
   scan_block_totals<In><<<unsigned(nb), kScanBlock, 0, s>>>(in, n_cap, dn, sc.totals.p);
-  scan_totals_single<<<1, kScanBlock, 0, s>>>(sc.totals.p, nb, sc.sum.p);
+  scan_totals_single<<<1, kScanBlock, 0, s>>>(sc.totals.p, nb, sum ? sum : sc.sum.p);
   scan_block_apply<In><<<unsigned(nb), kScanBlock, 0, s>>>(in, n_cap, dn, sc.totals.p, out);
   return IRSB_CK(cudaGetLastError());
 }

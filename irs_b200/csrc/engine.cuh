@@ -261,11 +261,25 @@ class MapMaker {
 
   // Tree -> expansions -> leaf records -> shoot on the resident star field,
   // timed with CUDA events (t_pipeline, t_shoot, t_lattice, t_deposit).
+  // One host synchronisation before the end: the tree's depth (the expansion
+  // order follows from it) and the number of lattice tiles are read together,
+  // after the build and the leaves' rectangles.
   bool device_pipeline() {
     const int n = prm.num_stars;
     IRSB_CKR(cudaEventRecord(ev0_, stream_));
-    if (!build_tree<T>(tree_, d_stars_.p, n, prm.root_half_length, stream_)) return false;
-    launches += tree_.launches;
+    const ShootParams lat = shoot_params(!IS_IRS);
+    const auto band = band_rows();
+    // rays: rows [lo, hi); cells: rows [lo, hi) need corner rows [lo, hi]
+    const long long jlo = band.first, jhi = IS_IRS ? band.second : band.second + 1;
+    auto rects = [&](long long cap) {
+      return lattice_rects<T>(tiles_, leaves_, tree_, cap, lat.base_x, lat.base_y, lat.rhs_x, lat.rhs_y, lat.nx,
+                              lat.ny, jlo, jhi, stream_);
+    };
+    if (!build_tree<T>(tree_, d_stars_.p, n, prm.root_half_length, leaves_.pos, leaves_.node, stream_, rects))
+      return false;
+    launches += tree_.launches + 4;
+    const unsigned long long* st = tiles_.h_stat.p;
+    mean_near = st[kLatPoints] > 0 ? double(st[kLatNear]) / double(st[kLatPoints]) : 0;
     prm.tree_levels = tree_.levels;
     prm.expansion_order =
         prm.expansion_order_override > 0 ? prm.expansion_order_override : expansion_order_of(prm);
@@ -277,16 +291,21 @@ class MapMaker {
       std::cerr << "Error. Maximum allowed expansion order is " << kMaxOrder << "\n";
       return false;
     }
-    if (!compute_fmm<T>(fmm_, tree_, d_stars_.p, prm.expansion_order, stream_)) return false;
-    launches += 2LL * (tree_.levels + 1) + std::max(0, tree_.levels - 1);
+    if (!fmm_reserve(fmm_, tree_.num_nodes, prm.expansion_order, stream_) ||
+        !compute_fmm<T>(fmm_, tree_, d_stars_.p, tree_.num_nodes, kFmmBlockNodes, stream_))
+      return false;
     const SmoothFold fold{smooth_folded() ? 1 : 0, double(prm.kappa_star), double(prm.corner.re),
                           double(prm.corner.im), 0.318309886183790671537767526745028724, prm.taylor_smooth, nullptr};
     if (!build_leaves<T>(leaves_, tree_, fmm_, d_stars_.p, double(prm.theta_star), stream_, fold)) return false;
-    launches += 6;
     num_leaves = leaves_.n;
+    if (!lattice_table<T>(tiles_, leaves_, tree_, stream_)) return false;
+    launches += 4;
+    num_tiles = tiles_.total;
     if (!shoot()) return false;
+    if (!fetch_leaf_status(tree_, stream_)) return false;
     IRSB_CKR(cudaEventRecord(ev2_, stream_));
     IRSB_CKR(cudaEventSynchronize(ev2_));
+    if (!leaves_ok(tree_)) return false;
     float ms_shoot = 0, ms_all = 0, ms_lat = 0, ms_dep = 0;
     IRSB_CKR(cudaEventElapsedTime(&ms_shoot, ev1_, ev2_));
     IRSB_CKR(cudaEventElapsedTime(&ms_all, ev0_, ev2_));
@@ -630,14 +649,6 @@ class MapMaker {
     have_parities = par;
     ShootParams sp = shoot_params(!IS_IRS);
     const auto band = band_rows();
-    // rays: rows [lo, hi); cells: rows [lo, hi) need corner rows [lo, hi]
-    const long long jlo = band.first, jhi = IS_IRS ? band.second : band.second + 1;
-    if (!build_lattice_tiles<T>(tiles_, leaves_, tree_, sp.base_x, sp.base_y, sp.rhs_x, sp.rhs_y, sp.nx, sp.ny, jlo,
-                                jhi, stream_))
-      return false;
-    num_tiles = tiles_.total;
-    launches += 4;
-    if (!mean_near_count()) return false;
     if (IS_IRS) {
       if (!d_pix_.alloc_exact(npix)) return false;
       if (par && (!d_pmin_.alloc_exact(npix) || !d_psad_.alloc_exact(npix))) return false;
@@ -704,27 +715,6 @@ class MapMaker {
         IRSB_LAUNCH_CK("ipm_finalize");
       }
     }
-    return true;
-  }
-
-  // Mean near-field size over the lattice points (algorithmic work per point).
-  bool mean_near_count() {
-    std::vector<int4> r(leaves_.n);
-    std::vector<int> nn(leaves_.n);
-    if (leaves_.n == 0) {
-      mean_near = 0;
-      return true;
-    }
-    IRSB_CKR(cudaMemcpyAsync(r.data(), tiles_.rect.p, r.size() * sizeof(int4), cudaMemcpyDeviceToHost, stream_));
-    IRSB_CKR(cudaMemcpyAsync(nn.data(), leaves_.nnear.p, nn.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    IRSB_CKR(cudaStreamSynchronize(stream_));
-    double acc = 0, pts = 0;
-    for (int l = 0; l < leaves_.n; l++) {
-      double c = double(std::max(0, r[l].y - r[l].x)) * double(std::max(0, r[l].w - r[l].z));
-      acc += c * nn[l];
-      pts += c;
-    }
-    mean_near = pts > 0 ? acc / pts : 0;
     return true;
   }
 

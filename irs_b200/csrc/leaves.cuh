@@ -68,16 +68,14 @@ constexpr int kTileY = 32;
 struct LeafSet {
   int n = 0;
   DevVec<double2> smooth0;  // folded smooth sheet at the leaf centres (when folded)
-  DevVec<int> flag;
-  DevVec<long long> pos;
-  DevVec<int> node;
+  DevVec<long long> pos;    // per node: leaves before it (the build numbers them)
+  DevVec<int> node;         // per leaf: its node
   DevVec<double> cx, cy, hl;
   DevVec<int> nnear;
   DevVec<double4> near64;
   DevVec<float4> near32;
   DevVec<double2> coef64;
   DevVec<float2> coef32;
-  ScanScratch scan;
 };
 
 // Lattice partition for one lattice (rays or vertices).
@@ -86,9 +84,14 @@ struct LatticeTiles {
   DevVec<long long> tiles;
   DevVec<long long> tile_off;  // [n + 1]
   DevVec<int4> table;          // per tile: leaf, i0, j0, (ni << 16) | nj
+  DevVec<unsigned long long> stat;    // LatticeStat
+  HostVec<unsigned long long> h_stat;  // pinned copy
   long long total = 0;
   ScanScratch scan;
 };
+// Lattice points in leaves, and those weighted with their leaf's near-field
+// star count (the tile total is in `scan.sum`, copied to the third word).
+enum LatticeStat : int { kLatPoints = 0, kLatNear = 1, kLatTiles = 2, kLatWords = 3 };
 
 // kTableLanes consecutive lanes per leaf write the table entries of its tiles
 // (row-major over the leaf's rectangle), lane q entries q, q + kTableLanes, ...
@@ -98,14 +101,14 @@ struct LatticeTiles {
 // (1.4e3 leaves, 2.5e5 tiles, B200); now 17 us.
 constexpr int kTableLanes = 8;
 __global__ void leaf_tile_table(int nleaves, const int* __restrict__ dn, const int4* __restrict__ rect,
-                                const long long* __restrict__ tile_off, int tx, int ty, int4* __restrict__ table,
-                                long long table_cap, int* __restrict__ err) {
+                                const long long* __restrict__ tile_off, const long long* __restrict__ total, int tx,
+                                int ty, int4* __restrict__ table, long long table_cap, int* __restrict__ err) {
   if (dn) nleaves = *dn;
   const int sub = threadIdx.x % kTableLanes;
   for (int l = (blockIdx.x * blockDim.x + threadIdx.x) / kTableLanes; l < nleaves;
        l += gridDim.x * blockDim.x / kTableLanes) {
     const int4 r = rect[l];
-    const long long t = tile_off[l], t_end = tile_off[l + 1];
+    const long long t = tile_off[l], t_end = l + 1 < nleaves ? tile_off[l + 1] : *total;
     if (t == t_end) continue;
     if (t_end > table_cap) {  // more tiles than the table holds
       if (sub == 0) atomicOr(err, kErrTableOverflow);
@@ -119,17 +122,6 @@ __global__ void leaf_tile_table(int nleaves, const int* __restrict__ dn, const i
       table[t + k] = make_int4(l, i0, j0, (ni << 16) | nj);
     }
   }
-}
-
-__global__ void leaf_flags(int n, const int* __restrict__ dn, const int* __restrict__ child0, int* flag) {
-  if (dn) n = *dn;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) flag[k] = child0[k] < 0;
-}
-__global__ void leaf_compact(int n, const int* __restrict__ dn, const int* __restrict__ flag,
-                             const long long* __restrict__ pos, int* node) {
-  if (dn) n = *dn;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    if (flag[k]) node[pos[k]] = k;
 }
 
 // One warp per leaf: gather the near field and the expansion coefficients.
@@ -150,7 +142,7 @@ __global__ void leaf_build(int nleaves, const int* __restrict__ dn, int p, doubl
                            const int* __restrict__ n_nbr, const StarRec<T>* __restrict__ stars,
                            const double2* __restrict__ loc, double* lcx, double* lcy, double* lhl, int* nnear,
                            double4* near64, float4* near32, double2* coef64, float2* coef32, int* leaf_rid,
-                           int* dstat, SmoothFold fold = SmoothFold{0, 0, 0, 0, 0, 0, nullptr}) {
+                           int* err, SmoothFold fold = SmoothFold{0, 0, 0, 0, 0, 0, nullptr}) {
   if (dn) nleaves = *dn;
   int lane = threadIdx.x & 31;
   int warps = (gridDim.x * blockDim.x) >> 5;
@@ -184,7 +176,7 @@ __global__ void leaf_build(int nleaves, const int* __restrict__ dn, int p, doubl
       out += c;
     }
     if (out > kMaxStarsDirect) {
-      if (lane == 0) atomicOr(&dstat[0], kErrNearOverflow);
+      if (lane == 0) atomicOr(err, kErrNearOverflow);
       out = kMaxStarsDirect;
     }
     // zero the unused slots so that any over-read is harmless
@@ -251,11 +243,17 @@ __device__ __forceinline__ long long lattice_lower_bound(double base, double rhs
   return lo;
 }
 
-__global__ void leaf_rects(int nleaves, const int* __restrict__ leaf_node, const double* __restrict__ lox,
-                           const double* __restrict__ hix, const double* __restrict__ loy,
-                           const double* __restrict__ hiy, double base_x, double base_y, double rhs_x, double rhs_y,
-                           long long nx, long long ny, long long jlo, long long jhi, int tx, int ty, int4* rect,
-                           long long* tiles) {
+// Rectangle and tile count of every leaf (count on the device), and the sums
+// of LatticeStat over the leaves.
+__global__ void leaf_rects(const int* __restrict__ dn, const int* __restrict__ leaf_node,
+                           const double* __restrict__ lox, const double* __restrict__ hix,
+                           const double* __restrict__ loy, const double* __restrict__ hiy,
+                           const int* __restrict__ scnt, const int* __restrict__ nbr, const int* __restrict__ n_nbr,
+                           double base_x, double base_y, double rhs_x, double rhs_y, long long nx, long long ny,
+                           long long jlo, long long jhi, int tx, int ty, int4* rect, long long* tiles,
+                           unsigned long long* __restrict__ stat) {
+  const int nleaves = *dn;
+  unsigned long long pts = 0, near = 0;
   for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nleaves; l += gridDim.x * blockDim.x) {
     int k = leaf_node[l];
     long long i0 = lattice_lower_bound(base_x, rhs_x, nx, lox[k]);
@@ -268,6 +266,20 @@ __global__ void leaf_rects(int nleaves, const int* __restrict__ leaf_node, const
     rect[l] = make_int4(int(i0), int(i1), int(j0), int(j1));
     long long ni = i1 - i0, nj = j1 - j0;
     tiles[l] = (ni > 0 && nj > 0) ? ((ni + tx - 1) / tx) * ((nj + ty - 1) / ty) : 0;
+    if (ni > 0 && nj > 0) {
+      int c = scnt[k];
+      for (int q = 0; q < n_nbr[k]; q++) c += scnt[nbr[k * kMaxNeighbors + q]];
+      pts += (unsigned long long)(ni * nj);
+      near += (unsigned long long)(ni * nj) * min(c, kMaxStarsDirect);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    pts += __shfl_down_sync(0xffffffffu, pts, o);
+    near += __shfl_down_sync(0xffffffffu, near, o);
+  }
+  if ((threadIdx.x & 31) == 0 && pts) {
+    atomicAdd(&stat[kLatPoints], pts);
+    atomicAdd(&stat[kLatNear], near);
   }
 }
 
@@ -310,62 +322,82 @@ __global__ void leaf_rects_batch(const int* __restrict__ dn, const int* __restri
   }
 }
 
+// Leaf records of the tree (whose build numbered the leaves) on stream s: no
+// synchronisation. An overflowing near field is reported in the tree's status
+// (kTreeNear, see leaves_ok).
 template <typename T>
 bool build_leaves(LeafSet& L, TreeDev<T>& t, FmmDev& f, const StarRec<T>* stars, double theta, cudaStream_t s,
                   SmoothFold fold = SmoothFold{0, 0, 0, 0, 0, 0, nullptr}) {
-  int n = t.num_nodes;
-  if (!L.flag.alloc_exact(n) || !L.pos.alloc_exact(n + 1)) return false;
-  int blocks = std::max(1, std::min(ceil_div(n, 256), 148 * 8));
-  leaf_flags<<<blocks, 256, 0, s>>>(n, nullptr, t.child0.p, L.flag.p);
-  if (!exclusive_scan<int>(L.flag.p, n, L.pos.p, L.scan, s)) return false;
-  long long nl = 0;
-  IRSB_CKR(cudaMemcpyAsync(&nl, L.scan.sum.p, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  IRSB_CKR(cudaStreamSynchronize(s));
-  L.n = int(nl);
-  if (!L.node.alloc_exact(L.n) || !L.cx.alloc_exact(L.n) || !L.cy.alloc_exact(L.n) || !L.hl.alloc_exact(L.n) ||
-      !L.nnear.alloc_exact(L.n) || !L.near64.alloc_exact((size_t)L.n * kMaxStarsDirect) ||
-      !L.near32.alloc_exact((size_t)L.n * kMaxStarsDirect) || !L.coef64.alloc_exact((size_t)L.n * kMaxOrder) ||
-      !L.coef32.alloc_exact((size_t)L.n * kMaxOrder))
+  L.n = t.num_leaves;
+  if (!L.cx.alloc_exact(L.n) || !L.cy.alloc_exact(L.n) || !L.hl.alloc_exact(L.n) || !L.nnear.alloc_exact(L.n) ||
+      !L.near64.alloc_exact((size_t)L.n * kMaxStarsDirect) || !L.near32.alloc_exact((size_t)L.n * kMaxStarsDirect) ||
+      !L.coef64.alloc_exact((size_t)L.n * kMaxOrder) || !L.coef32.alloc_exact((size_t)L.n * kMaxOrder))
     return false;
   if (fold.on) {
     if (!L.smooth0.alloc_exact(L.n)) return false;
     fold.smooth0 = L.smooth0.p;
   }
-  leaf_compact<<<blocks, 256, 0, s>>>(n, nullptr, L.flag.p, L.pos.p, L.node.p);
-  IRSB_LAUNCH_CK("leaf_compact");
-  IRSB_CKR(cudaMemsetAsync(t.dstat.p, 0, 2 * sizeof(int), s));
   int lb = std::max(1, std::min(ceil_div(L.n, 8), 148 * 16));
   leaf_build<T><<<lb, 256, 0, s>>>(L.n, nullptr, f.p, theta, nullptr, nullptr, L.node.p, t.cx.p, t.cy.p, t.hl.p, t.sbeg.p, t.scnt.p, t.nbr.p,
                                    t.n_nbr.p, stars, f.loc.p, L.cx.p, L.cy.p, L.hl.p, L.nnear.p, L.near64.p,
-                                   L.near32.p, L.coef64.p, L.coef32.p, nullptr, t.dstat.p, fold);
+                                   L.near32.p, L.coef64.p, L.coef32.p, nullptr, t.status.p + kTreeNear, fold);
   IRSB_LAUNCH_CK("leaf_build");
-  int st = 0;
-  IRSB_CKR(cudaMemcpyAsync(&st, t.dstat.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  IRSB_CKR(cudaStreamSynchronize(s));
-  if (st) {
+  return true;
+}
+
+// Fetches the tree's status after the expansions and leaf records on stream s;
+// leaves_ok reads it once the stream is synchronised.
+template <typename T>
+bool fetch_leaf_status(TreeDev<T>& t, cudaStream_t s) {
+  return IRSB_CK(cudaMemcpyAsync(t.h_status.p, t.status.p, kTreeOff * sizeof(int), cudaMemcpyDeviceToHost, s));
+}
+template <typename T>
+bool leaves_ok(const TreeDev<T>& t) {
+  if (t.h_status.p[kTreeBarrier]) {
+    std::fprintf(stderr, "Error. The expansions did not finish.\n");
+    return false;
+  }
+  if (t.h_status.p[kTreeNear]) {
     std::fprintf(stderr, "Error. A leaf's near field holds more than %d stars.\n", kMaxStarsDirect);
     return false;
   }
   return true;
 }
 
+// The leaves' rectangles on a lattice and the offsets of their tiles, from the
+// tree as it is on the device (at most cap leaves): no synchronisation. The
+// counts reach W.h_stat when the stream is next synchronised.
 template <typename T>
-bool build_lattice_tiles(LatticeTiles& W, const LeafSet& L, TreeDev<T>& t, double base_x, double base_y,
-                         double rhs_x, double rhs_y, long long nx, long long ny, long long jlo, long long jhi,
-                         cudaStream_t s) {
-  if (!W.rect.alloc_exact(L.n) || !W.tiles.alloc_exact(L.n) || !W.tile_off.alloc_exact(L.n + 1)) return false;
-  int blocks = std::max(1, std::min(ceil_div(L.n, 256), 148 * 8));
-  leaf_rects<<<blocks, 256, 0, s>>>(L.n, L.node.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p, base_x, base_y, rhs_x, rhs_y,
-                                    nx, ny, jlo, jhi, kTileX, kTileY, W.rect.p, W.tiles.p);
+bool lattice_rects(LatticeTiles& W, const LeafSet& L, TreeDev<T>& t, long long cap, double base_x, double base_y,
+                   double rhs_x, double rhs_y, long long nx, long long ny, long long jlo, long long jhi,
+                   cudaStream_t s) {
+  if (!W.rect.alloc_exact(cap) || !W.tiles.alloc_exact(cap) || !W.tile_off.alloc_exact(cap + 1) ||
+      !W.stat.alloc_exact(kLatWords) || !W.h_stat.alloc(kLatWords) || !scan_reserve(W.scan, cap, s))
+    return false;
+  const int* dn = t.status.p + kTreeLeaves;
+  IRSB_CKR(cudaMemsetAsync(W.stat.p, 0, kLatWords * sizeof(unsigned long long), s));
+  const int blocks = std::max(1, std::min(ceil_div(cap, 256), 148 * 8));
+  leaf_rects<<<blocks, 256, 0, s>>>(dn, L.node.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p, t.scnt.p, t.nbr.p, t.n_nbr.p,
+                                    base_x, base_y, rhs_x, rhs_y, nx, ny, jlo, jhi, kTileX, kTileY, W.rect.p,
+                                    W.tiles.p, W.stat.p);
   IRSB_LAUNCH_CK("leaf_rects");
-  if (!exclusive_scan<long long>(W.tiles.p, L.n, W.tile_off.p, W.scan, s)) return false;
-  IRSB_CKR(cudaMemcpyAsync(W.tile_off.p + L.n, W.scan.sum.p, sizeof(long long), cudaMemcpyDeviceToDevice, s));
-  IRSB_CKR(cudaMemcpyAsync(&W.total, W.scan.sum.p, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  IRSB_CKR(cudaStreamSynchronize(s));
+  if (!exclusive_scan_dev<long long>(W.tiles.p, dn, cap, W.tile_off.p, W.scan, s,
+                                     reinterpret_cast<long long*>(W.stat.p + kLatTiles)))
+    return false;
+  IRSB_CKR(cudaMemcpyAsync(W.h_stat.p, W.stat.p, kLatWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+  return true;
+}
+
+// The tile table of the lattice counted by lattice_rects (after the
+// synchronisation).
+template <typename T>
+bool lattice_table(LatticeTiles& W, const LeafSet& L, TreeDev<T>& t, cudaStream_t s) {
+  W.total = (long long)W.h_stat.p[kLatTiles];
   if (!W.table.alloc_exact(std::max<long long>(W.total, 1))) return false;
-  blocks = std::max(1, std::min(ceil_div((long long)L.n * kTableLanes, 256), 148 * 8));
-  leaf_tile_table<<<blocks, 256, 0, s>>>(L.n, nullptr, W.rect.p, W.tile_off.p, kTileX, kTileY, W.table.p, W.total,
-                                         t.dstat.p + 1);
+  const int blocks = std::max(1, std::min(ceil_div((long long)L.n * kTableLanes, 256), 148 * 8));
+  leaf_tile_table<<<blocks, 256, 0, s>>>(L.n, nullptr, W.rect.p, W.tile_off.p,
+                                         reinterpret_cast<const long long*>(W.stat.p + kLatTiles), kTileX, kTileY,
+                                         W.table.p, W.total, t.status.p + kTreeTable);
   IRSB_LAUNCH_CK("leaf_tile_table");
   return true;
 }

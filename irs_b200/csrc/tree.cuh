@@ -33,25 +33,12 @@
 
 namespace irsb {
 
-// Node range of one level: [beg, end) given by the host, or read on the device
-// from off[lvl], off[lvl + 1] when off is set (graph-captured builds, whose
-// level sizes are not known to the host).
-struct LevelRange {
-  const int* off = nullptr;
-  int lvl = 0;
-  __device__ __forceinline__ void get(int& beg, int& end) const {
-    if (off) {
-      beg = off[lvl];
-      end = off[lvl + 1];
-    }
-  }
-};
-
 template <typename T>
 struct TreeDev {
   int cap = 0;
   int num_nodes = 0;
   int levels = 0;  // number of levels - 1 (the reference's tree_levels)
+  int num_leaves = 0;
   std::vector<int> level_off;  // host copy, size levels + 2
   DevVec<T> cx, cy, hl;
   DevVec<int> level, parent, child0, sbeg, scnt;
@@ -61,26 +48,13 @@ struct TreeDev {
   DevVec<int> dil, n_dil;  // [cap][kMaxDiffLevelIL]
   DevVec<double> lox, hix, loy, hiy;
   // scratch
-  DevVec<int> split, cnt_near;
-  DevVec<long long> rank;
-  DevVec<int> dstat;  // [0] max near count, [1] error bits
-  ScanScratch scan;
+  DevVec<int> split, rank;
+  DevVec<int> cta;          // per-CTA counts of the build
+  DevVec<int> status;       // TreeStatus, then the level offsets (the FMM reads them there)
+  DevVec<unsigned long long> words;  // grid barriers of the build and of the expansions
   DevVec<StarRec<T>> tmp_stars, star_backup;
-  DevVec<int> d_off, d_lvl_n, d_stop;  // level offsets and sizes on the device
-  DevVec<int> chunk_cnt;               // per-chunk key counts of the wide partition
-  long long launches = 0;              // kernels the last build launched
-};
-
-template <typename T>
-struct NodeView {
-  const T* cx;
-  const T* cy;
-  const T* hl;
-  const int* child0;
-  const int* sbeg;
-  const int* scnt;
-  const int* nbr;
-  const int* n_nbr;
+  HostVec<int> h_status;    // pinned copy of `status`
+  long long launches = 0;   // kernels the last build launched
 };
 
 template <typename T>
@@ -106,87 +80,41 @@ bool tree_reserve(TreeDev<T>& t, int want, cudaStream_t s) {
   return true;
 }
 
-template <typename T>
-__global__ void tree_init_root(T* cx, T* cy, T* hl, int* level, int* parent, int* child0, int* sbeg, int* scnt,
-                               int* rid, int* n_nbr, int* n_sil, int* n_dil, double* lox, double* hix, double* loy,
-                               double* hiy, T root_hl, int nstars) {
-  rid[0] = 0;
-  cx[0] = T(0);
-  cy[0] = T(0);
-  hl[0] = root_hl;
-  level[0] = 0;
-  parent[0] = -1;
-  child0[0] = -1;
-  sbeg[0] = 0;
-  scnt[0] = nstars;
-  n_nbr[0] = n_sil[0] = n_dil[0] = 0;
-  lox[0] = -INFINITY;
-  hix[0] = INFINITY;
-  loy[0] = -INFINITY;
-  hiy[0] = INFINITY;
-}
-
-// Stars of a node and its neighbours; split flag; level maximum.
-__global__ void tree_near_count(int beg, int end, LevelRange lr, const int* __restrict__ scnt,
-                                const int* __restrict__ nbr, const int* __restrict__ n_nbr, int* __restrict__ split,
-                                int* __restrict__ dstat) {
-  lr.get(beg, end);
-  int local_max = 0;
-  for (int k = beg + blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x) {
-    int c = scnt[k];
-    int nn = n_nbr[k];
-    for (int j = 0; j < nn; j++) c += scnt[nbr[k * kMaxNeighbors + j]];
-    split[k - beg] = c > kMaxStarsDirect ? 1 : 0;
-    local_max = max(local_max, c);
-  }
-  for (int o = 16; o > 0; o >>= 1) local_max = max(local_max, __shfl_down_sync(0xffffffffu, local_max, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(&dstat[0], local_max);
-}
+// Words of TreeDev::status: the build's outcome, then off[0 .. kMaxLevels + 1]
+// (nodes of level l are [off[l], off[l + 1]); the offsets past the last level
+// all hold the number of nodes).
+enum TreeStatus : int {
+  kTreeErr = 0,        // DeviceError bits
+  kTreeBarrier = 1,    // a grid barrier gave up
+  kTreeLevels = 2,     // the deepest level
+  kTreeLeaves = 3,     // leaves
+  kTreeNear = 4,       // a leaf's near field overflowed (leaf_build, build_leaves)
+  kTreeTable = 5,      // the tile table overflowed (leaf_tile_table)
+  kTreeOff = 8,
+  kTreeStatusWords = kTreeOff + kMaxLevels + 2,
+};
+// Grid barriers of a build: at most four per level, one for the leaves; then
+// those of the expansions (fmm.cuh).
+constexpr int kTreeBarriers = 4 * kMaxLevels + 8;
+constexpr int kFmmBarriers = 2 * kMaxLevels + 4;
 
 template <typename T>
-__global__ void tree_make_children(int beg, int end, int child_base, LevelRange lr, const int* __restrict__ stop,
-                                   const int* __restrict__ split, const long long* __restrict__ rank, T* cx, T* cy,
-                                   T* hl, int* level, int* parent, int* child0, int* sbeg, int* scnt, int* rid,
-                                   int* n_nbr, int* n_sil, int* n_dil, double* lox, double* hix, double* loy,
-                                   double* hiy) {
-  if (lr.off) {
-    lr.get(beg, end);
-    child_base = end;
-  }
-  const bool halt = stop && *stop;
-  for (int k = beg + blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x) {
-    if (halt || !split[k - beg]) {
-      child0[k] = -1;
-      continue;
-    }
-    int c0 = child_base + 4 * int(rank[k - beg]);
-    child0[k] = c0;
-    T h = hl[k] / 2;
-    T pcx = cx[k], pcy = cy[k];
-    const T ox[4] = {T(1), T(-1), T(-1), T(1)};
-    const T oy[4] = {T(1), T(1), T(-1), T(-1)};
-    double plox = lox[k], phix = hix[k], ploy = loy[k], phiy = hiy[k];
-    for (int q = 0; q < 4; q++) {
-      int c = c0 + q;
-      cx[c] = pcx + h * ox[q];
-      cy[c] = pcy + h * oy[q];
-      hl[c] = h;
-      level[c] = level[k] + 1;
-      parent[c] = k;
-      rid[c] = rid[k];
-      child0[c] = -1;
-      sbeg[c] = sbeg[k];
-      scnt[c] = 0;
-      n_nbr[c] = n_sil[c] = n_dil[c] = 0;
-      // x >= pcx for q = 0, 3; y >= pcy for q = 0, 1
-      bool right = (q == 0 || q == 3), top = (q == 0 || q == 1);
-      lox[c] = right ? double(pcx) : plox;
-      hix[c] = right ? phix : double(pcx);
-      loy[c] = top ? double(pcy) : ploy;
-      hiy[c] = top ? phiy : double(pcy);
-    }
-  }
-}
+struct TreeBuild {
+  T *cx, *cy, *hl;
+  int *level, *parent, *child0, *sbeg, *scnt, *rid, *nbr, *n_nbr, *sil, *n_sil, *dil, *n_dil;
+  double *lox, *hix, *loy, *hiy;
+  int *split, *rank;  // per node of the level: split flag; rank among the CTA's split nodes
+  int* cta;           // [3 + 4 * kShareNodes][grid] counts per CTA
+  int* status;
+  unsigned long long* words;
+  long long* leaf_pos;  // per node: leaves before it
+  int* leaf_node;       // per leaf: its node
+  StarRec<T>*stars, *tmp;
+  int nroots, nstars, cap, nlev;
+  T root_hl;                  // one root over all stars, or
+  const T* root_hls;          // per root: half length
+  const long long* star_off;  // per root: first star (nroots + 1 values)
+};
 
 template <typename T>
 __device__ __forceinline__ int star_quadrant(T x, T y, T cx, T cy) {
@@ -196,485 +124,564 @@ __device__ __forceinline__ int star_quadrant(T x, T y, T cx, T cy) {
   return 3;
 }
 
-// Blocks of NT threads stride over the level's nodes; split nodes with stars
-// partition their star range into the 4 child ranges, keeping the relative
-// order of stars (stable). The top levels, a few nodes holding many stars each,
-// take NT = 1024 (a quarter of the block-synchronised chunks), the rest 256.
-template <typename T, int NT = 256>
-__global__ void __launch_bounds__(NT) tree_partition_stars(int beg, int end, LevelRange lr,
-                                                            const int* __restrict__ stop,
-                                                            const int* __restrict__ split,
-                                                            const T* __restrict__ cx, const T* __restrict__ cy,
-                                                            const int* __restrict__ child0, int* sbeg, int* scnt,
-                                                            StarRec<T>* __restrict__ stars,
-                                                            StarRec<T>* __restrict__ tmp) {
-  lr.get(beg, end);
-  if (stop && *stop) return;
-  __shared__ int cnt[4];
-  __shared__ int warp_cnt[NT / 32][4];
-  __shared__ int base[4];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int k = beg + blockIdx.x; k < end; k += gridDim.x) {
-    if (!split[k - beg]) continue;  // uniform over the block
-    const int b = sbeg[k], n = scnt[k];
-    const int c0 = child0[k];
-    if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const T pcx = cx[k], pcy = cy[k];
-    int lc[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      StarRec<T> st = stars[b + i];
-      lc[star_quadrant(st.x, st.y, pcx, pcy)]++;
-    }
-    for (int q = 0; q < 4; q++)
-      if (lc[q]) atomicAdd(&cnt[q], lc[q]);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = b;
-      for (int q = 0; q < 4; q++) {
-        base[q] = acc;
-        sbeg[c0 + q] = acc;
-        scnt[c0 + q] = cnt[q];
-        acc += cnt[q];
+// set_neighbors (tree_node.cuh:183-267) for node k (of a level >= 1) by one
+// warp: lane q examines candidate q in the order of the reference's loops (the
+// 4 siblings, then for each of the parent's neighbours either the neighbour
+// itself, a leaf, or its 4 children), and each list takes its candidates in
+// that order through a ballot prefix, so the lists are those of one thread
+// walking the loops. Returns the stars of the node and its neighbours.
+template <typename T>
+__device__ __forceinline__ int tree_node_lists(const TreeBuild<T>& b, int k, int lane, int& err) {
+  const unsigned below = (1u << lane) - 1u;
+  const int p = b.parent[k];
+  const T h = b.hl[k], x = b.cx[k], y = b.cy[k];
+  const int pc0 = b.child0[p];
+  const int nq = 4 + 4 * b.n_nbr[p];
+  int nn = 0, ns = 0, nd = 0, near = 0;
+  for (int q0 = 0; q0 < nq; q0 += 32) {
+    const int q = q0 + lane;
+    int cat = 0, c = -1, cnt = 0;  // 1 neighbour, 2 same-level interaction, 3 different-level interaction
+    if (q < 4) {
+      c = pc0 + q;
+      cnt = b.scnt[c];
+      if (cnt != 0 && c != k) cat = 1;
+    } else if (q < nq) {
+      const int i = (q - 4) >> 2, j = (q - 4) & 3;
+      const int nb = b.nbr[p * kMaxNeighbors + i];
+      cnt = b.scnt[nb];
+      if (cnt != 0) {
+        const int nc0 = b.child0[nb];
+        if (nc0 < 0) {
+          if (j == 0) {
+            c = nb;
+            cat = (double(xfabs(T(b.cx[nb] - x))) < 3.5 * double(h) && double(xfabs(T(b.cy[nb] - y))) < 3.5 * double(h))
+                      ? 1
+                      : 3;
+          }
+        } else {
+          c = nc0 + j;
+          cnt = b.scnt[c];
+          if (cnt != 0) cat = (xfabs(T(b.cx[c] - x)) < 3 * h && xfabs(T(b.cy[c] - y)) < 3 * h) ? 1 : 2;
+        }
       }
     }
+    const unsigned m1 = __ballot_sync(0xffffffffu, cat == 1);
+    const unsigned m2 = __ballot_sync(0xffffffffu, cat == 2);
+    const unsigned m3 = __ballot_sync(0xffffffffu, cat == 3);
+    if (cat == 1) {
+      const int pos = nn + __popc(m1 & below);
+      if (pos < kMaxNeighbors) {
+        b.nbr[k * kMaxNeighbors + pos] = c;
+        near += cnt;
+      } else {
+        err |= kErrNeighborOverflow;
+      }
+    } else if (cat == 2) {
+      const int pos = ns + __popc(m2 & below);
+      if (pos < kMaxSameLevelIL) b.sil[k * kMaxSameLevelIL + pos] = c;
+      else err |= kErrSameLevelOverflow;
+    } else if (cat == 3) {
+      const int pos = nd + __popc(m3 & below);
+      if (pos < kMaxDiffLevelIL) b.dil[k * kMaxDiffLevelIL + pos] = c;
+      else err |= kErrDiffLevelOverflow;
+    }
+    nn += __popc(m1);
+    ns += __popc(m2);
+    nd += __popc(m3);
+  }
+  if (lane == 0) {
+    b.n_nbr[k] = min(nn, kMaxNeighbors);
+    b.n_sil[k] = min(ns, kMaxSameLevelIL);
+    b.n_dil[k] = min(nd, kMaxDiffLevelIL);
+  }
+  return int(__reduce_add_sync(0xffffffffu, unsigned(near))) + b.scnt[k];
+}
+
+// The 4 children of node k from c0 on; their star ranges follow from the
+// partition of k's stars.
+template <typename T>
+__device__ __forceinline__ void tree_node_children(const TreeBuild<T>& b, int k, int c0) {
+  b.child0[k] = c0;
+  const T h = b.hl[k] / 2;
+  const T pcx = b.cx[k], pcy = b.cy[k];
+  const T ox[4] = {T(1), T(-1), T(-1), T(1)};
+  const T oy[4] = {T(1), T(1), T(-1), T(-1)};
+  const double plox = b.lox[k], phix = b.hix[k], ploy = b.loy[k], phiy = b.hiy[k];
+  const int lev = b.level[k] + 1, r = b.rid[k];
+  for (int q = 0; q < 4; q++) {
+    const int c = c0 + q;
+    b.cx[c] = pcx + h * ox[q];
+    b.cy[c] = pcy + h * oy[q];
+    b.hl[c] = h;
+    b.level[c] = lev;
+    b.parent[c] = k;
+    b.rid[c] = r;
+    b.child0[c] = -1;
+    b.n_nbr[c] = b.n_sil[c] = b.n_dil[c] = 0;
+    // x >= pcx for q = 0, 3; y >= pcy for q = 0, 1
+    const bool right = (q == 0 || q == 3), top = (q == 0 || q == 1);
+    b.lox[c] = right ? double(pcx) : plox;
+    b.hix[c] = right ? phix : double(pcx);
+    b.loy[c] = top ? double(pcy) : ploy;
+    b.hiy[c] = top ? phiy : double(pcy);
+  }
+}
+
+// Stars [s0, s0 + n) of a node with centre (x, y) into its 4 children's ranges
+// from child c0 on, keeping their relative order: by one warp.
+template <typename T>
+__device__ __forceinline__ void tree_partition_warp(const TreeBuild<T>& b, int s0, int n, int c0, T x, T y, int lane) {
+  int cnt[4] = {0, 0, 0, 0};
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    int q = -1;
+    if (i0 + lane < n) q = star_quadrant(b.stars[s0 + i0 + lane].x, b.stars[s0 + i0 + lane].y, x, y);
+#pragma unroll
+    for (int qq = 0; qq < 4; qq++) cnt[qq] += __popc(__ballot_sync(0xffffffffu, q == qq));
+  }
+  int base[4];
+  base[0] = s0;
+#pragma unroll
+  for (int q = 1; q < 4; q++) base[q] = base[q - 1] + cnt[q - 1];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (lane == q) {
+      b.sbeg[c0 + q] = base[q];
+      b.scnt[c0 + q] = cnt[q];
+    }
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    int q = -1;
+    StarRec<T> st;
+    if (i0 + lane < n) {
+      st = b.stars[s0 + i0 + lane];
+      q = star_quadrant(st.x, st.y, x, y);
+    }
+#pragma unroll
+    for (int qq = 0; qq < 4; qq++) {
+      const unsigned m = __ballot_sync(0xffffffffu, q == qq);
+      if (q == qq) b.tmp[base[qq] + __popc(m & ((1u << lane) - 1u))] = st;
+      base[qq] += __popc(m);
+    }
+  }
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) b.stars[s0 + i] = b.tmp[s0 + i];
+}
+
+constexpr int kTreeThreads = 512;
+constexpr int kTreeWarps = kTreeThreads / 32;
+// A node of up to this many stars is partitioned by one warp, up to
+// tree_big_node by its CTA, beyond that by all CTAs.
+constexpr int kPartWarpStars = 512;
+
+// The same by the whole CTA.
+template <typename T>
+__device__ __forceinline__ void tree_partition_block(const TreeBuild<T>& b, int s0, int n, int c0, T x, T y) {
+  __shared__ int cnt[4], base[4], warp_cnt[kTreeWarps][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  int lc[4] = {0, 0, 0, 0};
+  for (int i = threadIdx.x; i < n; i += kTreeThreads) {
+    const int q = star_quadrant(b.stars[s0 + i].x, b.stars[s0 + i].y, x, y);
+#pragma unroll
+    for (int qq = 0; qq < 4; qq++) lc[qq] += q == qq;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int v = int(__reduce_add_sync(0xffffffffu, unsigned(lc[q])));
+    if (lane == 0 && v) atomicAdd(&cnt[q], v);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int acc = s0;
+    for (int q = 0; q < 4; q++) {
+      base[q] = acc;
+      b.sbeg[c0 + q] = acc;
+      b.scnt[c0 + q] = cnt[q];
+      acc += cnt[q];
+    }
+  }
+  __syncthreads();
+  for (int start = 0; start < n; start += kTreeThreads) {
+    const int i = start + int(threadIdx.x);
+    int q = -1;
+    StarRec<T> st;
+    if (i < n) {
+      st = b.stars[s0 + i];
+      q = star_quadrant(st.x, st.y, x, y);
+    }
+    unsigned mine = 0;
+#pragma unroll
+    for (int qq = 0; qq < 4; qq++) {
+      const unsigned m = __ballot_sync(0xffffffffu, q == qq);
+      if (lane == 0) warp_cnt[w][qq] = __popc(m);
+      if (q == qq) mine = m;
+    }
     __syncthreads();
-    for (int start = 0; start < n; start += blockDim.x) {
-      int i = start + threadIdx.x;
+    if (q >= 0) {
+      int off = base[q];
+      for (int ww = 0; ww < w; ww++) off += warp_cnt[ww][q];
+      b.tmp[off + __popc(mine & ((1u << lane) - 1u))] = st;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+      int add = 0;
+      for (int ww = 0; ww < kTreeWarps; ww++) add += warp_cnt[ww][threadIdx.x];
+      base[threadIdx.x] += add;
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < n; i += kTreeThreads) b.stars[s0 + i] = b.tmp[s0 + i];
+  __syncthreads();
+}
+
+// The same by all CTAs, for every split node of the level [beg, end) that holds
+// more than `big` stars: CTA c takes the c-th share [s0, s1) of the whole star
+// array (the level's nodes are star ranges in node order, so a share meets a
+// few of them, all but the first and last inside it), counts its stars per node
+// and quadrant, and after a grid barrier places them in `tmp` behind those of
+// the CTAs before it; after another one it copies its share back. At most
+// kShareNodes such nodes meet a share (tree_big_node). Returns false when a
+// grid barrier gave up.
+constexpr int kShareNodes = 10;
+__host__ __device__ __forceinline__ int tree_big_node(int per) { return per / 8 > 2048 ? per / 8 : 2048; }
+
+template <typename T>
+__device__ __forceinline__ bool tree_partition_shared(const TreeBuild<T>& b, int beg, int end, int per, int big,
+                                                      unsigned long long*& word, long long spins) {
+  __shared__ int s_node[kShareNodes], s_n, run[kShareNodes][4], warp_cnt[kTreeWarps][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, grid = gridDim.x, me = blockIdx.x;
+  const int s0 = min(b.nstars, me * per), s1 = min(b.nstars, s0 + per);
+  int* seg_n = b.cta + 2 * grid;   // [grid] big nodes that meet the share
+  int* counts = b.cta + 3 * grid;  // [grid][kShareNodes][4]
+  if (threadIdx.x == 0) {
+    int lo = beg, hi = end - 1;  // last node that starts at or before s0
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (b.sbeg[mid] <= s0) lo = mid;
+      else hi = mid - 1;
+    }
+    int n = 0;
+    for (int k = lo; s0 < s1 && k < end && b.sbeg[k] < s1; k++)
+      if (b.split[k - beg] && b.scnt[k] > big && b.sbeg[k] + b.scnt[k] > s0 && n < kShareNodes) s_node[n++] = k;
+    s_n = n;
+    seg_n[me] = n;
+  }
+  if (threadIdx.x < kShareNodes * 4) run[threadIdx.x / 4][threadIdx.x % 4] = 0;
+  __syncthreads();
+  const int n = s_n;
+  for (int g = 0; g < n; g++) {
+    const int k = s_node[g], i0 = max(s0, b.sbeg[k]), i1 = min(s1, b.sbeg[k] + b.scnt[k]);
+    const T x = b.cx[k], y = b.cy[k];
+    int lc[4] = {0, 0, 0, 0};
+    for (int i = i0 + int(threadIdx.x); i < i1; i += kTreeThreads) {
+      const int q = star_quadrant(b.stars[i].x, b.stars[i].y, x, y);
+#pragma unroll
+      for (int qq = 0; qq < 4; qq++) lc[qq] += q == qq;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int v = int(__reduce_add_sync(0xffffffffu, unsigned(lc[q])));
+      if (lane == 0 && v) atomicAdd(&run[g][q], v);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < n * 4) counts[me * kShareNodes * 4 + threadIdx.x] = run[threadIdx.x / 4][threadIdx.x % 4];
+  if (grid_barrier_sum(word++, 0, b.status + kTreeBarrier, spins) < 0) return false;
+  // warp g: node g's counts before this CTA and in all. The node is the last
+  // big one of the CTA it starts in and the first of every CTA after that.
+  for (int g = w; g < n; g += kTreeWarps) {
+    const int k = s_node[g], c0 = b.sbeg[k] / per, c1 = (b.sbeg[k] + b.scnt[k] - 1) / per;
+    int before[4] = {0, 0, 0, 0}, all[4] = {0, 0, 0, 0};
+    for (int c = c0 + lane; c <= c1; c += 32) {
+      const int gg = c == me ? g : (c == c0 ? seg_n[c] - 1 : 0);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int v = counts[(c * kShareNodes + gg) * 4 + q];
+        all[q] += v;
+        before[q] += c < me ? v : 0;
+      }
+    }
+    int acc = b.sbeg[k];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      all[q] = int(__reduce_add_sync(0xffffffffu, unsigned(all[q])));
+      before[q] = int(__reduce_add_sync(0xffffffffu, unsigned(before[q])));
+      if (lane == 0) {
+        run[g][q] = acc + before[q];
+        if (c0 == me) {
+          b.sbeg[b.child0[k] + q] = acc;
+          b.scnt[b.child0[k] + q] = all[q];
+        }
+      }
+      acc += all[q];
+    }
+  }
+  __syncthreads();
+  for (int g = 0; g < n; g++) {
+    const int k = s_node[g], i0 = max(s0, b.sbeg[k]), i1 = min(s1, b.sbeg[k] + b.scnt[k]);
+    const T x = b.cx[k], y = b.cy[k];
+    for (int r = i0; r < i1; r += kTreeThreads) {  // rounds in star order
+      const int i = r + int(threadIdx.x);
       int q = -1;
       StarRec<T> st;
-      if (i < n) {
-        st = stars[b + i];
-        q = star_quadrant(st.x, st.y, pcx, pcy);
+      if (i < i1) {
+        st = b.stars[i];
+        q = star_quadrant(st.x, st.y, x, y);
       }
-      unsigned m[4];
-      for (int qq = 0; qq < 4; qq++) m[qq] = __ballot_sync(0xffffffffu, q == qq);
-      if (lane < 4) warp_cnt[w][lane] = __popc(m[lane]);
+      unsigned mine = 0;
+#pragma unroll
+      for (int qq = 0; qq < 4; qq++) {
+        const unsigned m = __ballot_sync(0xffffffffu, q == qq);
+        if (lane == 0) warp_cnt[w][qq] = __popc(m);
+        if (q == qq) mine = m;
+      }
       __syncthreads();
       if (q >= 0) {
-        int off = base[q];
-        for (int ww = 0; ww < w; ww++) off += warp_cnt[ww][q];
-        off += __popc(m[q] & ((1u << lane) - 1u));
-        tmp[off] = st;
+        int pos = run[g][q];
+        for (int ww = 0; ww < w; ww++) pos += warp_cnt[ww][q];
+        b.tmp[pos + __popc(mine & ((1u << lane) - 1u))] = st;
       }
       __syncthreads();
       if (threadIdx.x < 4) {
         int add = 0;
-        for (int ww = 0; ww < NT / 32; ww++) add += warp_cnt[ww][threadIdx.x];
-        base[threadIdx.x] += add;
+        for (int ww = 0; ww < kTreeWarps; ww++) add += warp_cnt[ww][threadIdx.x];
+        run[g][threadIdx.x] += add;
       }
       __syncthreads();
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) stars[b + i] = tmp[b + i];
-    __syncthreads();
   }
-}
-
-// The same stable partition for the first two levels, whose NN nodes (1 or 4)
-// hold every star between them, on many blocks: the stars are cut into chunks
-// of kPartChunk; a star's key is its node's index in the level times 4 plus its
-// quadrant (0 in a node that does not split). Count per chunk and key, scan
-// each key over the chunks (stable), scatter, copy back. A level that is
-// absent (the root did not split) is left alone.
-constexpr int kPartChunk = 1024;
-
-template <typename T, int NN>
-__device__ __forceinline__ int wide_key(int i, int beg, const int* __restrict__ split, const T* __restrict__ cx,
-                                        const T* __restrict__ cy, const int* __restrict__ sbeg,
-                                        const int* __restrict__ scnt, const StarRec<T>& st) {
-  int j = 0;
-#pragma unroll
-  for (int jj = 1; jj < NN; jj++)
-    if (i >= sbeg[beg + jj]) j = jj;  // the level's nodes are consecutive star ranges in node order
-  const int k = beg + j;
-  return 4 * j + (split[j] ? star_quadrant(st.x, st.y, cx[k], cy[k]) : 0);
-}
-
-template <int NN>
-__device__ __forceinline__ bool wide_level(LevelRange lr, const int* stop, int& beg) {
-  int b = 0, e = 0;
-  lr.get(b, e);
-  beg = b;
-  return !(stop && *stop) && e - b == NN;
-}
-
-template <typename T, int NN>
-__global__ void __launch_bounds__(256) tree_wide_count(LevelRange lr, const int* __restrict__ stop,
-                                                       const int* __restrict__ split, const T* __restrict__ cx,
-                                                       const T* __restrict__ cy, const int* __restrict__ sbeg,
-                                                       const int* __restrict__ scnt,
-                                                       const StarRec<T>* __restrict__ stars, int nstars, int* cnt) {
-  int beg;
-  if (!wide_level<NN>(lr, stop, beg)) return;
-  __shared__ int c[4 * NN];
-  if (threadIdx.x < 4 * NN) c[threadIdx.x] = 0;
-  __syncthreads();
-  const int i0 = blockIdx.x * kPartChunk, i1 = min(i0 + kPartChunk, nstars);
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x)
-    atomicAdd(&c[wide_key<T, NN>(i, beg, split, cx, cy, sbeg, scnt, stars[i])], 1);
-  __syncthreads();
-  if (threadIdx.x < 4 * NN) cnt[blockIdx.x * 4 * NN + threadIdx.x] = c[threadIdx.x];
-}
-
-// One block: per key, the exclusive scan over the chunks plus the key's base
-// (its node's first star plus the counts of the node's lower quadrants); the
-// children's star ranges.
-template <int NN>
-__global__ void tree_wide_offsets(LevelRange lr, const int* __restrict__ stop, const int* __restrict__ split,
-                                  const int* __restrict__ child0, int* sbeg, int* scnt, int nchunks, int* cnt) {
-  int beg;
-  if (!wide_level<NN>(lr, stop, beg)) return;
-  constexpr int K = 4 * NN;
-  __shared__ int tot[K], base[K];
-  if (threadIdx.x < K) {
-    int run = 0;
-    for (int c = 0; c < nchunks; c++) {
-      const int v = cnt[c * K + threadIdx.x];
-      cnt[c * K + threadIdx.x] = run;
-      run += v;
-    }
-    tot[threadIdx.x] = run;
+  if (grid_barrier_sum(word++, 0, b.status + kTreeBarrier, spins) < 0) return false;
+  for (int g = 0; g < n; g++) {
+    const int k = s_node[g], i0 = max(s0, b.sbeg[k]), i1 = min(s1, b.sbeg[k] + b.scnt[k]);
+    for (int i = i0 + int(threadIdx.x); i < i1; i += kTreeThreads) b.stars[i] = b.tmp[i];
   }
-  __syncthreads();
-  if (threadIdx.x < NN) {
-    const int j = threadIdx.x, k = beg + j;
-    int acc = sbeg[k];
-    for (int q = 0; q < 4; q++) {
-      base[4 * j + q] = acc;
-      if (split[j]) {
-        sbeg[child0[k] + q] = acc;
-        scnt[child0[k] + q] = tot[4 * j + q];
-      }
-      acc += tot[4 * j + q];
-    }
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < nchunks * K; idx += blockDim.x) cnt[idx] += base[idx % K];
+  return true;
 }
 
-template <typename T, int NN>
-__global__ void __launch_bounds__(256) tree_wide_scatter(LevelRange lr, const int* __restrict__ stop,
-                                                         const int* __restrict__ split, const T* __restrict__ cx,
-                                                         const T* __restrict__ cy, const int* __restrict__ sbeg,
-                                                         const int* __restrict__ scnt,
-                                                         const StarRec<T>* __restrict__ stars, int nstars,
-                                                         const int* __restrict__ off, StarRec<T>* __restrict__ tmp) {
-  int beg;
-  if (!wide_level<NN>(lr, stop, beg)) return;
-  constexpr int K = 4 * NN;
-  __shared__ int run[K];
-  __shared__ int wc[8][K];
+// Exclusive scan of a flag (0 or 1) over the CTA's threads; *total their sum.
+__device__ __forceinline__ int block_scan_flag(int flag, int* total) {
+  __shared__ int s_w[kTreeWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x < K) run[threadIdx.x] = off[blockIdx.x * K + threadIdx.x];
+  const unsigned m = __ballot_sync(0xffffffffu, flag != 0);
+  if (lane == 0) s_w[w] = __popc(m);
   __syncthreads();
-  const int i0 = blockIdx.x * kPartChunk, i1 = min(i0 + kPartChunk, nstars);
-  for (int r = i0; r < i1; r += 256) {  // rounds in star order
-    const int i = r + threadIdx.x;
-    int key = -1;
-    StarRec<T> st;
-    if (i < i1) {
-      st = stars[i];
-      key = wide_key<T, NN>(i, beg, split, cx, cy, sbeg, scnt, st);
-    }
-    unsigned mine = 0;
+  int before = __popc(m & ((1u << lane) - 1u)), all = 0;
 #pragma unroll
-    for (int kk = 0; kk < K; kk++) {
-      const unsigned m = __ballot_sync(0xffffffffu, key == kk);
-      if (lane == 0) wc[w][kk] = __popc(m);
-      if (key == kk) mine = m;
-    }
-    __syncthreads();
-    if (key >= 0) {
-      int pos = run[key];
-      for (int ww = 0; ww < w; ww++) pos += wc[ww][key];
-      tmp[pos + __popc(mine & ((1u << lane) - 1u))] = st;
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-      int add = 0;
-      for (int ww = 0; ww < 8; ww++) add += wc[ww][threadIdx.x];
-      run[threadIdx.x] += add;
-    }
-    __syncthreads();
+  for (int ww = 0; ww < kTreeWarps; ww++) {
+    const int v = s_w[ww];
+    before += ww < w ? v : 0;
+    all += v;
   }
+  __syncthreads();
+  *total = all;
+  return before;
 }
 
-template <typename T, int NN>
-__global__ void tree_wide_copy(LevelRange lr, const int* __restrict__ stop, int nstars,
-                               const StarRec<T>* __restrict__ tmp, StarRec<T>* __restrict__ stars) {
-  int beg;
-  if (!wide_level<NN>(lr, stop, beg)) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nstars; i += gridDim.x * blockDim.x) stars[i] = tmp[i];
-}
-
-// set_neighbors (tree_node.cuh:183-267) for the nodes of one level (>= 1).
-template <typename T>
-__global__ void tree_set_neighbors(int beg, int end, LevelRange lr, const T* __restrict__ cx,
-                                   const T* __restrict__ cy, const T* __restrict__ hl, const int* __restrict__ parent,
-                                   const int* __restrict__ child0, const int* __restrict__ scnt, int* nbr,
-                                   int* n_nbr, int* sil, int* n_sil, int* dil, int* n_dil, int* dstat) {
-  lr.get(beg, end);
-  for (int k = beg + blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x) {
-    int p = parent[k];
-    T h = hl[k];
-    T x = cx[k], y = cy[k];
-    int nn = 0, ns = 0, nd = 0, err = 0;
-    int pc0 = child0[p];
-    for (int i = 0; i < 4; i++) {
-      int c = pc0 + i;
-      if (scnt[c] == 0) continue;
-      if (c != k) {
-        if (nn < kMaxNeighbors) nbr[k * kMaxNeighbors + nn] = c;
-        else err |= kErrNeighborOverflow;
-        nn++;
-      }
+// Sums of an array over the CTAs before this one and over all of them.
+__device__ __forceinline__ void cta_prefix(const int* v, int* before, int* all) {
+  __shared__ int s_r[2];
+  if (threadIdx.x < 32) {
+    int p = 0, a = 0;
+    for (int c = threadIdx.x; c < int(gridDim.x); c += 32) {
+      const int x = v[c];
+      a += x;
+      p += c < int(blockIdx.x) ? x : 0;
     }
-    int pn = n_nbr[p];
-    for (int i = 0; i < pn; i++) {
-      int nb = nbr[p * kMaxNeighbors + i];
-      if (scnt[nb] == 0) continue;
-      int nc0 = child0[nb];
-      if (nc0 < 0) {
-        if (double(xfabs(T(cx[nb] - x))) < 3.5 * double(h) && double(xfabs(T(cy[nb] - y))) < 3.5 * double(h)) {
-          if (nn < kMaxNeighbors) nbr[k * kMaxNeighbors + nn] = nb;
-          else err |= kErrNeighborOverflow;
-          nn++;
-        } else {
-          if (nd < kMaxDiffLevelIL) dil[k * kMaxDiffLevelIL + nd] = nb;
-          else err |= kErrDiffLevelOverflow;
-          nd++;
-        }
-      } else {
-        for (int j = 0; j < 4; j++) {
-          int c = nc0 + j;
-          if (scnt[c] == 0) continue;
-          if (xfabs(T(cx[c] - x)) < 3 * h && xfabs(T(cy[c] - y)) < 3 * h) {
-            if (nn < kMaxNeighbors) nbr[k * kMaxNeighbors + nn] = c;
-            else err |= kErrNeighborOverflow;
-            nn++;
-          } else {
-            if (ns < kMaxSameLevelIL) sil[k * kMaxSameLevelIL + ns] = c;
-            else err |= kErrSameLevelOverflow;
-            ns++;
-          }
-        }
-      }
-    }
-    n_nbr[k] = min(nn, kMaxNeighbors);
-    n_sil[k] = min(ns, kMaxSameLevelIL);
-    n_dil[k] = min(nd, kMaxDiffLevelIL);
-    if (err) atomicOr(&dstat[1], err);
-  }
-}
-
-// The same lists with one warp per node: lane q examines candidate q in the
-// order of the loops above (the 4 siblings, then for each of the parent's
-// neighbours either the neighbour itself, a leaf, or its 4 children), and
-// each list takes its candidates in that order through a ballot prefix, so
-// the lists are identical to the one-thread form.
-template <typename T>
-__global__ void tree_set_neighbors_warp(LevelRange lr, const T* __restrict__ cx, const T* __restrict__ cy,
-                                        const T* __restrict__ hl, const int* __restrict__ parent,
-                                        const int* __restrict__ child0, const int* __restrict__ scnt, int* nbr,
-                                        int* n_nbr, int* sil, int* n_sil, int* dil, int* n_dil, int* dstat) {
-  int beg = 0, end = 0;
-  lr.get(beg, end);
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int k = beg + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < end; k += warps) {
-    const int p = parent[k];
-    const T h = hl[k], x = cx[k], y = cy[k];
-    const int pc0 = child0[p];
-    const int nq = 4 + 4 * n_nbr[p];
-    int nn = 0, ns = 0, nd = 0, err = 0;
-    for (int q0 = 0; q0 < nq; q0 += 32) {
-      const int q = q0 + lane;
-      int cat = 0, c = -1;  // 1 neighbour, 2 same-level interaction, 3 different-level interaction
-      if (q < 4) {
-        c = pc0 + q;
-        if (scnt[c] != 0 && c != k) cat = 1;
-      } else if (q < nq) {
-        const int i = (q - 4) >> 2, j = (q - 4) & 3;
-        const int nb = nbr[p * kMaxNeighbors + i];
-        if (scnt[nb] != 0) {
-          const int nc0 = child0[nb];
-          if (nc0 < 0) {
-            if (j == 0) {
-              c = nb;
-              cat = (double(xfabs(T(cx[nb] - x))) < 3.5 * double(h) && double(xfabs(T(cy[nb] - y))) < 3.5 * double(h))
-                        ? 1
-                        : 3;
-            }
-          } else {
-            c = nc0 + j;
-            if (scnt[c] != 0) cat = (xfabs(T(cx[c] - x)) < 3 * h && xfabs(T(cy[c] - y)) < 3 * h) ? 1 : 2;
-          }
-        }
-      }
-      const unsigned m1 = __ballot_sync(0xffffffffu, cat == 1);
-      const unsigned m2 = __ballot_sync(0xffffffffu, cat == 2);
-      const unsigned m3 = __ballot_sync(0xffffffffu, cat == 3);
-      if (cat == 1) {
-        const int pos = nn + __popc(m1 & below);
-        if (pos < kMaxNeighbors) nbr[k * kMaxNeighbors + pos] = c;
-        else err |= kErrNeighborOverflow;
-      } else if (cat == 2) {
-        const int pos = ns + __popc(m2 & below);
-        if (pos < kMaxSameLevelIL) sil[k * kMaxSameLevelIL + pos] = c;
-        else err |= kErrSameLevelOverflow;
-      } else if (cat == 3) {
-        const int pos = nd + __popc(m3 & below);
-        if (pos < kMaxDiffLevelIL) dil[k * kMaxDiffLevelIL + pos] = c;
-        else err |= kErrDiffLevelOverflow;
-      }
-      nn += __popc(m1);
-      ns += __popc(m2);
-      nd += __popc(m3);
-    }
-    err = __reduce_or_sync(0xffffffffu, unsigned(err));
-    if (lane == 0) {
-      n_nbr[k] = min(nn, kMaxNeighbors);
-      n_sil[k] = min(ns, kMaxSameLevelIL);
-      n_dil[k] = min(nd, kMaxDiffLevelIL);
-      if (err) atomicOr(&dstat[1], err);
+    p = int(__reduce_add_sync(0xffffffffu, unsigned(p)));
+    a = int(__reduce_add_sync(0xffffffffu, unsigned(a)));
+    if (threadIdx.x == 0) {
+      s_r[0] = p;
+      s_r[1] = a;
     }
   }
+  __syncthreads();
+  *before = s_r[0];
+  *all = s_r[1];
+  __syncthreads();
 }
 
-// Level bookkeeping of a build driven on the device: level l's nodes are
-// off[l] .. off[l + 1]; lvl_n[l] is their count.
-__global__ void tree_levels_init(int* off, int* lvl_n, int nlev, int roots, int* stop, int* dstat) {
-  off[0] = 0;
-  for (int l = 1; l <= nlev + 1; l++) off[l] = roots;
-  lvl_n[0] = roots;
-  for (int l = 1; l <= nlev; l++) lvl_n[l] = 0;
-  *stop = 0;
-  dstat[0] = dstat[1] = 0;
-}
-
-// After level l's split flags are scanned: the next level holds 4 children per
-// split node. Running out of levels or of node capacity stops the build (the
-// remaining level kernels see an empty range) and raises an error bit.
-__global__ void tree_advance_level(int l, int nlev, int* off, int* lvl_n, const long long* __restrict__ nsplit_p,
-                                   int node_cap, int* stop, int* dstat) {
-  const int end = off[l + 1];
-  long long nsplit = *stop ? 0 : *nsplit_p;
-  if (nsplit > 0 && l == nlev - 1) {
-    atomicOr(&dstat[1], kErrLevelOverflow);
-    *stop = 1;
-    nsplit = 0;
-  }
-  if (end + 4 * nsplit > node_cap) {
-    atomicOr(&dstat[1], kErrNodeOverflow);
-    *stop = 1;
-    nsplit = 0;
-  }
-  off[l + 2] = end + int(4 * nsplit);
-  lvl_n[l + 1] = int(4 * nsplit);
-}
-
-template <typename T, int NN>
-bool wide_partition(TreeDev<T>& t, LevelRange lr, StarRec<T>* stars, int nstars, int nchunks, cudaStream_t s) {
-  tree_wide_count<T, NN><<<nchunks, 256, 0, s>>>(lr, t.d_stop.p, t.split.p, t.cx.p, t.cy.p, t.sbeg.p, t.scnt.p, stars,
-                                                nstars, t.chunk_cnt.p);
-  tree_wide_offsets<NN><<<1, 256, 0, s>>>(lr, t.d_stop.p, t.split.p, t.child0.p, t.sbeg.p, t.scnt.p, nchunks,
-                                          t.chunk_cnt.p);
-  tree_wide_scatter<T, NN><<<nchunks, 256, 0, s>>>(lr, t.d_stop.p, t.split.p, t.cx.p, t.cy.p, t.sbeg.p, t.scnt.p,
-                                                  stars, nstars, t.chunk_cnt.p, t.tmp_stars.p);
-  tree_wide_copy<T, NN><<<std::min(nchunks * 4, 148 * 8), 256, 0, s>>>(lr, t.d_stop.p, nstars, t.tmp_stars.p, stars);
-  return IRSB_CK(cudaGetLastError());
-}
-
-// Builds the tree over `stars` (device, permuted in place into tree order).
-// Returns false on a CUDA error or a list overflow.
+// The whole tree in one cooperative launch: per level, the nodes' lists and
+// split flags (a warp per node), a grid barrier, the children of the split
+// nodes and the stable partition of their stars (by a warp, the CTA or, for the
+// few nodes of the top levels, all CTAs), a grid barrier; finally the leaves are numbered in node order. CTA c owns the
+// c-th contiguous share of a level's nodes, so node slots and leaf numbers are
+// those of an exclusive scan.
 //
-// The level loop runs on the device: every level kernel reads its node range
-// from the device offsets (LevelRange) on a grid sized by the most nodes the
-// level can hold (4^l), and the host reads the offsets back once per block of
-// levels (the first block covers the depth a uniform field of this size
-// reaches) instead of synchronising on every level. Node storage is reserved
-// up front; a field that needs more restores its star order and builds again
-// with twice the capacity.
+// Bound by latency: a handful of dependent loads per level and phase. As eight
+// to eleven launches per level with three scan passes among them, a field of
+// 2.2e3 stars (7 levels) took 0.35 ms (B200); now 0.09.
 template <typename T>
-bool build_tree(TreeDev<T>& t, StarRec<T>* stars, int nstars, T root_hl, cudaStream_t s) {
-  if (!t.tmp_stars.reserve(nstars, s) || !t.star_backup.reserve(nstars, s) || !t.dstat.reserve(2, s) ||
-      !t.d_off.reserve(kMaxLevels + 2, s) || !t.d_lvl_n.reserve(kMaxLevels + 1, s) || !t.d_stop.reserve(1, s))
-    return false;
-  const int nchunks = std::max(1, ceil_div(nstars, kPartChunk));
-  if (!t.chunk_cnt.reserve(size_t(nchunks) * 16, s)) return false;
+__global__ void __launch_bounds__(kTreeThreads, 1) tree_build_kernel(TreeBuild<T> b) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int grid = gridDim.x, me = blockIdx.x;
+  const long long spins = (1LL << 23) + b.nstars;
+  unsigned long long* word = b.words;
+  int* off = b.status + kTreeOff;
+  int* berr = b.status + kTreeBarrier;
+  {  // roots
+    const int per = (b.nroots + grid - 1) / grid;
+    for (int r = me * per + int(threadIdx.x); r < min(b.nroots, (me + 1) * per); r += kTreeThreads) {
+      b.cx[r] = b.cy[r] = T(0);
+      b.hl[r] = b.root_hls ? b.root_hls[r] : b.root_hl;
+      b.level[r] = 0;
+      b.parent[r] = -1;
+      b.child0[r] = -1;
+      b.sbeg[r] = b.star_off ? int(b.star_off[r]) : 0;
+      b.scnt[r] = b.star_off ? int(b.star_off[r + 1] - b.star_off[r]) : b.nstars;
+      b.rid[r] = r;
+      b.n_nbr[r] = b.n_sil[r] = b.n_dil[r] = 0;
+      b.lox[r] = b.loy[r] = -INFINITY;
+      b.hix[r] = b.hiy[r] = INFINITY;
+    }
+    __syncthreads();
+  }
+  const int share = (b.nstars + grid - 1) / grid, big = tree_big_node(share);
+  int beg = 0, end = b.nroots, l = 0;
+  for (;; l++) {
+    const int n = end - beg, per = (n + grid - 1) / grid;
+    const int k0 = min(end, beg + me * per), k1 = min(end, k0 + per);
+    // ---- lists, split flags and their ranks within the CTA
+    int err = 0;
+    for (int k = k0 + w; k < k1; k += kTreeWarps) {
+      const int near = l > 0 ? tree_node_lists(b, k, lane, err) : b.scnt[k];
+      if (lane == 0) b.split[k - beg] = near > kMaxStarsDirect ? 1 : 0;
+    }
+    if (err) atomicOr(b.status + kTreeErr, err);
+    __syncthreads();
+    int mine = 0, bigs = 0;
+    for (int base = k0; base < k1; base += kTreeThreads) {
+      const int k = base + int(threadIdx.x);
+      const int f = k < k1 ? b.split[k - beg] : 0;
+      bigs |= f && b.scnt[k] > big;
+      int total;
+      const int before = block_scan_flag(f, &total);
+      if (k < k1) b.rank[k - beg] = mine + before;
+      mine += total;
+    }
+    if (threadIdx.x == 0) b.cta[(l & 1) * grid + me] = mine;
+    bigs = __any_sync(0xffffffffu, bigs) ? 1 : 0;
+    bigs = grid_barrier_sum(word++, bigs, berr, spins);  // > 0: some node is partitioned by all CTAs
+    if (bigs < 0) return;
+    // ---- children
+    int before, nsplit;
+    cta_prefix(b.cta + (l & 1) * grid, &before, &nsplit);
+    if (me == 0 && threadIdx.x == 0) off[l] = beg;
+    int stop = 0;  // running out of levels or of node capacity ends the build with this level's nodes as leaves
+    if (nsplit > 0 && l == b.nlev - 1) stop = kErrLevelOverflow;
+    else if ((long long)end + 4LL * nsplit > b.cap) stop = kErrNodeOverflow;
+    if (stop && me == 0 && threadIdx.x == 0) atomicOr(b.status + kTreeErr, stop);
+    if (stop || nsplit == 0) break;
+    int mid = 0;  // nodes of the CTA's share that the whole CTA partitions
+    for (int k = k0 + int(threadIdx.x); k < k1; k += kTreeThreads)
+      if (b.split[k - beg]) {
+        tree_node_children(b, k, end + 4 * (before + b.rank[k - beg]));
+        mid |= b.scnt[k] > kPartWarpStars && b.scnt[k] <= big;
+      }
+    mid = __syncthreads_or(mid);
+    for (int k = k0 + w; k < k1; k += kTreeWarps)
+      if (b.split[k - beg] && b.scnt[k] <= kPartWarpStars)
+        tree_partition_warp(b, b.sbeg[k], b.scnt[k], b.child0[k], b.cx[k], b.cy[k], lane);
+    for (int k = k0; mid && k < k1; k++)
+      if (b.split[k - beg] && b.scnt[k] > kPartWarpStars && b.scnt[k] <= big)  // CTA-uniform
+        tree_partition_block(b, b.sbeg[k], b.scnt[k], b.child0[k], b.cx[k], b.cy[k]);
+    if (bigs > 0 && !tree_partition_shared(b, beg, end, share, big, word, spins)) return;
+    if (grid_barrier_sum(word++, 0, berr, spins) < 0) return;
+    beg = end;
+    end += 4 * nsplit;
+  }
+  // ---- leaves in node order
+  const int per = (end + grid - 1) / grid, k0 = min(end, me * per), k1 = min(end, k0 + per);
+  int mine = 0;
+  for (int base = k0; base < k1; base += kTreeThreads) {
+    const int k = base + int(threadIdx.x);
+    int total;
+    const int pos = block_scan_flag(k < k1 && b.child0[k] < 0, &total);
+    if (k < k1) b.leaf_pos[k] = mine + pos;
+    mine += total;
+  }
+  int* counts = b.cta + 2 * grid;
+  if (threadIdx.x == 0) counts[me] = mine;
+  if (grid_barrier_sum(word++, 0, berr, spins) < 0) return;
+  int before, leaves;
+  cta_prefix(counts, &before, &leaves);
+  for (int k = k0 + int(threadIdx.x); k < k1; k += kTreeThreads) {
+    const long long pos = b.leaf_pos[k] + before;
+    b.leaf_pos[k] = pos;
+    if (b.child0[k] < 0) b.leaf_node[pos] = k;
+  }
+  if (me == 0 && threadIdx.x == 0) {
+    b.status[kTreeLevels] = l;
+    b.status[kTreeLeaves] = leaves;
+    for (int i = l + 1; i <= kMaxLevels + 1; i++) off[i] = end;
+  }
+}
+
+// Launches the build of nroots trees over `stars` (device, permuted in place
+// into tree order) on stream s: no synchronisation. t's node arrays hold cap
+// nodes. leaf_pos / leaf_node: DevVecs of at least cap entries.
+template <typename T>
+bool launch_tree_build(TreeDev<T>& t, StarRec<T>* stars, int nstars, int nroots, T root_hl, const T* root_hls,
+                       const long long* star_off, int cap, int nlev, long long* leaf_pos, int* leaf_node,
+                       cudaStream_t s) {
+  int grid = 0;
+  // a CTA per 64 stars: fewer arrivals per barrier where a field has less work
+  // than the whole chip
+  if (!cooperative_grid(tree_build_kernel<T>, kTreeThreads, std::max(nroots, ceil_div(nstars, 64)), &grid)) return false;
+  TreeBuild<T> b{t.cx.p, t.cy.p, t.hl.p, t.level.p, t.parent.p, t.child0.p, t.sbeg.p, t.scnt.p, t.rid.p, t.nbr.p,
+                 t.n_nbr.p, t.sil.p, t.n_sil.p, t.dil.p, t.n_dil.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p, t.split.p,
+                 t.rank.p, t.cta.p, t.status.p, t.words.p, leaf_pos, leaf_node, stars, t.tmp_stars.p, nroots, nstars,
+                 cap, nlev, root_hl, root_hls, star_off};
+  IRSB_CKR(cudaMemsetAsync(t.words.p, 0, (kTreeBarriers + kFmmBarriers) * sizeof(unsigned long long), s));
+  IRSB_CKR(cudaMemsetAsync(t.status.p, 0, kTreeStatusWords * sizeof(int), s));
+  void* args[] = {&b};
+  IRSB_CKR(cudaLaunchCooperativeKernel((const void*)tree_build_kernel<T>, dim3(grid), dim3(kTreeThreads), args, 0, s));
+  return true;
+}
+
+// Buffers of a build over nstars stars with room for cap nodes.
+template <typename T>
+bool tree_build_reserve(TreeDev<T>& t, int nstars, int cap, cudaStream_t s) {
+  return tree_reserve(t, cap, s) && t.split.reserve(cap, s) && t.rank.reserve(cap, s) &&
+         t.cta.reserve((3 + 4 * kShareNodes) * 1024, s) && t.status.reserve(kTreeStatusWords, s) &&
+         t.words.reserve(kTreeBarriers + kFmmBarriers, s) && t.tmp_stars.reserve(nstars, s) &&
+         t.h_status.alloc(kTreeStatusWords);
+}
+
+// Builds the tree over `stars` (device, permuted in place into tree order) and
+// numbers its leaves (leaf_pos, leaf_node: grown as needed). Returns false on a
+// CUDA error or a list overflow. Node storage is reserved up front; a field
+// that needs more restores its star order and builds again with twice the
+// capacity. `before_sync(cap)` enqueues work that needs only the device's
+// tree ahead of the one synchronisation.
+template <typename T, typename F>
+bool build_tree(TreeDev<T>& t, StarRec<T>* stars, int nstars, T root_hl, DevVec<long long>& leaf_pos,
+                DevVec<int>& leaf_node, cudaStream_t s, F before_sync) {
+  if (!t.star_backup.reserve(nstars, s)) return false;
   IRSB_CKR(cudaMemcpyAsync(t.star_backup.p, stars, size_t(nstars) * sizeof(StarRec<T>), cudaMemcpyDeviceToDevice, s));
   long long cap = std::max<long long>(t.cap, nstars + nstars / 2 + 1024);
-  int depth = 1;  // levels of a uniform field: 4^depth >= nstars
-  while (depth < kMaxLevels && (1LL << (2 * depth)) < nstars) depth++;
-  const int G = 148 * 8;
-  auto grid = [&](int l, int per_block) {
-    const long long most = l >= 15 ? (1LL << 30) : (1LL << (2 * l));
-    return int(std::max<long long>(1, std::min<long long>(ceil_div(most, (long long)per_block), G)));
-  };
-  std::vector<int> hoff(kMaxLevels + 2);
   t.launches = 0;
   for (int attempt = 0;; attempt++) {
     if (cap > (1LL << 28)) {
       std::fprintf(stderr, "Error. Tree needs more than %lld nodes.\n", 1LL << 28);
       return false;
     }
-    if (!tree_reserve(t, int(cap), s) || !t.split.reserve(cap, s) || !t.rank.reserve(cap + 1, s) ||
-        !scan_reserve(t.scan, cap, s))
+    if (!tree_build_reserve(t, nstars, int(cap), s) || !leaf_pos.alloc_exact(cap) || !leaf_node.alloc_exact(cap))
       return false;
     if (attempt > 0)
       IRSB_CKR(cudaMemcpyAsync(stars, t.star_backup.p, size_t(nstars) * sizeof(StarRec<T>), cudaMemcpyDeviceToDevice,
                                s));
-    tree_init_root<T><<<1, 1, 0, s>>>(t.cx.p, t.cy.p, t.hl.p, t.level.p, t.parent.p, t.child0.p, t.sbeg.p, t.scnt.p,
-                                      t.rid.p, t.n_nbr.p, t.n_sil.p, t.n_dil.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p,
-                                      root_hl, nstars);
-    tree_levels_init<<<1, 1, 0, s>>>(t.d_off.p, t.d_lvl_n.p, kMaxLevels, 1, t.d_stop.p, t.dstat.p);
-    IRSB_LAUNCH_CK("tree_init_root");
-    t.launches += 2;
-    int l = 0, levels = -1, err = 0, block = depth + 1;
-    while (levels < 0 && l < kMaxLevels) {
-      const int lend = std::min(kMaxLevels, l + block);
-      for (; l < lend; l++) {
-        const LevelRange lr{t.d_off.p, l}, next{t.d_off.p, l + 1};
-        const int g1 = grid(l, 256);
-        tree_near_count<<<g1, 256, 0, s>>>(0, 0, lr, t.scnt.p, t.nbr.p, t.n_nbr.p, t.split.p, t.dstat.p);
-        if (!exclusive_scan_dev<int>(t.split.p, t.d_lvl_n.p + l, cap, t.rank.p, t.scan, s)) return false;
-        tree_advance_level<<<1, 1, 0, s>>>(l, kMaxLevels, t.d_off.p, t.d_lvl_n.p, t.scan.sum.p, int(cap), t.d_stop.p,
-                                           t.dstat.p);
-        tree_make_children<T><<<g1, 256, 0, s>>>(0, 0, 0, lr, t.d_stop.p, t.split.p, t.rank.p, t.cx.p, t.cy.p, t.hl.p,
-                                                 t.level.p, t.parent.p, t.child0.p, t.sbeg.p, t.scnt.p, t.rid.p,
-                                                 t.n_nbr.p, t.n_sil.p, t.n_dil.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p);
-        if (l == 0) {  // the root: every star, on many blocks
-          if (!wide_partition<T, 1>(t, lr, stars, nstars, nchunks, s)) return false;
-          t.launches += 3;
-        } else if (l == 1) {  // the root's 4 children: every star
-          if (!wide_partition<T, 4>(t, lr, stars, nstars, nchunks, s)) return false;
-          t.launches += 3;
-        } else if (l <= 3)  // a few nodes holding many stars each
-          tree_partition_stars<T, 1024><<<grid(l, 1), 1024, 0, s>>>(0, 0, lr, t.d_stop.p, t.split.p, t.cx.p, t.cy.p,
-                                                                      t.child0.p, t.sbeg.p, t.scnt.p, stars,
-                                                                      t.tmp_stars.p);
-        else
-          tree_partition_stars<T><<<grid(l, 1), 256, 0, s>>>(0, 0, lr, t.d_stop.p, t.split.p, t.cx.p, t.cy.p,
-                                                              t.child0.p, t.sbeg.p, t.scnt.p, stars, t.tmp_stars.p);
-        tree_set_neighbors_warp<T><<<grid(l + 1, 8), 256, 0, s>>>(next, t.cx.p, t.cy.p, t.hl.p, t.parent.p,
-                                                                  t.child0.p, t.scnt.p, t.nbr.p, t.n_nbr.p, t.sil.p,
-                                                                  t.n_sil.p, t.dil.p, t.n_dil.p, t.dstat.p);
-        IRSB_LAUNCH_CK("tree level");
-        t.launches += 9;
-      }
-      int hst[2];
-      IRSB_CKR(cudaMemcpyAsync(hoff.data(), t.d_off.p, hoff.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-      IRSB_CKR(cudaMemcpyAsync(hst, t.dstat.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-      IRSB_CKR(cudaStreamSynchronize(s));
-      err = hst[1];
-      if (err) break;
-      for (int k = 0; k < l; k++)
-        if (hoff[k + 2] == hoff[k + 1]) {  // level k split nothing: its nodes are the last leaves
-          levels = k;
-          break;
-        }
-      block = 4;
+    if (!launch_tree_build<T>(t, stars, nstars, 1, root_hl, nullptr, nullptr, int(cap), kMaxLevels, leaf_pos.p,
+                              leaf_node.p, s))
+      return false;
+    t.launches++;
+    if (!before_sync(cap)) return false;
+    IRSB_CKR(cudaMemcpyAsync(t.h_status.p, t.status.p, kTreeStatusWords * sizeof(int), cudaMemcpyDeviceToHost, s));
+    IRSB_CKR(cudaStreamSynchronize(s));
+    const int* st = t.h_status.p;
+    const int err = st[kTreeErr];
+    if (st[kTreeBarrier]) {
+      std::fprintf(stderr, "Error. The tree build did not finish.\n");
+      return false;
     }
     if (err & kErrNodeOverflow) {
       cap *= 2;
@@ -688,13 +695,10 @@ bool build_tree(TreeDev<T>& t, StarRec<T>* stars, int nstars, T root_hl, cudaStr
       std::fprintf(stderr, "Error. Tree neighbour/interaction list overflow (code %d).\n", err);
       return false;
     }
-    if (levels < 0) {
-      std::fprintf(stderr, "Error. Tree exceeded %d levels.\n", kMaxLevels);
-      return false;
-    }
-    t.levels = levels;
-    t.level_off.assign(hoff.begin(), hoff.begin() + levels + 2);
+    t.levels = st[kTreeLevels];
+    t.level_off.assign(st + kTreeOff, st + kTreeOff + t.levels + 2);
     t.num_nodes = t.level_off.back();
+    t.num_leaves = st[kTreeLeaves];
     return true;
   }
 }

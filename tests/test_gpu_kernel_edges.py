@@ -130,11 +130,12 @@ def _corner_lattice(kind, rng):
     if kind == "point_lens":  # cells stretched over many pixels around a lens
         r2 = x * x + y * y + 0.01
         return np.stack([x - 30 * x / r2, y - 30 * y / r2], -1)
-    if kind == "far":  # beyond the range of int, not finite
+    if kind == "far":  # beyond the range of int, not finite (x below 2^31: the oracle takes columns as int)
         v = np.stack([x, y], -1)
         pick = rng.random(x.shape)
-        for k, val in enumerate([3.0e9, -3.0e9, 5.0e9, 1e18, -1e300, np.inf, -np.inf, np.nan, 2147483648.0, -2147483649.0]):
-            v[(pick >= 0.01 * k) & (pick < 0.01 * (k + 1)), k % 2] = val
+        for k, (axis, val) in enumerate([(0, 2.0e9), (1, -3.0e9), (1, 5.0e9), (1, 1e18), (0, -1e300), (1, np.inf),
+                                         (0, -np.inf), (1, np.nan), (1, 2147483648.0), (1, -2147483649.0)]):
+            v[(pick >= 0.01 * k) & (pick < 0.01 * (k + 1)), axis] = val
         return v
     if kind == "fine":  # most triangles inside one pixel
         return np.stack([x * 0.04 + 0.013 * y, y * 0.05 - 0.01 * x], -1)
