@@ -154,13 +154,10 @@ struct AdaGeom {
 
 // Corner (a, b) of tile t at level s, in the tile's corner grid
 // [0, ncell_x * s] x [0, ncell_y * s].
-// `stage`: the records of the tile's own leaf in shared memory, when the tile
-// has one (the values are those of the leaf in global memory).
 template <typename T, bool GENERIC_SMOOTH>
 __device__ __forceinline__ double2 tile_corner(const AdaGeom& g, const ShootParams& sp, const LeafPtrs& lp,
                                                const DescentPtrs<T>& dp, const double2* __restrict__ base_verts,
-                                               int tx, int ty, int s, int a, int b,
-                                               const LeafView* stage = nullptr) {
+                                               int tx, int ty, int s, int a, int b) {
   const long long i0 = (long long)tx * kAdaTile, j0 = (long long)ty * kAdaTile;
   const int sh = __ffs(s) - 1;  // levels are powers of two
   if (((a | b) & (s - 1)) == 0) {
@@ -171,7 +168,6 @@ __device__ __forceinline__ double2 tile_corner(const AdaGeom& g, const ShootPara
   const long long G = (j0 * kAdaMaxLevel) + (long long)b * (kAdaMaxLevel >> sh);
   const double x = fine_coord(g.base_x, g.rhs_x, F), y = fine_coord(g.base_y, g.rhs_y, G);
   const int own = dp.tile_leaf ? dp.tile_leaf[ty * g.ntx + tx] : -1;  // the descent's answer, when uniform
-  if (own >= 0 && stage) return eval_point_f32<GENERIC_SMOOTH>(sp, *stage, x, y);
   return eval_point_f32<GENERIC_SMOOTH>(sp, leaf_view(sp, lp, own >= 0 ? own : descend_leaf(dp, x, y)), x, y);
 }
 
@@ -182,7 +178,7 @@ template <typename T, bool GENERIC_SMOOTH>
 __device__ __forceinline__ double2 refine_point(const AdaGeom& g, const ShootParams& sp, const LeafPtrs& lp,
                                                 const DescentPtrs<T>& dp, const double2* __restrict__ base_verts,
                                                 const int* __restrict__ tile_level, int t, int tx, int ty, int s,
-                                                int a, int b, int wa, int hb, const LeafView* stage) {
+                                                int a, int b, int wa, int hb) {
   // neighbour across the edge this point lies on (a point on two edges is a
   // tile corner, hence a base point)
   int nlev = s;
@@ -204,68 +200,170 @@ __device__ __forceinline__ double2 refine_point(const AdaGeom& g, const ShootPar
     const int step = s >> (__ffs(nlev) - 1);
     const int u = along_b ? b : a;
     const int u0 = u & ~(step - 1), u1 = u0 + step;
-    const double2 p0 = along_b ? tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, u0, stage)
-                               : tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, u0, b, stage);
-    const double2 p1 = along_b ? tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, u1, stage)
-                               : tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, u1, b, stage);
+    const double2 p0 = along_b ? tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, u0)
+                               : tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, u0, b);
+    const double2 p1 = along_b ? tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, u1)
+                               : tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, u1, b);
     const double f = double(u - u0) / double(step);
     return make_double2(p0.x + (p1.x - p0.x) * f, p0.y + (p1.y - p0.y) * f);
   }
-  return tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, b, stage);
+  return tile_corner<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tx, ty, s, a, b);
 }
 
 // Refined corner grids of the tiles in `list` (all at level s), written at
-// out + slot * stride with row stride ncell_x * s + 1; one CTA per band of
-// kAdaBandRows corner rows of a tile (refine_point for each corner). When
-// every point of the tile belongs to one leaf (DescentPtrs::tile_leaf), its
-// near stars and local coefficients are staged in shared memory and the
-// band's corners read them as broadcasts; the other tiles take the descent
-// per point.
-constexpr int kAdaBandRows = 16;
-__host__ __device__ __forceinline__ long long ada_band_items(long long ntiles, int s) {
-  return ntiles * ((kAdaTile * s + 1 + kAdaBandRows - 1) / kAdaBandRows);
-}
+// out + slot * stride with row stride ncell_x * s + 1. A CTA of 4 warps takes a
+// band of 32 corner rows of a tile, a warp 8 of them; it walks the row in groups
+// of 32 columns, lane q column q with its 8 rows, through near_far_pairs (the
+// paired arithmetic of shoot_f32, the same bits as eval_point_f32). A leaf owns
+// the points of a half-open box (DescentPtrs::lox ...): the warp stages the stars
+// and coefficients of the leaf that owns its first point, keeps the positions
+// of the group's points in that box, and repeats for the points left (a leaf
+// boundary crosses one group in ten), descending only when a point leaves the
+// staged box. The last column and row of the tile (257 = 8 x 32 + 1) and the
+// points on an edge shared with a coarser neighbour go point by point
+// (refine_point).
+//
+// Bound by the reciprocals and FMAs of the lens equation. One point per thread,
+// each star read from shared memory for one point, and every point of a tile
+// that a leaf boundary crosses found by its own descent: 58 ms for 2.0e9 corners of a
+// 1024^2 map (B200); now 31 ms.
+constexpr int kAdaThreads = 128;
+constexpr int kAdaRows = 8;  // corner rows per warp
+constexpr int kAdaBand = kAdaRows * kAdaThreads / 32;
+static_assert(kAdaBand == kAdaTile, "s bands per tile of level s");
+// Work items (CTA visits) of a refinement of ntiles tiles to level s.
+__host__ __device__ __forceinline__ long long ada_refine_items(long long ntiles, int s) { return ntiles * s; }
+
+// refine_point as a call: inlined, its registers doubled the kernel's.
 template <typename T, bool GENERIC_SMOOTH>
-__global__ void __launch_bounds__(256) ada_refine_tiles(AdaGeom g, ShootParams sp, LeafPtrs lp, DescentPtrs<T> dp,
-                                                        const double2* __restrict__ base_verts,
-                                                        const int* __restrict__ tile_level,
-                                                        const int* __restrict__ list, int nlist, int s,
-                                                        long long stride, double2* __restrict__ out) {
-  __shared__ float4 s_near[kMaxStarsDirect];
-  __shared__ float2 s_coef[kMaxOrder];
-  __shared__ LeafView s_view;
-  const int nbands = (kAdaTile * s + 1 + kAdaBandRows - 1) / kAdaBandRows;
-  for (long long item = blockIdx.x; item < (long long)nlist * nbands; item += gridDim.x) {
-    const int slot = int(item / nbands), band = int(item - (long long)slot * nbands);
+__device__ __noinline__ double2 refine_point_call(const AdaGeom& g, const ShootParams& sp, const LeafPtrs& lp,
+                                                  const DescentPtrs<T>& dp, const double2* base_verts,
+                                                  const int* tile_level, int t, int s, int a, int b) {
+  const int tx = t % g.ntx, ty = t / g.ntx;
+  const int wa = int(llmin_(kAdaTile, g.ncx - (long long)tx * kAdaTile)) * s;
+  const int hb = int(llmin_(kAdaTile, g.ncy - (long long)ty * kAdaTile)) * s;
+  return refine_point<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tile_level, t, tx, ty, s, a, b, wa, hb);
+}
+
+template <typename T, bool GENERIC_SMOOTH>
+__global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refine_tiles(const __grid_constant__ AdaGeom g,
+                                                                const __grid_constant__ ShootParams sp,
+                                                                const __grid_constant__ LeafPtrs lp,
+                                                                const __grid_constant__ DescentPtrs<T> dp,
+                                                                const double2* __restrict__ base_verts,
+                                                                const int* __restrict__ tile_level,
+                                                                const int* __restrict__ list, int nlist, int s,
+                                                                long long stride, double2* __restrict__ out) {
+  constexpr int R = kAdaRows;
+  // per warp: the staged leaf (its constants are read back where they are used,
+  // which leaves the registers to the points)
+  __shared__ NearPairs s_pairs[kAdaThreads / 32];
+  __shared__ LeafView s_view[kAdaThreads / 32];
+  __shared__ double4 s_box[kAdaThreads / 32];  // lox, hix, loy, hiy
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  NearPairs& pairs = s_pairs[w];
+  const LeafView& L = s_view[w];
+  const double4& box = s_box[w];
+  const int sh = __ffs(s) - 1, fstep = kAdaMaxLevel >> sh;
+  if (lane == 0) s_box[w] = make_double4(1.0, 0.0, 1.0, 0.0);  // nothing staged: empty
+  __syncwarp();
+  for (long long item = blockIdx.x; item < ada_refine_items(nlist, s); item += gridDim.x) {
+    const int slot = int(item >> sh), band = int(item & (s - 1));
     const int t = list[slot];
-    const int leaf = dp.tile_leaf ? dp.tile_leaf[t] : -1;  // CTA-uniform
-    if (leaf >= 0) {
-      if (threadIdx.x < kMaxStarsDirect) s_near[threadIdx.x] = lp.near32[(size_t)leaf * kMaxStarsDirect + threadIdx.x];
-      if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxOrder)
-        s_coef[threadIdx.x - 64] = lp.coef32[(size_t)leaf * kMaxOrder + threadIdx.x - 64];
-      if (threadIdx.x == 0)
-        s_view = make_leaf_view(sp, s_near, s_coef, lp.nnear[leaf], lp.cx[leaf], lp.cy[leaf], lp.hl[leaf],
-                                lp.smooth0 ? lp.smooth0[leaf] : make_double2(0.0, 0.0));
-    }
-    __syncthreads();
-    const LeafView* stage = leaf >= 0 ? &s_view : nullptr;
     const int tx = t % g.ntx, ty = t / g.ntx;
     const int wa = int(llmin_(kAdaTile, g.ncx - (long long)tx * kAdaTile)) * s;
     const int hb = int(llmin_(kAdaTile, g.ncy - (long long)ty * kAdaTile)) * s;
-    const int w1 = wa + 1, b0 = band * kAdaBandRows, b1 = min(hb + 1, b0 + kAdaBandRows);
+    const int bb0 = band * kAdaBand;
+    if (bb0 >= hb) continue;  // a tile cut by the lattice's end
+    const int w1 = wa + 1;
     double2* o = out + (long long)slot * stride;
-    // corners (a, b) of the band in row-major order, thread k taking k, k + 256, ...
-    int b = b0 + int(threadIdx.x) / w1, a = int(threadIdx.x) - (b - b0) * w1;
-    while (b < b1) {
-      o[(long long)b * w1 + a] =
-          refine_point<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tile_level, t, tx, ty, s, a, b, wa, hb, stage);
-      a += blockDim.x;
-      while (a >= w1) {
-        a -= w1;
-        b++;
+    const long long i0 = (long long)tx * kAdaTile, j0 = (long long)ty * kAdaTile;
+    const int r0 = bb0 + w * R;
+    // first column or row shared with a coarser neighbour: point by point, at the end
+    const bool coarse_left = tile_level && tx > 0 && tile_level[t - 1] < s;
+    const bool coarse_low = bb0 == 0 && tile_level && ty > 0 && tile_level[t - g.ntx] < s;
+    auto coord_x = [&](int a) { return fine_coord(g.base_x, g.rhs_x, i0 * kAdaMaxLevel + (long long)a * fstep); };
+    auto coord_y = [&](int b) { return fine_coord(g.base_y, g.rhs_y, j0 * kAdaMaxLevel + (long long)b * fstep); };
+    if (r0 < hb) {
+      const int rlast = min(r0 + R, hb) - 1;
+      for (int a0 = 0; a0 < wa; a0 += 32) {
+        const int a = a0 + lane;
+        const double x = coord_x(a);
+        unsigned todo = a < wa ? (1u << (rlast - r0 + 1)) - 1u : 0u;  // the lane's rows still without a position
+        for (unsigned m; (m = __ballot_sync(0xffffffffu, todo != 0u)) != 0u;) {
+          // the first point left, and its leaf when it is not in the staged one
+          const int src = __ffs(m) - 1;
+          const double lx = __shfl_sync(0xffffffffu, x, src);
+          const double ly = coord_y(r0 + __ffs(__shfl_sync(0xffffffffu, todo, src)) - 1);
+          if (!(lx >= box.x && lx < box.y && ly >= box.z && ly < box.w)) {
+            const int node = descend_node(dp, lx, ly), leaf = int(dp.leaf_of_node[node]);
+            const int nn = lp.nnear[leaf];
+            __syncwarp();
+            float4 v = lp.near32[(size_t)leaf * kMaxStarsDirect + lane];
+            if (lane >= nn) v = make_float4(1e18f, 1e18f, 0.f, 0.f);  // far away, zero mass
+            pairs.xy[lane] = make_ulonglong2(pk2(v.x, v.x).v, pk2(v.y, v.y).v);
+            pairs.m[lane] = pk2(v.z, v.z).v;
+            if (lane < kMaxOrder) {
+              const float2 c = lp.coef32[(size_t)leaf * kMaxOrder + lane];
+              pairs.coef[lane] = make_ulonglong2(pk2(c.x, c.x).v, pk2(c.y, c.y).v);
+            }
+            if (lane == 0) {
+              s_view[w] = leaf_view(sp, lp, leaf);
+              s_box[w] = make_double4(dp.lox[node], dp.hix[node], dp.loy[node], dp.hiy[node]);
+            }
+            __syncwarp();
+          }
+          const float ux = float(x - L.cx);
+          float uy[R];
+          unsigned rows = 0u;  // rows inside the leaf's box
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const double y = coord_y(r0 + r);
+            uy[r] = float(y - L.cy);
+            if (y >= box.z && y < box.w) rows |= 1u << r;
+          }
+          const unsigned now = x >= box.x && x < box.y ? todo & rows : 0u;
+          todo &= ~now;
+          float sx[R], sy[R], cxr[R], cyr[R], Ar[R], Ai[R];
+          near_far_pairs<R>(ux, uy, L.inv_hl, (L.nn + 3) & ~3, sp.p, pairs, sx, sy, cxr, cyr, Ar, Ai);
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const int b = r0 + r;
+            if (!(now >> r & 1u) || (a == 0 && coarse_left) || (b == 0 && coarse_low)) continue;  // the last two below
+            double2 v;
+            if (((a | b) & (s - 1)) == 0) {  // base lattice points: the tiled pass's positions
+              v = base_verts[(j0 + (b >> sh)) * (g.ncx + 1) + i0 + (a >> sh)];
+            } else {
+              const float Sx = sx[r] + cxr[r], Sy = sy[r] + cyr[r];
+              const float wr = fmaf(float(L.lin_x), ux, -(Sx + Ar[r]));
+              const float wi = fmaf(float(L.lin_y), uy[r], -(Sy - Ai[r]));
+              double px = L.pcx + double(wr) * L.scx;
+              double py = L.pcy + double(wi) * L.scy;
+              if (GENERIC_SMOOTH) {
+                const cplx<double> corner = mk(sp.corner_re, sp.corner_im);
+                const cplx<double> z = mk(L.cx + double(ux), L.cy + double(uy[r]));
+                const cplx<double> a_sm =
+                    alpha_smooth_(z, sp.kstar, sp.rect, corner, sp.approx, sp.taylor_smooth, sp.inv_pi);
+                px += (-a_sm.re - sp.kstar * z.re) * L.scx;
+                py += (-a_sm.im - sp.kstar * z.im) * L.scy;
+              }
+              v = make_double2(px, double(sp.npy) - py);
+            }
+            o[(long long)b * w1 + a] = v;
+          }
+        }
       }
     }
-    __syncthreads();  // the stage is rewritten for the next tile
+    // point by point: the last column of the band's rows, the first one where it
+    // is shared with a coarser neighbour, the same for the tile's rows
+    const int blast = min(bb0 + kAdaBand, hb), ncol = blast - bb0;
+    const int n1 = ncol, n2 = n1 + (coarse_left ? ncol : 0), n3 = n2 + (coarse_low ? wa : 0);
+    const int n = n3 + (blast == hb ? w1 : 0);
+    for (int k = threadIdx.x; k < n; k += kAdaThreads) {
+      const int a = k < n1 ? wa : (k < n2 ? 0 : (k < n3 ? k - n2 : k - n3));
+      const int b = k < n1 ? bb0 + k : (k < n2 ? bb0 + k - n1 : (k < n3 ? 0 : hb));
+      o[(long long)b * w1 + a] = refine_point_call<T, GENERIC_SMOOTH>(g, sp, lp, dp, base_verts, tile_level, t, s, a, b);
+    }
   }
 }
 

@@ -181,7 +181,8 @@ class AdaptiveIPM {
 
   DescentPtrs<T> descent() const {
     return DescentPtrs<T>{base.tree_.cx.p, base.tree_.cy.p, base.tree_.child0.p, base.leaves_.pos.p,
-                          tile_leaf_ready_ ? d_tile_leaf_.p : nullptr};
+                          tile_leaf_ready_ ? d_tile_leaf_.p : nullptr, base.tree_.lox.p, base.tree_.hix.p,
+                          base.tree_.loy.p, base.tree_.hiy.p};
   }
 
   int tile_cells_x(int t) const { return int(std::min<long long>(kAdaTile, g_.ncx - (long long)(t % ntx) * kAdaTile)); }
@@ -277,12 +278,12 @@ class AdaptiveIPM {
     std::vector<DepositPiece<float>> pieces;
     for (size_t k0 = 0; k0 < tiles.size(); k0 += chunk) {
       const int n = int(std::min<size_t>(chunk, tiles.size() - k0));
-      const int grid = int(std::max<long long>(1, std::min<long long>(ada_band_items(n, kAdaMaxLevel), 148LL * 8)));
+      const int grid = int(std::max<long long>(1, std::min<long long>(ada_refine_items(n, kAdaMaxLevel), 148LL * 64)));
       if (generic_)
-        ada_refine_tiles<T, true><<<grid, 256, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
+        ada_refine_tiles<T, true><<<grid, kAdaThreads, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
                                                        nullptr, d_list_.p + k0, n, kAdaMaxLevel, per, d_ref_.p);
       else
-        ada_refine_tiles<T, false><<<grid, 256, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
+        ada_refine_tiles<T, false><<<grid, kAdaThreads, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
                                                         nullptr, d_list_.p + k0, n, kAdaMaxLevel, per, d_ref_.p);
       ada_tile_windows<<<std::min(n, 148 * 8), 256, 0, s>>>(g_, d_list_.p + k0, n, per, d_ref_.p, d_win_.p);
       IRSB_LAUNCH_CK("ada windows");
@@ -544,13 +545,13 @@ class AdaptiveIPM {
         verts = d_ref_.p;
       } else if (L.s > 1) {
         const long long per = (long long)(kAdaTile * L.s + 1) * (kAdaTile * L.s + 1);
-        const int grid = int(std::max<long long>(1, std::min<long long>(ada_band_items(L.nlist, L.s), 148LL * 8)));
+        const int grid = int(std::max<long long>(1, std::min<long long>(ada_refine_items(L.nlist, L.s), 148LL * 64)));
         if (generic_)
-          ada_refine_tiles<T, true><<<grid, 256, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
+          ada_refine_tiles<T, true><<<grid, kAdaThreads, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
                                                          d_level_.p, d_list_.p + L.list_off, L.nlist, L.s, per,
                                                          d_ref_.p);
         else
-          ada_refine_tiles<T, false><<<grid, 256, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
+          ada_refine_tiles<T, false><<<grid, kAdaThreads, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
                                                           d_level_.p, d_list_.p + L.list_off, L.nlist, L.s, per,
                                                           d_ref_.p);
         IRSB_LAUNCH_CK("ada_refine_tiles");

@@ -47,10 +47,12 @@ struct DescentPtrs {
   const int* child0;
   const long long* leaf_of_node;  // exclusive scan of the leaf flags
   const int* tile_leaf;           // per tile: the leaf owning all its points, or -1 (nullptr: not known)
+  // the half-open box of points that the descent maps to the node (adaptive refinement)
+  const double *lox = nullptr, *hix = nullptr, *loy = nullptr, *hiy = nullptr;
 };
 
 template <typename T>
-__device__ __forceinline__ int descend_leaf(const DescentPtrs<T>& d, double x, double y) {
+__device__ __forceinline__ int descend_node(const DescentPtrs<T>& d, double x, double y) {
   int k = 0;
   for (int it = 0; it < kMaxLevels + 1; it++) {
     const int c0 = d.child0[k];
@@ -59,7 +61,11 @@ __device__ __forceinline__ int descend_leaf(const DescentPtrs<T>& d, double x, d
     const bool right = x >= cx, top = y >= cy;
     k = c0 + (right ? (top ? 0 : 3) : (top ? 1 : 2));
   }
-  return int(d.leaf_of_node[k]);
+  return k;
+}
+template <typename T>
+__device__ __forceinline__ int descend_leaf(const DescentPtrs<T>& d, double x, double y) {
+  return int(d.leaf_of_node[descend_node(d, x, y)]);
 }
 
 constexpr int kTileX = 32;
