@@ -449,57 +449,66 @@ constexpr int kAdaWindowLarge = 512;  // window of a chunk holding a tile whose 
 constexpr int kAdaWindowMargin = 2;
 constexpr double kAdaMapWeight = 20.0;  // mode 2: weight of the map-relative error
 
-// Window of each tile: the pixel bounding box of its level-16 image within the
-// map, widened by kAdaWindowMargin; win[slot] = (x0, y0, w, h), w = 0 when the
-// image misses the map. A box wider than the chunk's window is covered at a
-// coarser pixel scale (ada_window_scale).
-__global__ void __launch_bounds__(256) ada_tile_windows(AdaGeom g, const int* __restrict__ list, int nlist,
-                                                        long long stride, const double2* __restrict__ fine,
-                                                        int4* __restrict__ win) {
-  __shared__ double red[4][8];
-  for (int slot = blockIdx.x; slot < nlist; slot += gridDim.x) {
-    const int t = list[slot];
-    const int tx = t % g.ntx, ty = t / g.ntx;
-    const int ncx_t = int(llmin_(kAdaTile, g.ncx - (long long)tx * kAdaTile));
-    const int ncy_t = int(llmin_(kAdaTile, g.ncy - (long long)ty * kAdaTile));
-    const int n = (ncx_t * kAdaMaxLevel + 1) * (ncy_t * kAdaMaxLevel + 1);
-    const double2* P = fine + (long long)slot * stride;
-    double m[4] = {1e300, 1e300, -1e300, -1e300};  // xmin, ymin, xmax, ymax
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-      const double2 v = P[q];
-      if (!(fabs(v.x) < 1e12 && fabs(v.y) < 1e12)) continue;
-      m[0] = fmin(m[0], v.x);
-      m[1] = fmin(m[1], v.y);
-      m[2] = fmax(m[2], v.x);
-      m[3] = fmax(m[3], v.y);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      double v = m[c];
-      for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_down_sync(0xffffffffu, v, o);
-        v = c < 2 ? fmin(v, u) : fmax(v, u);
-      }
-      if ((threadIdx.x & 31) == 0) red[c][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double r[4] = {red[0][0], red[1][0], red[2][0], red[3][0]};
-      for (int w = 1; w < int(blockDim.x >> 5); w++) {
-        r[0] = fmin(r[0], red[0][w]);
-        r[1] = fmin(r[1], red[1][w]);
-        r[2] = fmax(r[2], red[2][w]);
-        r[3] = fmax(r[3], red[3][w]);
-      }
-      const double x0 = fmax(floor(r[0]) - kAdaWindowMargin, 0.0), y0 = fmax(floor(r[1]) - kAdaWindowMargin, 0.0);
-      const double x1 = fmin(ceil(r[2]) + kAdaWindowMargin, double(g.npx));
-      const double y1 = fmin(ceil(r[3]) + kAdaWindowMargin, double(g.npy));
-      int4 o = make_int4(0, 0, 0, 0);
-      if (x1 > x0 && y1 > y0) o = make_int4(int(x0), int(y0), int(x1 - x0), int(y1 - y0));
-      win[slot] = o;
-    }
-    __syncthreads();
+// Unsigned key of a double in the doubles' order.
+__device__ __forceinline__ unsigned long long ordered_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b >> 63 ? ~b : b | (1ull << 63);
+}
+__device__ __forceinline__ double key_value(unsigned long long k) {
+  return __longlong_as_double((long long)(k >> 63 ? k & ~(1ull << 63) : ~k));
+}
+
+// Pixel bounding box of each tile's level-16 image, as ordered keys (xmin, ymin
+// inverted, xmax, ymax: all maxima, zeroed before): kAdaParts CTAs per tile.
+// Bound by reading the corners; with one CTA for a tile's 2.6e5 corners a launch
+// of 64 tiles left more than half of the chip idle (B200, 922 tiles: 9.1 ms,
+// now 0.9 ms).
+constexpr int kAdaParts = 16;
+__global__ void __launch_bounds__(256) ada_tile_bounds(AdaGeom g, const int* __restrict__ list, long long stride,
+                                                       const double2* __restrict__ fine,
+                                                       unsigned long long* __restrict__ keys) {
+  const int slot = blockIdx.y, t = list[slot];
+  const int tx = t % g.ntx, ty = t / g.ntx;
+  const int ncx_t = int(llmin_(kAdaTile, g.ncx - (long long)tx * kAdaTile));
+  const int ncy_t = int(llmin_(kAdaTile, g.ncy - (long long)ty * kAdaTile));
+  const int n = (ncx_t * kAdaMaxLevel + 1) * (ncy_t * kAdaMaxLevel + 1);
+  const double2* P = fine + (long long)slot * stride;
+  double m[4] = {1e300, 1e300, -1e300, -1e300};  // xmin, ymin, xmax, ymax
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const double2 v = P[q];
+    if (!(fabs(v.x) < 1e12 && fabs(v.y) < 1e12)) continue;
+    m[0] = fmin(m[0], v.x);
+    m[1] = fmin(m[1], v.y);
+    m[2] = fmax(m[2], v.x);
+    m[3] = fmax(m[3], v.y);
   }
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    double v = m[c];
+    for (int o = 16; o > 0; o >>= 1) {
+      const double u = __shfl_down_sync(0xffffffffu, v, o);
+      v = c < 2 ? fmin(v, u) : fmax(v, u);
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(&keys[slot * 4 + c], c < 2 ? ~ordered_key(v) : ordered_key(v));
+  }
+}
+
+// Window of each tile: that bounding box within the map, widened by
+// kAdaWindowMargin; win[slot] = (x0, y0, w, h), w = 0 when the image misses the
+// map. A box wider than the chunk's window is covered at a coarser pixel scale
+// (ada_window_scale).
+__global__ void ada_tile_windows(AdaGeom g, int nlist, const unsigned long long* __restrict__ keys,
+                                 int4* __restrict__ win) {
+  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot >= nlist) return;
+  const unsigned long long* k = keys + slot * 4;
+  const double r[4] = {key_value(~k[0]), key_value(~k[1]), key_value(k[2]), key_value(k[3])};
+  const double x0 = fmax(floor(r[0]) - kAdaWindowMargin, 0.0), y0 = fmax(floor(r[1]) - kAdaWindowMargin, 0.0);
+  const double x1 = fmin(ceil(r[2]) + kAdaWindowMargin, double(g.npx));
+  const double y1 = fmin(ceil(r[3]) + kAdaWindowMargin, double(g.npy));
+  int4 o = make_int4(0, 0, 0, 0);
+  if (x1 > x0 && y1 > y0) o = make_int4(int(x0), int(y0), int(x1 - x0), int(y1 - y0));
+  win[slot] = o;
 }
 
 // Map pixels per window pixel for a tile's window (1 unless its image is
@@ -509,10 +518,71 @@ __host__ __device__ __forceinline__ int ada_window_scale(int4 w, int ws) {
   return m <= ws ? 1 : (m + ws - 1) / ws;
 }
 
-// Differences of the resolved windows of side ws (window of slot k, level c
-// at acc + (k * 5 + c) * ws^2, placed at (win.x, win.y) on the map): the flux
-// the tile puts in other map pixels at level 2^c than at level 16, as a share
-// of
+// Sums of the differences of the windows of side ws (window of slot k, level c:
+// pieces at acc + (k * 5 + c) * ws^2, row differences at diff + (k * 5 + c) *
+// ws (ws + 1), placed at (win.x, win.y) on the map): sums[k * 5 + c] = sum
+// |W_c - W_16| over the map pixels, c < 4, and sums[k * 5 + 4] the reference
+// flux of mode >= 1 (below). A warp per row resolves the five levels' row sums
+// side by side; only the rows and columns of the tile's box are visited (nothing
+// is deposited beyond them). Integer sums: their order does not matter.
+// One CTA per tile over the whole resolved windows took 16.2 ms for 922 tiles,
+// and the pass that resolved them 5.7 ms (B200); now 2.2 ms together.
+__global__ void __launch_bounds__(256) ada_window_sums(AdaGeom g, int ws, int mode, const int4* __restrict__ win,
+                                                       const unsigned long long* __restrict__ acc,
+                                                       const unsigned long long* __restrict__ diff,
+                                                       const unsigned long long* __restrict__ ref,
+                                                       unsigned long long* __restrict__ sums) {
+  const int slot = blockIdx.y, lane = threadIdx.x & 31;
+  const int4 w = win[slot];
+  if (w.z <= 0) return;  // uniform over the block
+  const int k = ada_window_scale(w, ws);
+  const int nx = (w.z + k - 1) / k, ny = (w.w + k - 1) / k;
+  const long long W2 = (long long)ws * ws, WD = (long long)ws * (ws + 1);
+  const unsigned long long* A = acc + (long long)slot * 5 * W2;
+  const unsigned long long* Q = diff + (long long)slot * 5 * WD;
+  unsigned long long d[5] = {0, 0, 0, 0, 0};
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < ny; row += (gridDim.x * blockDim.x) >> 5) {
+    unsigned long long carry[5] = {0, 0, 0, 0, 0};
+    for (int x0 = 0; x0 < nx; x0 += 32) {
+      const int x = x0 + lane;
+      unsigned long long v[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) v[c] = x < nx ? Q[c * WD + (long long)row * (ws + 1) + x] : 0ULL;
+      long long a[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long u = __shfl_up_sync(0xffffffffu, v[c], o);
+          if (lane >= o) v[c] += u;
+        }
+        v[c] += carry[c];
+        carry[c] = __shfl_sync(0xffffffffu, v[c], 31);
+        a[c] = x < nx ? (long long)(A[c * W2 + (long long)row * ws + x] + v[c]) : 0;
+      }
+      bool touched = a[4] != 0;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        touched = touched || a[c] != 0;
+        d[c] += (unsigned long long)llabs(a[c] - a[4]);
+      }
+      // where the plain map holds less than the tile's own flux, the tile's
+      // flux is the reference
+      if (mode >= 1 && touched) {
+        const long long rv = (long long)ref[(long long)(w.y + row * k) * g.npx + w.x + x * k];
+        d[4] += (unsigned long long)(rv > a[4] ? rv : a[4]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 5; c++) {
+    for (int o = 16; o > 0; o >>= 1) d[c] += __shfl_down_sync(0xffffffffu, d[c], o);
+    if (lane == 0 && d[c]) atomicAdd(&sums[slot * 5 + c], d[c]);
+  }
+}
+
+// err[slot * 4 + c]: the flux a tile puts in other map pixels at level 2^c than
+// at level 16, as a share of
 //   mode 0: the tile's whole flux (2 factor per cell): its own relative error,
 //           which the map inherits where the errors of overlapping tiles have
 //           the same sign (the bias of the triangle approximation);
@@ -525,60 +595,22 @@ __host__ __device__ __forceinline__ int ada_window_scale(int4 w, int ws) {
 //           when its error is a small part of the map where it lands (images
 //           close to a star, stretched thin over pixels that other images
 //           fill).
-__global__ void __launch_bounds__(256) ada_window_errors(AdaGeom g, const int* __restrict__ list, int nlist, int ws,
-                                                         float factor, int mode, const int4* __restrict__ win,
-                                                         const unsigned long long* __restrict__ acc,
-                                                         const unsigned long long* __restrict__ ref,
-                                                         float* __restrict__ err) {
-  __shared__ double red[5][8];
-  const long long W2 = (long long)ws * ws;
-  for (int slot = blockIdx.x; slot < nlist; slot += gridDim.x) {
-    const int4 w = win[slot];
-    if (w.z <= 0) {  // uniform over the block
-      if (threadIdx.x < 4) err[(long long)slot * 4 + threadIdx.x] = 0.f;
-      continue;
-    }
-    const int k = ada_window_scale(w, ws);
-    const unsigned long long* A = acc + (long long)slot * 5 * W2;
-    double d[4] = {0, 0, 0, 0}, tot = 0;
-    for (long long q = threadIdx.x; q < W2; q += blockDim.x) {
-      const int x = w.x + int(q % ws) * k, y = w.y + int(q / ws) * k;
-      if (x >= g.npx || y >= g.npy) continue;  // the window runs past the map's edge
-      const long long a16 = (long long)A[4 * W2 + q];
-      bool touched = a16 != 0;
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const long long ac = (long long)A[c * W2 + q];
-        touched = touched || ac != 0;
-        d[c] += fabs(double(ac - a16));
-      }
-      // where the plain map holds less than the tile's own flux, the tile's
-      // flux is the reference
-      if (touched && mode >= 1) tot += fmax(double((long long)ref[(long long)y * g.npx + x]), double(a16));
-    }
-#pragma unroll
-    for (int c = 0; c < 5; c++) {
-      double v = c < 4 ? d[c] : tot;
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if ((threadIdx.x & 31) == 0) red[c][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-      double num = 0, den = 0;
-      for (int k = 0; k < int(blockDim.x >> 5); k++) {
-        num += red[threadIdx.x][k];
-        den += red[4][k];
-      }
-      const int t = list[slot];
-      const long long cells = llmin_(kAdaTile, g.ncx - (long long)(t % g.ntx) * kAdaTile) *
-                              llmin_(kAdaTile, g.ncy - (long long)(t / g.ntx) * kAdaTile);
-      const double own = double(cells) * 2.0 * double(factor) * kFixScale;
-      const double e_map = den > 0 ? num / den : (num > 0 ? 1.0 : 0.0);
-      const double e = mode == 0 ? num / own : (mode == 1 ? e_map : fmin(num / own, kAdaMapWeight * e_map));
-      err[(long long)slot * 4 + threadIdx.x] = float(e);
-    }
-    __syncthreads();
+__global__ void ada_window_errors(AdaGeom g, const int* __restrict__ list, int nlist, float factor, int mode,
+                                  const int4* __restrict__ win, const unsigned long long* __restrict__ sums,
+                                  float* __restrict__ err) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, slot = q >> 2, c = q & 3;
+  if (slot >= nlist) return;
+  if (win[slot].z <= 0) {
+    err[q] = 0.f;
+    return;
   }
+  const int t = list[slot];
+  const long long cells = llmin_(kAdaTile, g.ncx - (long long)(t % g.ntx) * kAdaTile) *
+                          llmin_(kAdaTile, g.ncy - (long long)(t / g.ntx) * kAdaTile);
+  const double num = double(sums[slot * 5 + c]), den = double(sums[slot * 5 + 4]);
+  const double own = double(cells) * 2.0 * double(factor) * kFixScale;
+  const double e_map = den > 0 ? num / den : (num > 0 ? 1.0 : 0.0);
+  err[q] = float(mode == 0 ? num / own : (mode == 1 ? e_map : fmin(num / own, kAdaMapWeight * e_map)));
 }
 
 // Per-tile features from the base corner lattice and the tree (one thread per

@@ -161,7 +161,7 @@ class AdaptiveIPM {
   DevVec<int4> d_win_;
   DevVec<int> d_slot_;
   LatticeTiles rtiles_;  // lattice tiles of a refinement pass
-  DevVec<unsigned long long> d_acc_, d_diff_, d_wacc_, d_wdiff_, d_bacc_, d_bdiff_;
+  DevVec<unsigned long long> d_acc_, d_diff_, d_wacc_, d_wdiff_, d_bacc_, d_bdiff_, d_wkeys_, d_wsums_;
   bool base_map_ready_ = false;
   DevVec<T> d_map_;
   DevVec<int> d_tile_leaf_;  // per tile: the leaf owning all its points, or -1
@@ -271,7 +271,8 @@ class AdaptiveIPM {
     const int chunk = int(std::max<long long>(1, std::min<long long>(64, buffer_cap() / per)));
     const int nc = int(std::min<size_t>(chunk, tiles.size()));
     if (!d_ref_.alloc_exact(nc * per) || !d_list_.alloc_exact(tiles.size()) || !d_err_.alloc_exact(tiles.size() * 4) ||
-        !d_win_.alloc_exact(nc) || !d_pieces_.alloc_exact(nc * 5))
+        !d_win_.alloc_exact(nc) || !d_pieces_.alloc_exact(nc * 5) || !d_wkeys_.alloc_exact(nc * 4) ||
+        !d_wsums_.alloc_exact(nc * 5))
       return false;
     IRSB_CKR(cudaMemcpyAsync(d_list_.p, tiles.data(), tiles.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     std::vector<int4> win(nc);
@@ -285,7 +286,9 @@ class AdaptiveIPM {
       else
         ada_refine_tiles<T, false><<<grid, kAdaThreads, 0, s>>>(g_, sp_, base.leaf_ptrs(), descent(), base.d_verts_.p,
                                                         nullptr, d_list_.p + k0, n, kAdaMaxLevel, per, d_ref_.p);
-      ada_tile_windows<<<std::min(n, 148 * 8), 256, 0, s>>>(g_, d_list_.p + k0, n, per, d_ref_.p, d_win_.p);
+      IRSB_CKR(cudaMemsetAsync(d_wkeys_.p, 0, n * 4 * sizeof(unsigned long long), s));
+      ada_tile_bounds<<<dim3(kAdaParts, n), 256, 0, s>>>(g_, d_list_.p + k0, per, d_ref_.p, d_wkeys_.p);
+      ada_tile_windows<<<ceil_div(n, 64), 64, 0, s>>>(g_, n, d_wkeys_.p, d_win_.p);
       IRSB_LAUNCH_CK("ada windows");
       IRSB_CKR(cudaMemcpyAsync(win.data(), d_win_.p, n * sizeof(int4), cudaMemcpyDeviceToHost, s));
       IRSB_CKR(cudaStreamSynchronize(s));
@@ -328,11 +331,12 @@ class AdaptiveIPM {
         const int gd = deposit_grid(nchunks);
         ipm_deposit_batch<float><<<gd, kDepositThreads, 0, s>>>(d_ref_.p, d_pieces_.p, int(pieces.size()), nchunks, ws, ws, M,
                                                     W2, WD);
-        const int gr = std::max(1, std::min(ceil_div((long long)ws * 5 * n * 32, 256), 148 * 8));
-        ipm_resolve_rows<<<gr, 256, 0, s>>>(ws, ws * 5 * n, M);
       }
-      ada_window_errors<<<std::min(n, 148 * 8), 256, 0, s>>>(g_, d_list_.p + k0, n, ws, factor, err_mode, d_win_.p,
-                                                            d_wacc_.p, d_bacc_.p, d_err_.p + k0 * 4);
+      IRSB_CKR(cudaMemsetAsync(d_wsums_.p, 0, n * 5 * sizeof(unsigned long long), s));
+      ada_window_sums<<<dim3(kAdaParts, n), 256, 0, s>>>(g_, ws, err_mode, d_win_.p, d_wacc_.p, d_wdiff_.p, d_bacc_.p,
+                                                         d_wsums_.p);
+      ada_window_errors<<<ceil_div(n * 4, 64), 64, 0, s>>>(g_, d_list_.p + k0, n, factor, err_mode, d_win_.p, d_wsums_.p,
+                                                           d_err_.p + k0 * 4);
       IRSB_LAUNCH_CK("ada window errors");
       IRSB_CKR(cudaStreamSynchronize(s));  // the host pieces are rebuilt for the next chunk
     }
