@@ -222,7 +222,8 @@ __device__ __forceinline__ void setup_tail(Tri<D>& t, D factor) {
 // by row (one array per field: lane k touches word k, no bank conflicts).
 template <typename D>
 struct TriSlots {
-  D x[3][64], y[3][64], area[64];
+  D x[3][64], y[3][64], scale[64];  // scale: the area until setup_tail
+  D idy[3][64], sl[3][64];          // from setup_tail
   int ox[64], oy[64], rlo[64], nrows[64], map[64];
   __device__ __forceinline__ void put(int k, const Tri<D>& t) {
 #pragma unroll
@@ -230,26 +231,40 @@ struct TriSlots {
       x[q][k] = t.x[q];
       y[q][k] = t.y[q];
     }
-    area[k] = t.scale;
+    scale[k] = t.scale;
     ox[k] = t.ox;
     oy[k] = t.oy;
     rlo[k] = t.rlo;
     nrows[k] = t.nrows;
     map[k] = t.map;
   }
-  __device__ __forceinline__ void get(int k, Tri<D>& t) const {
+  __device__ __forceinline__ void put_tail(int k, const Tri<D>& t) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      idy[q][k] = t.idy[q];
+      sl[q][k] = t.sl[q];
+    }
+    scale[k] = t.scale;
+  }
+  __device__ __forceinline__ void get_head(int k, Tri<D>& t) const {
 #pragma unroll
     for (int q = 0; q < 3; q++) {
       t.x[q] = x[q][k];
       t.y[q] = y[q][k];
     }
-    t.scale = area[k];
+    t.scale = scale[k];
     t.ox = ox[k];
     t.oy = oy[k];
     t.rlo = rlo[k];
-    t.nrows = nrows[k];
     t.map = map[k];
-    t.single = 0;
+  }
+  __device__ __forceinline__ void get(int k, Tri<D>& t) const {
+    get_head(k, t);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      t.idy[q] = idy[q][k];
+      t.sl[q] = sl[q][k];
+    }
   }
 };
 constexpr int kDepositWarps = 2;  // warps per CTA of the deposition kernels
@@ -398,21 +413,28 @@ __device__ __forceinline__ void deposit_row(const Tri<D>& t, int r, int npx, con
   }
 }
 
-// The rows of the triangles of a warp, one triangle per lane (nrows = 0: none):
-// each lane deposits its own triangle's first row; the warp then scans the
-// counts of the remaining rows and works through those (triangle, row) items
-// 32 at a time, each lane finding its item's owner lane by a binary search
-// over the scan and reading the triangle through shuffles, so a triangle with
-// many rows is spread over the warp instead of holding one lane.
+// The rows of the staged triangles [k0, k0 + 32) of a warp, one triangle per lane
+// (n staged in all): each lane finishes its own triangle (setup_tail) and
+// deposits its first row; the warp then scans the counts of the remaining rows
+// and works through those (triangle, row) items 32 at a time, each lane finding
+// its item's owner by a binary search over the scan and reading the triangle
+// from the slots (consecutive words: no bank conflicts), so a triangle with many
+// rows is spread over the warp instead of holding one lane, and no triangle is
+// held in registers across the rows.
 template <typename D>
-__device__ __forceinline__ void deposit_rows_warp(const Tri<D>& mine, int npx, const DepositMaps& m_total,
-                                                  const DepositMaps& m_min, const DepositMaps& m_sad) {
+__device__ __forceinline__ void deposit_rows_warp(TriSlots<D>& stage, int k0, int n, D factor, int npx,
+                                                  const DepositMaps& m_total, const DepositMaps& m_min,
+                                                  const DepositMaps& m_sad) {
   const int lane = threadIdx.x & 31;
-  if (mine.nrows > 0) {
-    const DepositMaps& M = mine.map == 0 ? m_total : (mine.map == 1 ? m_min : m_sad);
-    deposit_row<D>(mine, mine.rlo, npx, M);
+  int extra = 0;
+  if (k0 + lane < n) {
+    Tri<D> t;
+    stage.get_head(k0 + lane, t);
+    setup_tail(t, factor);
+    extra = stage.nrows[k0 + lane] - 1;
+    if (extra > 0) stage.put_tail(k0 + lane, t);
+    deposit_row<D>(t, t.rlo, npx, t.map == 0 ? m_total : (t.map == 1 ? m_min : m_sad));
   }
-  const int extra = mine.nrows > 1 ? mine.nrows - 1 : 0;
   int incl = extra;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -420,6 +442,7 @@ __device__ __forceinline__ void deposit_rows_warp(const Tri<D>& mine, int npx, c
     if (lane >= o) incl += v;
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
+  __syncwarp();
   for (int it0 = 0; it0 < total; it0 += 32) {
     const int item = it0 + lane;
     int lo = 0, hi = 31;  // owner: first lane whose inclusive count exceeds item
@@ -430,24 +453,12 @@ __device__ __forceinline__ void deposit_rows_warp(const Tri<D>& mine, int npx, c
       if (v > item) hi = mid;
       else lo = mid + 1;
     }
-    const int owner = lo;
+    const int owner = lo & 31;
     const int before = __shfl_sync(0xffffffffu, incl - extra, owner);
-    Tri<D> t;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      t.x[q] = __shfl_sync(0xffffffffu, mine.x[q], owner);
-      t.y[q] = __shfl_sync(0xffffffffu, mine.y[q], owner);
-      t.sl[q] = __shfl_sync(0xffffffffu, mine.sl[q], owner);
-      t.idy[q] = __shfl_sync(0xffffffffu, mine.idy[q], owner);
-    }
-    t.scale = __shfl_sync(0xffffffffu, mine.scale, owner);
-    t.ox = __shfl_sync(0xffffffffu, mine.ox, owner);
-    t.oy = __shfl_sync(0xffffffffu, mine.oy, owner);
-    t.rlo = __shfl_sync(0xffffffffu, mine.rlo, owner);
-    t.map = __shfl_sync(0xffffffffu, mine.map, owner);
     if (item < total) {
-      const DepositMaps& M = t.map == 0 ? m_total : (t.map == 1 ? m_min : m_sad);
-      deposit_row<D>(t, t.rlo + 1 + (item - before), npx, M);
+      Tri<D> t;
+      stage.get(k0 + owner, t);
+      deposit_row<D>(t, t.rlo + 1 + (item - before), npx, t.map == 0 ? m_total : (t.map == 1 ? m_min : m_sad));
     }
   }
 }
@@ -548,15 +559,7 @@ __device__ __forceinline__ void deposit_warp_cells(const double2* __restrict__ v
   __syncwarp();
   // the staged ones go row by row, one per lane: one round when at most 32
   // of the warp's 64 triangles need it (fine lattices), else two
-  for (int r0 = 0; r0 < n; r0 += 32) {
-    Tri<D> mine;
-    mine.nrows = 0;
-    if (r0 + lane < n) {
-      stage.get(r0 + lane, mine);
-      setup_tail(mine, factor);
-    }
-    deposit_rows_warp<D>(mine, npx, m_total, m_min, m_sad);
-  }
+  for (int k0 = 0; k0 < n; k0 += 32) deposit_rows_warp<D>(stage, k0, n, factor, npx, m_total, m_min, m_sad);
   __syncwarp();  // slots free for the warp's next cells
 }
 
