@@ -32,6 +32,7 @@
 #pragma once
 #include "common.cuh"
 
+#include <algorithm>
 #include <limits>
 
 namespace irsb {
@@ -269,11 +270,30 @@ struct TriSlots {
 };
 constexpr int kDepositWarps = 2;  // warps per CTA of the deposition kernels
 constexpr int kDepositThreads = kDepositWarps * 32;
-// Grid of the deposition kernels over nchunks 32-cell chunks: one warp per
-// chunk, at most 256 CTAs per SM (148 SMs), the warps striding over the rest.
-// Small CTAs retire as soon as their two warps are done, so the SMs stay full
-// to the end: 6.25 ms against 6.72 ms with 8-warp CTAs at 16 per SM on the
-// 2000-pixel bench workload, maps bit-identical.
+// Order of the deposition's work units (32-cell chunks, or blocks of them) over
+// at most 256 CTAs per SM. CTAs start in order, so about kWave warps are at work
+// at a time; the warps of such a wave share one stretch of the lattice, striding
+// through it (neighbouring warps on neighbouring units, each warp's units spread
+// over the stretch, which evens out the cells' cost). The stretch's images share
+// a part of the map, whose words stay in L2. With the warps striding over the
+// whole lattice every wave swept it end to end, and its adds missed L2 where the
+// fixed-point map is larger: 1.0e9 cells into 4096^2 pixels (268 MB of map
+// words) took 168 ms, now 81.5 (B200); with consecutive units per warp 92 ms,
+// but 5.3 against 4.9 ms for 8.8e7 cells into 2000^2 pixels. Small CTAs retire
+// as soon as their two warps are done, which keeps the SMs full to the end.
+struct DepositOrder {
+  long long first, stride;  // this warp's first unit and the step to its next
+  int count;                // units (those past the last unit are absent)
+};
+template <typename D>
+__device__ __forceinline__ DepositOrder deposit_order(long long nunits) {
+  constexpr long long kWave = 148LL * (sizeof(D) == 4 ? 16 : 8) * kDepositWarps;  // resident warps
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long count = (nunits + nwarps - 1) / nwarps, wave = w / kWave, in = w - wave * kWave;
+  const long long size = nwarps - wave * kWave < kWave ? nwarps - wave * kWave : kWave;
+  return {wave * kWave * count + in, size, int(count)};
+}
 inline int deposit_grid(long long nchunks) {
   const long long ctas = (nchunks + kDepositWarps - 1) / kDepositWarps, cap = 148LL * 256;
   return int(ctas < 1 ? 1 : (ctas > cap ? cap : ctas));
@@ -311,7 +331,8 @@ inline int deposit_grid(long long nchunks) {
 // Bound by instruction issue (FP32 and ALU pipes). Against the form that
 // clamped both segment ends for every pixel and computed both chords of every
 // row: 8.76e7 cells of a 2000^2 map 6.36 -> 4.91 ms (FP32), 4.1e7 cells 2.61 ->
-// 2.45 ms (FP64), maps bit-identical (B200).
+// 2.45 ms (FP64), maps bit-identical (B200); 4.63 and 2.28 ms with the triangles
+// read back from the slots (deposit_rows_warp) and deposit_order.
 template <typename D>
 __device__ __forceinline__ void deposit_row(const Tri<D>& t, int r, int npx, const DepositMaps& M) {
   const D rb = D(r), rt = D(r + 1);
@@ -564,7 +585,7 @@ __device__ __forceinline__ void deposit_warp_cells(const double2* __restrict__ v
 }
 
 // Cells of an ncx x ncy lattice whose (ncx+1) x (ncy+1) corner positions are in
-// `verts`. A warp takes 32 consecutive cells; each lane classifies the two
+// `verts`. A warp takes 32 consecutive cells at a time (deposit_order); each lane classifies the two
 // triangles of its cell (setup_head); a triangle inside one pixel is
 // deposited at once; the others are staged in shared memory, compacted, and
 // then get their reciprocals and scale (setup_tail) and go row by row
@@ -575,11 +596,11 @@ __global__ void __launch_bounds__(kDepositThreads, sizeof(D) == 4 ? 16 : 8)
     ipm_deposit_cells(const double2* __restrict__ verts, long long ncx, long long ncy, D factor, int npx, int npy,
                       DepositMaps m_total, DepositMaps m_min, DepositMaps m_sad, int parities) {
   const long long ncells = ncx * ncy;
-  const long long warp0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   __shared__ TriSlots<D> slots[kDepositWarps];
   TriSlots<D>& stage = slots[threadIdx.x >> 5];
-  for (long long base = warp0 * 32; base < ncells; base += nwarps * 32)
+  const DepositOrder o = deposit_order<D>((ncells + 31) / 32);
+  long long base = o.first * 32;
+  for (int i = 0; i < o.count && base < ncells; i++, base += o.stride * 32)
     deposit_warp_cells<D>(verts, ncx, ncx + 1, ncells, base, factor, npx, npy, m_total, m_min, m_sad, parities, stage);
 }
 
@@ -598,22 +619,22 @@ struct DepositPiece {
   int r;               // realization (map index)
 };
 
-// Batched deposition: the warps stride over blocks of 8 consecutive 32-cell
-// chunks of all pieces of the pass; a block's first piece is found by a
-// binary search over chunk0 and the next chunks advance from it (one search
-// per 8 chunks: 1.79 against 1.88 s for the 4096-pixel adaptive map).
-// Realization r accumulates into the maps at r * map_stride / r * diff_stride.
+// Batched deposition over the 32-cell chunks of all pieces of the pass, in blocks
+// of 8 consecutive ones (deposit_order): a block's first piece is found by a
+// binary search over chunk0 and the next chunks advance from it (one search per
+// 8 chunks). Realization r accumulates into the maps at r * map_stride /
+// r * diff_stride.
 template <typename D>
 __global__ void __launch_bounds__(kDepositThreads, sizeof(D) == 4 ? 16 : 8)
     ipm_deposit_batch(const double2* __restrict__ verts, const DepositPiece<D>* __restrict__ pieces, int npieces,
                       long long nchunks, int npx, int npy, DepositMaps maps, long long map_stride,
                       long long diff_stride) {
-  const long long warp0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   __shared__ TriSlots<D> slots[kDepositWarps];
   TriSlots<D>& stage = slots[threadIdx.x >> 5];
-  constexpr int K = 8;  // consecutive chunks per visit: one piece search per K chunks
-  for (long long g0 = warp0 * K; g0 < nchunks; g0 += nwarps * K) {
+  constexpr int K = 8;
+  const DepositOrder o = deposit_order<D>((nchunks + K - 1) / K);
+  long long g0 = o.first * K;
+  for (int i = 0; i < o.count && g0 < nchunks; i++, g0 += o.stride * K) {
     int lo = 0, hi = npieces - 1;  // last piece with chunk0 <= g0
     while (lo < hi) {
       int mid = (lo + hi + 1) >> 1;

@@ -168,3 +168,34 @@ def test_deposition_of_awkward_cells(gpu, dbl, kind):
     got = d_map.cpu().numpy()
     np.testing.assert_array_equal(got, (q.astype(np.float64) * 2.0 ** -32).astype(got.dtype))
     assert q.any()
+
+
+@pytest.mark.parametrize("dbl", [False, True])
+@pytest.mark.parametrize("ncx,ncy", [(31, 1), (33, 3), (64, 148), (1000, 301), (3000, 1700)])
+def test_deposition_order_covers_every_cell_once(gpu, dbl, ncx, ncy):
+    """Lattices of fewer cells than a warp, of one chunk per warp, and of more
+    chunks than one wave or one grid of warps holds: every cell deposits its
+    area exactly once."""
+    import ctypes
+
+    import torch
+
+    import irs_b200._lib as L
+    T, tdt = (ctypes.c_double, torch.float64) if dbl else (ctypes.c_float, torch.float32)
+    f = L.load("ipm", dbl).ipm_deposit_noalloc
+    f.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_longlong, T, ctypes.c_int, ctypes.c_int,
+                  ctypes.c_void_p, ctypes.c_void_p]
+    f.restype = ctypes.c_int
+    npx = npy = 16
+    # cell (i, j) lies inside pixel (i mod 16, j mod 16): both triangles deposit there whole
+    i, j = torch.arange(ncx + 1, device="cuda"), torch.arange(ncy + 1, device="cuda")
+    x = 0.5 + 14.9 * (i.double() / ncx)
+    y = 0.5 + 14.9 * (j.double() / ncy)
+    v = torch.stack([x[None, :].expand(ncy + 1, -1), y[:, None].expand(-1, ncx + 1)], -1).contiguous()
+    d_map = torch.zeros((npy, npx), dtype=tdt, device="cuda")
+    assert f(v.data_ptr(), ncx, ncy, 0.5, npx, npy, d_map.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    # 2 triangles of factor 0.5 per cell; a triangle loses at most 2^-32 per pixel it touches
+    got = float(d_map.double().sum())
+    tol = ncx * ncy * 2 * 6 * 2.0 ** -32 + ncx * ncy * 2.0 ** -22
+    assert abs(got - ncx * ncy) <= tol
