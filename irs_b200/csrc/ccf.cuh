@@ -146,30 +146,31 @@ __device__ __forceinline__ cplx<double> recip(cplx<double> d) {
   return mk(d.re * inv, -d.im * inv);
 }
 
-// sum over k = lane, lane + 32, ... < n, k != skip, of 1 / (z - p[k]): four
-// independent accumulators (four reciprocals in flight per lane), added in a
-// fixed order.
-__device__ __forceinline__ cplx<double> lane_recip_sum(const double2* p, int n, cplx<double> z,
-                                                       int skip, int lane) {
-  cplx<double> acc[4];
+// sum over k = lane, lane + 32, ... < n, k != skip, of 1 / (z - p[k]): eight
+// independent accumulators (eight reciprocals in flight per lane, the last
+// batch included), added in a fixed order. rcp_f64 instead of a general
+// division: about an ulp per term.
+__device__ __forceinline__ cplx<double> lane_recip_sum(const double2* p, int n, cplx<double> z, int skip, int lane) {
+  constexpr int U = 8;
+  cplx<double> acc[U];
 #pragma unroll
-  for (int u = 0; u < 4; u++) acc[u] = mk(0.0, 0.0);
-  int i = lane;
-  for (; i + 96 < n; i += 128) {
+  for (int u = 0; u < U; u++) acc[u] = mk(0.0, 0.0);
+  for (int i = lane; i < n; i += 32 * U) {
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
+    for (int u = 0; u < U; u++) {
       const int k = i + 32 * u;
-      const double2 w = p[k];
-      const cplx<double> r = recip(mk(z.re - w.x, z.im - w.y));
-      if (k != skip) acc[u] = cadd(acc[u], r);
+      const bool use = k < n && k != skip;
+      const double2 w = p[use ? k : lane];
+      const double dx = z.re - w.x, dy = z.im - w.y;
+      const double inv = rcp_f64(fma(dx, dx, dy * dy));
+      if (use) acc[u] = mk(fma(dx, inv, acc[u].re), fma(-dy, inv, acc[u].im));
     }
   }
-  for (; i < n; i += 32) {
-    const double2 w = p[i];
-    const cplx<double> r = recip(mk(z.re - w.x, z.im - w.y));
-    if (i != skip) acc[0] = cadd(acc[0], r);
-  }
-  return cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3]));
+#pragma unroll
+  for (int o = U / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int u = 0; u < o; u++) acc[u] = cadd(acc[u], acc[u + o]);
+  return acc[0];
 }
 
 __device__ __forceinline__ cplx<double> warp_sum(cplx<double> v) {
@@ -184,10 +185,13 @@ __device__ __forceinline__ cplx<double> warp_sum(cplx<double> v) {
 // ccf_field with the work of one root spread over a warp: lane l takes the
 // near-field stars l, l + 32, ... (one each for a leaf's <= 32) and the
 // partial sums meet in a butterfly reduction (fixed order: deterministic);
-// every lane then evaluates the local expansion (the same dz) itself.
+// every lane then evaluates the local expansion (the same dz) itself. `node` is
+// the root's tree node of its last update (-1: none): it is kept while the root
+// stays in that node's box, which is what the descent would find.
 template <typename T>
 __device__ __forceinline__ CcfField ccf_field_warp(const CcfParams& P, const LeafPtrs& lp, const DescentPtrs<T>& dp,
-                                                   const StarRec<T>* __restrict__ stars, cplx<double> z, int lane) {
+                                                   const StarRec<T>* __restrict__ stars, cplx<double> z, int lane,
+                                                   int& node) {
   CcfField f;
   f.s1 = f.s2 = f.s3 = f.a0 = f.a1 = f.a2 = mk(0.0, 0.0);
   f.hl = 1.0;
@@ -196,24 +200,22 @@ __device__ __forceinline__ CcfField ccf_field_warp(const CcfParams& P, const Lea
   if (outside) {  // the root node: every star, no expansion
     for (int i = lane; i < P.nstars; i += 32) ccf_add_star(f, z, double(stars[i].x), double(stars[i].y), double(stars[i].m));
   } else {
-    leaf = descend_leaf(dp, z.re, z.im);
+    if (node < 0 || !(z.re >= dp.lox[node] && z.re < dp.hix[node] && z.im >= dp.loy[node] && z.im < dp.hiy[node]))
+      node = descend_node(dp, z.re, z.im);
+    leaf = int(dp.leaf_of_node[node]);
     const int nn = lp.nnear[leaf];
-    if (lane < nn) {
-      const double4 st = lp.near64[(size_t)leaf * kMaxStarsDirect + lane];
-      ccf_add_star(f, z, st.x, st.y, st.z);
-    }
+    const double4 st = lp.near64[(size_t)leaf * kMaxStarsDirect + lane];
+    if (lane < nn) ccf_add_star(f, z, st.x, st.y, st.z);
   }
-  f.s1 = warp_sum(f.s1);
   f.s2 = warp_sum(f.s2);
   f.s3 = warp_sum(f.s3);
   if (outside) return f;
   f.hl = lp.hl[leaf];
   const cplx<double> dz = mk((z.re - lp.cx[leaf]) / f.hl, (z.im - lp.cy[leaf]) / f.hl);
   const double2* coef = lp.coef64 + (size_t)leaf * kMaxOrder;
-  for (int k = P.p; k >= 1; k--) {
+  for (int k = P.p; k >= 2; k--) {
     const double2 c = coef[k - 1];  // k c_k
-    f.a0 = cadd(cmul(f.a0, dz), mk(c.x, c.y));
-    if (k >= 2) f.a1 = cadd(cmul(f.a1, dz), mk(c.x * (k - 1), c.y * (k - 1)));
+    f.a1 = cadd(cmul(f.a1, dz), mk(c.x * (k - 1), c.y * (k - 1)));
     if (k >= 3) f.a2 = cadd(cmul(f.a2, dz), mk(c.x * ((k - 1) * (k - 2)), c.y * ((k - 1) * (k - 2))));
   }
   return f;
@@ -234,16 +236,17 @@ __global__ void ccf_phases(CcfParams P, double2* __restrict__ cs) {
 // the chain's roots `src` (root a is z itself), phase cs = (cos, sin) phi. The
 // lanes split the sums over all stars (their positions `spos`, in tree order)
 // and over the chain's other roots (strided, so a warp reads 32 consecutive
-// positions at a time; both arrays stay in L1) and reduce them in a fixed
-// order. Returns whether the root is final; zn (lane 0) is its new position.
+// positions at a time) and reduce them in a fixed order. Returns whether the
+// root is final; zn (lane 0) is its new position.
 template <typename T>
 __device__ __forceinline__ bool ccf_update(const CcfParams& P, const LeafPtrs& lp, const DescentPtrs<T>& dp,
-                                           const StarRec<T>* __restrict__ stars, const double2* __restrict__ spos,
-                                           const double2* src, int a, double2 cs, int lane, double2& out) {
+                                           const StarRec<T>* __restrict__ stars, const double2* spos,
+                                           const double2* src, int a, double2 cs, double theta, int lane, int& node,
+                                           double2& out) {
   const double2 z2 = src[a];
   const cplx<double> z = mk(z2.x, z2.y);
   out = z2;
-  const CcfField f = ccf_field_warp(P, lp, dp, stars, z, lane);
+  const CcfField f = ccf_field_warp(P, lp, dp, stars, z, lane, node);
   const CcfDerivs d = ccf_derivs(P, f, z);
   const cplx<double> f0 = csub(cconj(d.dwdzb), mk(d.dwdz * cs.x, -d.dwdz * cs.y));  // ccf_f0
   if (ccf_inv_mu_bound(cabs_(f0), d.dwdz) < 1e-9) return true;  // already a root to the precision sought
@@ -255,7 +258,7 @@ __device__ __forceinline__ bool ccf_update(const CcfParams& P, const LeafPtrs& l
   const cplx<double> den = cadd(f1, cmul(f0, csub(ps, rs)));
   const cplx<double> zn = csub(z, cdiv(f0, den));
   out = make_double2(zn.re, zn.im);
-  return cabs_(csub(zn, z)) / sqrt(P.theta2) < 1e-9;
+  return cabs_(csub(zn, z)) / theta < 1e-9;
 }
 
 // Reads of a barrier word (about a microsecond each) after which a CTA gives
@@ -275,20 +278,34 @@ __host__ __device__ __forceinline__ long long ccf_spins(const CcfParams& P) {
 // the barrier reports that no root is left to move: a final root is never
 // moved again, so the updates left out change nothing.
 //
-// Bound by latency: a chain of dependent updates, each a tree descent, a Horner
+// The barrier's acquire empties L1, so what every update reads again is kept
+// elsewhere: up to kCcfShared star positions in shared memory, and per root the
+// tree node of its last update.
+//
+// Bound by latency: a chain of dependent updates (about 4 a step), each a Horner
 // evaluation and two sums, with 2 chains x 274 roots for the default field;
 // from 1000 stars on by the FP64 reciprocals (2 N^2 per update and chain).
 // As ~1000 graph-captured launches, most of which found every root final, the
 // root finding of 137 / 1000 stars took 4.6 / 13.0 ms (B200) besides 3 - 5 ms
-// to capture and instantiate the graphs; now 2.5 / 12.4 ms.
+// to capture and instantiate the graphs; as this launch 2.5 / 12.4 ms with every
+// descent, general divisions and four reciprocals in flight, now 2.1 / 7.0 ms.
+constexpr int kCcfShared = 4096;  // star positions held in shared memory (64 KB)
 template <typename T>
 __global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs lp, DescentPtrs<T> dp,
                                                           const StarRec<T>* __restrict__ stars,
                                                           const double2* __restrict__ spos,
                                                           const double2* __restrict__ cs, int it0, int it1,
                                                           double2* roots, double2* s0, double2* s1,
-                                                          unsigned char* fin, unsigned long long* words, int* err,
-                                                          int centres, double2** last) {
+                                                          unsigned char* fin, int* nodes, unsigned long long* words,
+                                                          int* err, int centres, double2** last) {
+  extern __shared__ double2 s_pos[];
+  const bool shared = P.nstars <= kCcfShared;
+  if (shared) {
+    for (int i = threadIdx.x; i < P.nstars; i += kCcfThreads) s_pos[i] = spos[i];
+    __syncthreads();
+  }
+  const double2* pos = shared ? s_pos : spos;
+  const double theta = sqrt(P.theta2);
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (kCcfThreads / 32);
   const int warp = blockIdx.x * (kCcfThreads / 32) + (threadIdx.x >> 5);
@@ -314,8 +331,12 @@ __global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs 
           roots[(size_t)ccf_row(P, c, sj) * P.nroots + a] = z;
         }
         bool done = true;
-        if (state == 0)
-          done = ccf_update<T>(P, lp, dp, stars, spos, src, a, cs[(j == 0 ? 2 * c : ch) * (half + 1) + j], lane, z);
+        if (state == 0) {
+          int node = i == 0 && j <= 1 ? -1 : nodes[q];
+          done = ccf_update<T>(P, lp, dp, stars, pos, src, a, cs[(j == 0 ? 2 * c : ch) * (half + 1) + j], theta, lane,
+                               node, z);
+          if (lane == 0) nodes[q] = node;
+        }
         done = __shfl_sync(0xffffffffu, int(done), 0) != 0;
         if (lane == 0) {
           nxt[(size_t)ch * P.nroots + a] = z;

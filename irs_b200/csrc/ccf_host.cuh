@@ -233,7 +233,7 @@ class CCF {
     const int half = num_phi / (2 * num_branches);
     const size_t nwords = size_t(it0) + size_t(half) * it1;  // a grid barrier per update
     if (!d_roots_.alloc_exact((size_t)rows * num_roots) || !d_scratch_.alloc_exact(2 * (size_t)nch * num_roots) ||
-        !d_fin_.alloc_exact((size_t)nch * num_roots) || !d_stat_.alloc_exact(2) || !d_words_.alloc_exact(nwords + 2) ||
+        !d_fin_.alloc_exact((size_t)nch * num_roots) || !d_nodes_.alloc_exact((size_t)nch * num_roots) || !d_stat_.alloc_exact(2) || !d_words_.alloc_exact(nwords + 2) ||
         !d_phase_.alloc_exact((size_t)nch * (half + 1)))
       return false;
     double2 *b0 = d_scratch_.p, *b1 = d_scratch_.p + (size_t)nch * num_roots;
@@ -243,14 +243,18 @@ class CCF {
     IRSB_CKR(cudaMemcpyAsync(b0, init.data(), init.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
     IRSB_CKR(cudaMemsetAsync(words, 0, (nwords + 2) * sizeof(unsigned long long), s));
     const LeafPtrs lp = leaf_ptrs();
-    const DescentPtrs<T> dp{tree_.cx.p, tree_.cy.p, tree_.child0.p, leaves_.pos.p, nullptr};
+    const DescentPtrs<T> dp{tree_.cx.p, tree_.cy.p, tree_.child0.p, leaves_.pos.p, nullptr,
+                            tree_.lox.p, tree_.hix.p, tree_.loy.p, tree_.hiy.p};
     ccf_phases<<<std::max(1, std::min(ceil_div((long long)nch * (half + 1), 64), 148)), 64, 0, s>>>(Q, d_phase_.p);
     IRSB_LAUNCH_CK("ccf_phases");
     // a warp per root, as many CTAs as can be resident together (the grid
     // waits for one another at every update)
+    const size_t smem = n <= kCcfShared ? n * sizeof(double2) : 0;
+    IRSB_CKR(cudaFuncSetAttribute(ccf_follow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCcfShared * sizeof(double2))));
     auto follow = [&](int centres, int chains, unsigned long long* w) -> bool {
       int grid = 0;
-      if (!cooperative_grid(ccf_follow<T>, kCcfThreads, ceil_div((long long)chains * num_roots, kCcfThreads / 32), &grid))
+      if (!cooperative_grid(ccf_follow<T>, kCcfThreads, ceil_div((long long)chains * num_roots, kCcfThreads / 32), &grid,
+                            smem))
         return false;
       CcfParams q = Q;
       LeafPtrs l = lp;
@@ -260,8 +264,9 @@ class CCF {
       int i0 = it0, i1 = it1;
       double2 *ro = d_roots_.p, *s0 = b0, *s1 = b1;
       unsigned char* fi = d_fin_.p;
-      void* args[] = {&q, &l, &d, &st, &sp, &ph, &i0, &i1, &ro, &s0, &s1, &fi, &w, &err, &centres, &last};
-      return IRSB_CK(cudaLaunchCooperativeKernel((const void*)ccf_follow<T>, dim3(grid), dim3(kCcfThreads), args, 0, s));
+      int* no = d_nodes_.p;
+      void* args[] = {&q, &l, &d, &st, &sp, &ph, &i0, &i1, &ro, &s0, &s1, &fi, &no, &w, &err, &centres, &last};
+      return IRSB_CK(cudaLaunchCooperativeKernel((const void*)ccf_follow<T>, dim3(grid), dim3(kCcfThreads), args, smem, s));
     };
     // branch centres (include/ccf.cuh:906-977), then the steps away from them (:979-1037)
     IRSB_CKR(cudaEventRecord(e0_, s));
@@ -411,6 +416,7 @@ class CCF {
   DevVec<double2> d_roots_, d_scratch_, d_ccs_, d_caus_, d_spos_, d_phase_;
   DevVec<double> d_mu_;
   DevVec<unsigned char> d_fin_;
+  DevVec<int> d_nodes_;
   DevVec<unsigned long long> d_stat_, d_words_;
 
   // Corner of a circular field of num_stars stars (include/ccf.cuh:427-432).

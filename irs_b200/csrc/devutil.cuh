@@ -122,11 +122,11 @@ __device__ __forceinline__ int grid_barrier_sum(unsigned long long* word, int va
 
 // CTAs of a cooperative grid: `want`, at most what is resident at once.
 template <typename K>
-bool cooperative_grid(K kernel, int threads, long long want, int* grid) {
+bool cooperative_grid(K kernel, int threads, long long want, int* grid, size_t smem = 0) {
   int dev = 0, sms = 0, per_sm = 0;
   IRSB_CKR(cudaGetDevice(&dev));
   IRSB_CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  IRSB_CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+  IRSB_CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   const long long most = (long long)sms * per_sm;
   *grid = int(want < 1 ? 1 : (want > most ? most : want));
   return true;

@@ -75,6 +75,31 @@ def test_critical_curves_of_few_stars_match_oracle(gpu, tmp_path, n, nphi, nb):
     c.close()
 
 
+@pytest.mark.parametrize("n", [31, 256, 257, 4096, 4097])
+def test_critical_curves_on_both_sides_of_the_shared_positions(gpu, tmp_path, n):
+    """Star positions are held in shared memory up to 4096 stars, read in steps
+    of 8 x 32: every root of every phi solves the directly summed equation
+    dw/dzbar* = dw/dz e^{-i phi} (1/mu there is the stop's bound 1e-9 plus the
+    expansion's error, together below 1e-8), and no two roots are the same."""
+    from oracle import ccf_ref
+    from tests.test_gpu_ccf import as_complex, star_field, write_stars
+    stars, rad = star_field(n, kstar=0.3, seed=7 + n)
+    write_stars(str(tmp_path / "s.bin"), stars, rad)
+    c = irs_b200.CCF(kappa_tot=0.45, shear=0.25, starfile=str(tmp_path / "s.bin"), num_phi=4, num_branches=1)
+    c.run()
+    got = as_complex(c.critical_curves)  # (roots, phi)
+    L = ccf_ref.Lens(stars, 0.45, 0.25, c.kappa_star, 1.0, 1, rad)
+    assert got.shape[0] == 2 * n
+    cell = 1e-7 * c.value("expansion_order") / (1.1 * rad / 2.0 ** c.value("tree_levels"))
+    for z in got.T:
+        for part in np.array_split(z, max(1, 2 * n // 512)):
+            _, dwdz, dwdzb, d2 = L.fields(part)
+            inv_mu = np.abs(dwdz) ** 2 - np.abs(dwdzb) ** 2
+            assert np.all(np.abs(inv_mu) < 2e-9 * (1 + np.abs(dwdzb) * np.abs(d2)) + 2 * cell * np.abs(dwdzb))
+        assert np.unique(z).size == z.size
+    c.close()
+
+
 @pytest.mark.parametrize("index", [11, 17])
 def test_batch_mass_sums_of_large_fields(gpu, index):
     """Kroupa fields of 3.8e5 and 7.6e5 float masses: the sums of m are exact in
