@@ -20,8 +20,10 @@ IRSB_HD T boxcar_(cplx<T> z, cplx<T> c) {
   return (-c.re <= z.re && z.re <= c.re && -c.im <= z.im && z.im <= c.im) ? T(1) : T(0);
 }
 
+// inv_i: 1 / i for i = 1 .. ts where the caller holds a table (nullptr: divided here)
 template <typename T>
-IRSB_HD cplx<T> alpha_smooth_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi) {
+IRSB_HD cplx<T> alpha_smooth_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi,
+                              const T* inv_i = nullptr) {
   cplx<T> a;
   if (rect) {
     cplx<T> zb = cconj(z);
@@ -29,7 +31,7 @@ IRSB_HD cplx<T> alpha_smooth_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, 
       cplx<T> s1 = mk<T>(0, 0), s2 = s1, s3 = s1, s4 = s1;
       cplx<T> r1 = cdiv(zb, c), r2 = cdiv(zb, cconj(c)), r3 = cdiv(zb, cneg(c)), r4 = cdiv(zb, cneg(cconj(c)));
       for (int i = ts; i >= 1; i--) {
-        T inv = T(1) / T(i);
+        T inv = inv_i ? inv_i[i] : T(1) / T(i);
         s1.re += inv;
         s2.re += inv;
         s3.re += inv;
