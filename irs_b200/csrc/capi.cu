@@ -139,6 +139,7 @@ bool derive(Obj* self) {
   if (!irsb::check_input_params(p)) return false;
   std::vector<irsb::StarRec<dtype>> st;
   if (!irsb::derive_params<dtype>(p, st)) return false;
+  if (!st.empty()) p.mean_mass2_ln_mass = irsb::star_field_log_moment<dtype>(int(st.size()), st.data());
   self->prm = p;
   return true;
 }

@@ -131,7 +131,8 @@ class CCF {
         return false;
       }
       star_field_moments<T>(num_stars, rectangular, corner, theta_star, field.data(), kappa_star, m_lower_run,
-                            m_upper_run, mean_mass, mean_mass2, mean_mass2_ln_mass);
+                            m_upper_run, mean_mass, mean_mass2);
+      mean_mass2_ln_mass = star_field_log_moment<T>(num_stars, field.data());
       if (kappa_star > kappa_tot) std::cerr << "Warning. kappa_star > kappa_tot\n";
     }
     mu_ave = T(1) / ((1 - kappa_tot) * (1 - kappa_tot) - shear * shear);
@@ -176,7 +177,8 @@ class CCF {
       IRSB_CKR(cudaMemcpyAsync(d_stars_.p, field.data(), size_t(n) * sizeof(StarRec<T>), cudaMemcpyHostToDevice, s));
     }
     star_field_moments<T>(n, rectangular, corner, theta_star, field.data(), kappa_star_actual, m_lower_actual,
-                          m_upper_actual, mean_mass_actual, mean_mass2_actual, mean_mass2_ln_mass_actual);
+                          m_upper_actual, mean_mass_actual, mean_mass2_actual);
+    mean_mass2_ln_mass_actual = star_field_log_moment<T>(n, field.data());
     if (starfile.empty())  // the corner from the realised mean mass (include/ccf.cuh:684-697)
       corner = rectangular ? scaled_rect(corner, mean_mass_actual) : scaled_circle(corner, mean_mass_actual);
     // ---- initial roots at each branch centre: star +/- 1, the rest on the

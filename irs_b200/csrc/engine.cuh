@@ -236,15 +236,19 @@ class MapMaker {
       IRSB_CKR(cudaStreamSynchronize(stream_));
     }
     star_field_moments<T>(n, p.rectangular, p.corner, p.theta_star, stars_out.data(), p.kappa_star_actual,
-                          p.m_lower_actual, p.m_upper_actual, p.mean_mass_actual, p.mean_mass2_actual,
-                          p.mean_mass2_ln_mass_actual);
+                          p.m_lower_actual, p.m_upper_actual, p.mean_mass_actual, p.mean_mass2_actual);
     if (!from_stars) recompute_corner(p);
     p.root_half_length = root_half_length_of(p);
     if (use_host_stars) p.starfile = "";
     prm = p;
 
     launches = from_stars ? 0 : 1;  // star generation
-    if (!device_pipeline()) return false;
+    // the logarithmic moment, for the parameter file, while the tree is built
+    const auto log_moment = [&] {
+      prm.mean_mass2_ln_mass_actual = star_field_log_moment<T>(n, stars_out.data());
+      if (from_stars) prm.mean_mass2_ln_mass = prm.mean_mass2_ln_mass_actual;
+    };
+    if (!device_pipeline(log_moment)) return false;
     // stars in tree order, as the reference leaves them
     IRSB_CKR(cudaMemcpyAsync(stars_out.data(), d_stars_.p, size_t(n) * sizeof(StarRec<T>), cudaMemcpyDeviceToHost,
                              stream_));
@@ -263,17 +267,24 @@ class MapMaker {
   // timed with CUDA events (t_pipeline, t_shoot, t_lattice, t_deposit).
   // One host synchronisation before the end: the tree's depth (the expansion
   // order follows from it) and the number of lattice tiles are read together,
-  // after the build and the leaves' rectangles.
-  bool device_pipeline() {
+  // after the build and the leaves' rectangles; host_work() runs on the host
+  // meanwhile.
+  template <typename F>
+  bool device_pipeline(F host_work) {
     const int n = prm.num_stars;
     IRSB_CKR(cudaEventRecord(ev0_, stream_));
     const ShootParams lat = shoot_params(!IS_IRS);
     const auto band = band_rows();
     // rays: rows [lo, hi); cells: rows [lo, hi) need corner rows [lo, hi]
     const long long jlo = band.first, jhi = IS_IRS ? band.second : band.second + 1;
+    bool worked = false;
     auto rects = [&](long long cap) {
-      return lattice_rects<T>(tiles_, leaves_, tree_, cap, lat.base_x, lat.base_y, lat.rhs_x, lat.rhs_y, lat.nx,
-                              lat.ny, jlo, jhi, stream_);
+      if (!lattice_rects<T>(tiles_, leaves_, tree_, cap, lat.base_x, lat.base_y, lat.rhs_x, lat.rhs_y, lat.nx, lat.ny,
+                            jlo, jhi, stream_))
+        return false;
+      if (!worked) host_work();  // once, also when the build is repeated
+      worked = true;
+      return true;
     };
     if (!build_tree<T>(tree_, d_stars_.p, n, prm.root_half_length, leaves_.pos, leaves_.node, stream_, rects))
       return false;
@@ -330,7 +341,7 @@ class MapMaker {
     double tot = 0;
     launches = 0;
     for (int r = 0; r < repeats; r++) {
-      if (!device_pipeline()) return false;
+      if (!device_pipeline([] {})) return false;
       tot += t_pipeline;
     }
     if (seconds) *seconds = tot;
@@ -540,7 +551,9 @@ class MapMaker {
   DevVec<T> d_map_, d_map_min_, d_map_sad_;
   DevVec<double2> d_verts_;
   DevVec<unsigned long long> d_red_;
+  static constexpr int kMaxRanges = 3;
   DevVec<long long> d_mm_;
+  HostVec<long long> h_mm_;
 
   bool init_stream() {
     if (stream_) return true;
@@ -718,28 +731,30 @@ class MapMaker {
     return true;
   }
 
+  // Smallest and largest value of each of the nmaps maps of n values, with one
+  // synchronisation.
   template <typename V>
-  bool minmax(const V* v, long long n, long long& lo, long long& hi) {
+  bool value_ranges(const V* const* maps, int nmaps, long long n, V* lo, V* hi) {
     using K = typename OrderedKey<V>::K;
-    if (!d_mm_.alloc_exact(2)) return false;
-    K init[2];
-    if constexpr (sizeof(K) == 4) {
-      init[0] = 0x7fffffff;
-      init[1] = int(0x80000000);
-    } else {
-      init[0] = 0x7fffffffffffffffLL;
-      init[1] = (long long)0x8000000000000000ULL;
+    static_assert(sizeof(K) <= sizeof(long long), "keys fit the buffers");
+    if (!d_mm_.alloc_exact(2 * kMaxRanges) || !h_mm_.alloc(2 * kMaxRanges)) return false;
+    K *dm = reinterpret_cast<K*>(d_mm_.p), *hm = reinterpret_cast<K*>(h_mm_.p);
+    for (int i = 0; i < nmaps; i++) {
+      hm[2 * i] = std::numeric_limits<K>::max();
+      hm[2 * i + 1] = std::numeric_limits<K>::min();
     }
-    K* dm = reinterpret_cast<K*>(d_mm_.p);
-    IRSB_CKR(cudaMemcpyAsync(dm, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
+    IRSB_CKR(cudaMemcpyAsync(dm, hm, 2 * nmaps * sizeof(K), cudaMemcpyHostToDevice, stream_));
     int g = int(std::max<long long>(1, std::min<long long>((n + 255) / 256, 148LL * 8)));
-    minmax_nonneg<V><<<g, 256, 0, stream_>>>(v, n, dm);
-    IRSB_LAUNCH_CK("minmax_nonneg");
-    K out[2];
-    IRSB_CKR(cudaMemcpyAsync(out, dm, sizeof(out), cudaMemcpyDeviceToHost, stream_));
+    for (int i = 0; i < nmaps; i++) {
+      minmax_nonneg<V><<<g, 256, 0, stream_>>>(maps[i], n, dm + 2 * i);
+      IRSB_LAUNCH_CK("minmax_nonneg");
+    }
+    IRSB_CKR(cudaMemcpyAsync(hm, dm, 2 * nmaps * sizeof(K), cudaMemcpyDeviceToHost, stream_));
     IRSB_CKR(cudaStreamSynchronize(stream_));
-    lo = (long long)out[0];
-    hi = (long long)out[1];
+    for (int i = 0; i < nmaps; i++) {
+      lo[i] = decode<V>((long long)hm[2 * i]);
+      hi[i] = decode<V>((long long)hm[2 * i + 1]);
+    }
     return true;
   }
   template <typename V>
@@ -755,15 +770,6 @@ class MapMaker {
       std::memcpy(&d, &k, 8);
       return d;
     }
-  }
-
-  template <typename V>
-  bool value_range(const V* v, long long n, V& lo, V& hi) {
-    long long a, b;
-    if (!minmax<V>(v, n, a, b)) return false;
-    lo = decode<V>(a);
-    hi = decode<V>(b);
-    return true;
   }
 
   // Histogram of a device map, counted on the device and kept there: `out`
@@ -819,8 +825,10 @@ class MapMaker {
     }
     if (p.write_histograms) {
       const int factor = IS_IRS ? 1 : 1000;
-      Pix lo, hi;
-      if (!value_range<Pix>(dmap, npix, lo, hi)) return false;
+      const Pix* maps[kMaxRanges] = {dmap, dmin, dsad};  // total, minima, saddles
+      Pix los[kMaxRanges], his[kMaxRanges];
+      if (!value_ranges<Pix>(maps, par ? 3 : 1, npix, los, his)) return false;
+      const Pix lo = los[0], hi = his[0];
       long long mn = llround(double(lo) * factor), mx = llround(double(hi) * factor);
       if (IS_IRS) {
         mn = (long long)lo;
@@ -834,8 +842,7 @@ class MapMaker {
       if (p.mu_ave > 1 && mu_min_actual < mu_min_theory)
         std::cerr << "Warning. Minimum magnification after shooting is less than the theoretical minimum.\n";
       if (par) {
-        Pix a, b, c, d;
-        if (!value_range<Pix>(dmin, npix, a, b) || !value_range<Pix>(dsad, npix, c, d)) return false;
+        const Pix a = los[1], b = his[1], c = los[2], d = his[2];
         long long mna, mxa, mnc, mxc;
         if (IS_IRS) {
           mna = a; mxa = b; mnc = c; mxc = d;
@@ -874,8 +881,7 @@ class MapMaker {
         long long lmn = (lo > 0) ? lg(lo) : lg(std::max<Pix>(hi * Pix(1e-6), Pix(1e-30)));
         long long lmx = (hi > 0) ? lg(hi) : 0;
         if (par) {
-          Pix a, b, c, d;
-          if (!value_range<Pix>(dmin, npix, a, b) || !value_range<Pix>(dsad, npix, c, d)) return false;
+          const Pix a = los[1], b = his[1], c = los[2], d = his[2];
           if (a > 0) lmn = std::min(lmn, lg(a));
           if (c > 0) lmn = std::min(lmn, lg(c));
           if (b > 0) lmx = std::max(lmx, lg(b));

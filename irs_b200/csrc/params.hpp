@@ -124,29 +124,37 @@ bool check_input_params(const Params<T>& p) {
 }
 
 // Moments and kappa_star of a concrete star field (include/star.cuh:124-161):
-// sums in double, in star order.
+// sums in double, in star order. The logarithmic moment, which only the
+// parameter file reads, is a sum of its own (star_field_log_moment), so that a
+// caller can form it while the device works.
 template <typename T>
 void star_field_moments(int n, int rectangular, cplx<T> corner, T theta, const StarRec<T>* s,
-                        T& kappastar, T& m_lower, T& m_upper, T& mean_mass, T& mean_mass2,
-                        T& mean_mass2_ln_mass) {
+                        T& kappastar, T& m_lower, T& m_upper, T& mean_mass, T& mean_mass2) {
   m_lower = std::numeric_limits<T>::max();
   m_upper = std::numeric_limits<T>::min();
-  double m_tot = 0, m2_tot = 0, m2_ln_tot = 0;
+  double m_tot = 0, m2_tot = 0;
   for (int i = 0; i < n; i++) {
     T m = s[i].m;
     m_tot += m;
     m2_tot += m * m;
-    m2_ln_tot += m * m * std::log(m);
     m_lower = std::min(m_lower, m);
     m_upper = std::max(m_upper, m);
   }
   mean_mass = T(m_tot / n);
   mean_mass2 = T(m2_tot / n);
-  mean_mass2_ln_mass = T(m2_ln_tot / n);
   if (rectangular)
     kappastar = T(m_tot * kPi<T> * theta * theta / (4 * corner.re * corner.im));
   else
     kappastar = T(m_tot * theta * theta / (cabs_(corner) * cabs_(corner)));
+}
+template <typename T>
+T star_field_log_moment(int n, const StarRec<T>* s) {
+  double m2_ln_tot = 0;
+  for (int i = 0; i < n; i++) {
+    T m = s[i].m;
+    m2_ln_tot += m * m * std::log(m);
+  }
+  return T(m2_ln_tot / n);
 }
 
 // ---------------------------------------------------------------- star files
@@ -281,7 +289,8 @@ bool write_star_file_bin(const std::string& path, int n, int rect, cplx<T> corne
 // star field when a star file is given.
 // With `preloaded`, stars_io already holds the field and num_stars,
 // rectangular, corner and theta_star are set (a star field passed in memory);
-// it then follows the star-file branch without reading a file.
+// it then follows the star-file branch without reading a file. A field's
+// logarithmic moment is left to the caller (star_field_log_moment).
 template <typename T>
 bool derive_params(Params<T>& p, std::vector<StarRec<T>>& stars_io, bool preloaded = false) {
   const bool from_stars = preloaded || !p.starfile.empty();
@@ -315,7 +324,7 @@ bool derive_params(Params<T>& p, std::vector<StarRec<T>>& stars_io, bool preload
       return false;
     }
     star_field_moments<T>(p.num_stars, p.rectangular, p.corner, p.theta_star, stars_io.data(), p.kappa_star,
-                          p.m_lower, p.m_upper, p.mean_mass, p.mean_mass2, p.mean_mass2_ln_mass);
+                          p.m_lower, p.m_upper, p.mean_mass, p.mean_mass2);
     if (p.kappa_star > p.kappa_tot) std::cerr << "Warning. kappa_star > kappa_tot\n";
   }
 
