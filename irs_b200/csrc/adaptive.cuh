@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refin
           const unsigned now = x >= box.x && x < box.y ? todo & rows : 0u;
           todo &= ~now;
           float sx[R], sy[R], cxr[R], cyr[R], Ar[R], Ai[R];
-          near_far_pairs<R>(ux, uy, L.inv_hl, (L.nn + 3) & ~3, sp.p, pairs, sx, sy, cxr, cyr, Ar, Ai);
+          near_far_pairs<R>(ux, uy, L.inv_hl, L.nn, sp.p, pairs, sx, sy, cxr, cyr, Ar, Ai);
 #pragma unroll
           for (int r = 0; r < R; r++) {
             const int b = r0 + r;

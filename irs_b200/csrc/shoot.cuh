@@ -196,7 +196,10 @@ __device__ __forceinline__ void red_add_s32(int* p, int v) {
 __device__ __forceinline__ void irs_deposit(double px, double py, int npx, int npy, int* __restrict__ pix,
                                             int* __restrict__ pmin, int* __restrict__ psad, bool parity_min,
                                             bool parities) {
-  int ix = int(px), iy = int(py);
+  // the integer parts of values in [0, 2^31): the low word of v + 1.5 * 2^52,
+  // rounded down (the conversion pipe, which also makes the reciprocals, is
+  // four times slower)
+  int ix = __double2loint(__dadd_rd(px, 6755399441055744.0)), iy = __double2loint(__dadd_rd(py, 6755399441055744.0));
   if (ix == npx) ix--;
   if (iy == npy) iy--;
   long long idx = (long long)(npy - 1 - iy) * npx + ix;
@@ -363,9 +366,11 @@ __global__ void __launch_bounds__(kShootThreads, PAR || GEN ? 2 : 3) shoot_f64(S
 // column offset ux (rows uy[0..R-1], R even), on pairs of points: the same
 // operations in the same order as the scalar form of shoot_f32_tile, so the
 // results are the same bits. fmaf(-Ai, dzi, c) is written fma(Ai, -dzi, c),
-// the same product.
+// the same product. The reciprocals bound it (one per star and point on a pipe
+// of a quarter of the FMA rate), so exactly nn stars are visited: padding to a
+// multiple of 4 with stars of zero mass cost 7 % of them at 19 stars.
 template <int R>
-__device__ __forceinline__ void near_far_pairs(float ux, const float* uy, float inv_hl, int nn4, int p,
+__device__ __forceinline__ void near_far_pairs(float ux, const float* uy, float inv_hl, int nn, int p,
                                                const NearPairs& sp2, float* sx, float* sy, float* cxr, float* cyr,
                                                float* Ar, float* Ai) {
   constexpr int P = R / 2;
@@ -391,19 +396,19 @@ __device__ __forceinline__ void near_far_pairs(float ux, const float* uy, float 
       by[q] = fma2(w, ey, by[q]);
     }
   };
-  for (int s0 = 0; s0 < nn4; s0 += 16) {
+  for (int s0 = 0; s0 < nn; s0 += 16) {
     f32x2 bx[P], by[P];
 #pragma unroll
     for (int q = 0; q < P; q++) bx[q] = by[q] = zero;
+    const int s1 = min(nn, s0 + 16);
+    int s = s0;
+#pragma unroll 1
+    for (; s + 4 <= s1; s += 4) {
 #pragma unroll
-    for (int s = 0; s < 4; s++) star(s0 + s, bx, by);
-#pragma unroll
-    for (int g = 1; g < 4; g++) {
-      if (s0 + 4 * (g + 1) <= nn4) {
-#pragma unroll
-        for (int s = 0; s < 4; s++) star(s0 + 4 * g + s, bx, by);
-      }
+      for (int k = 0; k < 4; k++) star(s + k, bx, by);
     }
+#pragma unroll 1
+    for (; s < s1; s++) star(s, bx, by);
 #pragma unroll
     for (int q = 0; q < P; q++) {  // two-sum of the block into the running sum
       f32x2 t = add2(Sx[q], bx[q]);
@@ -490,6 +495,23 @@ __device__ __forceinline__ void shoot_f32_tile(const ShootParams& sp, const Leaf
     }
     __syncthreads();
     const int nn4 = (nn + 3) & ~3;
+    // A ray that lands clearly off the map is dropped on the FP32 value f of its
+    // position: f, formed from pcx and scx rounded to float by one FMA, is within
+    // 2^-23 (|pcx| + |wr scx|) <= 2^-22 (|pcx| + |f|) (1 + 2^-20) of the FP64 one,
+    // so f below -2^-20 |pcx| or above (npx + 2^-20 |pcx|)(1 + 2^-19) is off the
+    // map (NaN passes on; 2^-100 covers what rounds to subnormals, and a scale
+    // outside [2^-60, 2^100] sets no limit). Two in three rays of a lattice miss
+    // the map and need neither conversion nor FP64: 2.5e8 rays 2.20 ms, now
+    // 2.11 ms (B200).
+    constexpr bool pre = !VERT && !GENERIC_SMOOTH;
+    const float fpcx = float(pcx), fpcy = float(pcy), fscx = float(scx), fscy = float(scy);
+    auto limits = [](float pc, float sc, int np) {
+      const float eps = 9.5367431640625e-7f, tiny = 7.8886091e-31f, inf = __int_as_float(0x7f800000);
+      const bool set = fabsf(sc) >= 8.6736174e-19f && fabsf(sc) <= 1.2676506e30f;
+      return set ? make_float2(fmaf(-eps, fabsf(pc), -tiny), fmaf(eps, fabsf(pc), float(np)) * (1.f + 2.f * eps))
+                 : make_float2(-inf, inf);
+    };
+    const float2 xlim = limits(fpcx, fscx, sp.npx), ylim = limits(fpcy, fscy, sp.npy);
     if (tx < ti.ni) {
       const long long i = ti.i0 + tx;
       const double xg = sp.base_x + 2.0 * (sp.rhs_x * double(i));
@@ -504,7 +526,7 @@ __device__ __forceinline__ void shoot_f32_tile(const ShootParams& sp, const Leaf
       float Ar[R], Ai[R], Dr[R], Di[R];
       if constexpr (!PAR && R % 2 == 0) {
         // the same operations on pairs of points (rows r, r + 1)
-        near_far_pairs<R>(ux, uy, inv_hl, nn4, sp.p, *s_pair, sx, sy, cxr, cyr, Ar, Ai);
+        near_far_pairs<R>(ux, uy, inv_hl, nn, sp.p, *s_pair, sx, sy, cxr, cyr, Ar, Ai);
       } else {
         // ---- near field, blocked compensated summation
 #pragma unroll
@@ -590,6 +612,10 @@ __device__ __forceinline__ void shoot_f32_tile(const ShootParams& sp, const Leaf
         // w - w(centre) = lin * u - alpha_star - conj(A)
         const float wr = fmaf(flin_x, ux, -(Sx + Ar[r]));
         const float wi = fmaf(flin_y, uy[r], -(Sy - Ai[r]));
+        if constexpr (pre) {
+          const float fx = fmaf(wr, fscx, fpcx), fy = fmaf(wi, fscy, fpcy);
+          if (fx < xlim.x || fx > xlim.y || fy < ylim.x || fy > ylim.y) continue;
+        }
         double px = pcx + double(wr) * scx;
         double py = pcy + double(wi) * scy;
         if (GENERIC_SMOOTH) {

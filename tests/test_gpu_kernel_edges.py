@@ -48,6 +48,28 @@ def test_ray_bands_with_parities_add_up(gpu, dbl):
     m.close()
 
 
+@pytest.mark.parametrize("centre", [(0.0, 0.0), (0.35, -0.2), (-6.0, 4.0)])
+@pytest.mark.parametrize("npix,half", [((1, 1), (0.5, 0.5)), ((1, 64), (0.02, 1.28)), ((57, 3), (1.14, 0.06))])
+def test_rays_at_the_edges_of_small_maps(gpu, centre, npix, half):
+    """Most rays miss these maps. With the approximate sheet they are dropped on
+    the FP32 value of their position, with the exact sheet every ray is decided
+    in FP64. Inside the field's circle, where all rays of the lattice are, the
+    two sheets are the same -kappa_star z, so the counts agree ray for ray."""
+    cfg = dict(IRS_SMALL, num_pixels_y1=npix[0], num_pixels_y2=npix[1], half_length_y1=half[0], half_length_y2=half[1],
+               center_y1=centre[0], center_y2=centre[1], num_rays_y=400)
+    maps = []
+    for approx in (True, False):
+        m = irs_b200.IRS(**cfg, approx=approx, expansion_order=10)
+        m.run()
+        assert (abs(m.value("center_x1")) + m.value("half_length_x1")) ** 2 + (
+            abs(m.value("center_x2")) + m.value("half_length_x2")) ** 2 < (
+            m.value("corner_x1") ** 2 + m.value("corner_x2") ** 2)
+        maps.append(m.magnifications.copy())
+        m.close()
+    assert maps[0].sum() > 0
+    np.testing.assert_array_equal(maps[0], maps[1])
+
+
 @pytest.mark.parametrize("n,nphi,nb", [(1, 40, 2), (2, 12, 3), (3, 8, 4), (33, 8, 2)])
 def test_critical_curves_of_few_stars_match_oracle(gpu, tmp_path, n, nphi, nb):
     """Fields of fewer roots than a CTA has warps, one phi step per side, several
