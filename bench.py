@@ -853,7 +853,7 @@ def our_arm(args):
         roof = {"kernel": "ipm_deposit_cells", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "traffic_unit": "GB per launch",
                 "traffic_source": "ncu on the 500^2 case (17.8 B per cell), scaled by cells",
-                "limiter": "instruction issue and latency (ncu, 500^2 case: 65 % issue-active, ALU pipe 51 %)",
+                "limiter": "instruction issue (ncu, a band of a rectangular lattice: 73 % issue-active, ALU pipe 55 %)",
                 "algorithmic": f"16 B x {nverts} corner positions + 8 B x {npix} map words"}
     # the lens-equation kernel against the FP32 FMA roofline, whichever kernel dominates
     lens_tflops = flop_per_vertex * nverts / (lat_ms * 1e-3) / 1e12
