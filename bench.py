@@ -389,7 +389,7 @@ def reference_arm(args):
             jj = np.arange(j0, j0 + rows + 1)
             ii = np.arange(nx + 1)
             X, Y = np.meshgrid(ox + 2.0 * (rx * ii), oy + 2.0 * (ry * jj))
-            wx, wy = t.shoot(L, X, Y)
+            wx, wy = (v.reshape(X.shape) for v in t.shoot(L, X, Y))
             px = (wx + hly[0]) * npx / (2 * hly[0])
             py = npy - (wy + hly[1]) * npy / (2 * hly[1])
             factor = 2 * rx * ry * npx * npy / (4 * hly[0] * hly[1])
