@@ -322,7 +322,10 @@ __global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refin
             uy[r] = float(y - L.cy);
             if (y >= box.z && y < box.w) rows |= 1u << r;
           }
-          const unsigned now = x >= box.x && x < box.y ? todo & rows : 0u;
+          // the first point is among them, since the descent led to this box; it is
+          // taken all the same where no box holds it (a NaN coordinate, from a NaN
+          // centre of the map), so that every round leaves fewer points
+          const unsigned now = (x >= box.x && x < box.y ? todo & rows : 0u) | (lane == src ? todo & (0u - todo) : 0u);
           todo &= ~now;
           float sx[R], sy[R], cxr[R], cyr[R], Ar[R], Ai[R];
           near_far_pairs<R>(ux, uy, L.inv_hl, L.nn, sp.p, pairs, sx, sy, cxr, cyr, Ar, Ai);

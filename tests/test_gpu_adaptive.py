@@ -179,3 +179,19 @@ def test_audit_escalates_above_the_bound(gpu):
         assert b.value("escalation") > 0
         assert b.value("fail_rate") <= b.value("fail_rate_initial")
         assert np.all(b.levels() >= a.levels(predicted=True))
+
+
+@pytest.mark.parametrize("axis", [1, 2])
+def test_refinement_of_a_lattice_without_coordinates_ends(gpu, axis):
+    """A NaN map centre, which a given rectangular field lets pass: no leaf's box
+    holds a refined point, so none has a position and nothing is deposited
+    (every triangle of level 2 has a refined corner)."""
+    rng = np.random.default_rng(3)
+    stars = np.concatenate([rng.uniform(-20, 20, (110, 2)), np.ones((110, 1))], 1)
+    a = irs_b200.AdaptiveIPM(kappa_tot=0.3, shear=0.1, smooth_fraction=0.0, half_length_y1=1.0, half_length_y2=1.0,
+                             num_pixels_y1=16, num_pixels_y2=16, light_loss=0.01, write_histograms=0,
+                             policy="uniform", level=2, audit_fraction=0.0, **{f"center_y{axis}": float("nan")})
+    a.base.set_stars(stars, rectangular=True, corner=(20.0, 20.0), theta_star=1.0)
+    a.run()
+    assert not a.magnifications.any()
+    a.close()
