@@ -63,6 +63,7 @@ double get_value(Obj* self, const char* name) {
   if (n == "min_num") return self->min_num;
   if (n == "max_num") return self->max_num;
   if (n == "errors") return self->errors;
+  if (n == "pinned_bytes") return double(irsb::pinned_bytes());
   return std::numeric_limits<double>::quiet_NaN();
 }
 

@@ -8,6 +8,7 @@
 #include "post.cuh"
 
 #include <algorithm>
+#include <cstdlib>
 #include <filesystem>
 #include <fstream>
 #include <iostream>
@@ -15,6 +16,64 @@
 #include <vector>
 
 namespace irsb {
+
+// Host memory of the map and of a few words of status behind it, on pages of
+// its own so that it can be pinned in place. Pinned memory makes the transfers
+// faster but takes long to get, also for a few bytes (B200, first run of a new
+// object, pinned against pageable: 100^2 pixels 2.4 / 0.53 ms, 1000^2 7.9 / 4.5;
+// repeated runs 0.10 / 0.11 and 0.63 / 0.90). Pinning memory that is there takes
+// 0.33 ms (100^2) and 2 - 4 ms (1000^2), what about 10 to 30 runs gain by it. So
+// it is pinned when it has been filled kPinAfter times: an object that runs once
+// never pays for it, one that runs often about twice at most.
+struct HostMap {
+  static constexpr int kWords = 3;
+  int *p = nullptr, *words = nullptr;
+  size_t n = 0;
+  HostMap() = default;
+  HostMap(const HostMap&) = delete;
+  HostMap& operator=(const HostMap&) = delete;
+  ~HostMap() { release(); }
+  void release() {
+    if (pinned_) {
+      cudaHostUnregister(p);
+      pinned_bytes() -= bytes();
+    }
+    std::free(p);
+    p = words = nullptr;
+    n = cap_ = 0;
+    fills_ = 0;
+    pinned_ = false;
+  }
+  // Room for want values, to be filled once; contents kept only where it suffices.
+  bool prepare(size_t want) {
+    if (want > cap_) {
+      release();
+      const size_t room = ((want + kWords) * sizeof(int) + kPage - 1) / kPage * kPage;
+      p = static_cast<int*>(std::aligned_alloc(kPage, room));
+      if (!p) {
+        std::cerr << "Error. No host memory for the map.\n";
+        return false;
+      }
+      cap_ = room / sizeof(int) - kWords;
+      words = p + cap_;
+    } else if (fills_ == kPinAfter) {
+      pinned_ = cudaHostRegister(p, size_t(bytes()), cudaHostRegisterDefault) == cudaSuccess;
+      if (pinned_) pinned_bytes() += bytes();
+      else cudaGetLastError();  // stays pageable
+    }
+    fills_++;
+    n = want;
+    return true;
+  }
+
+ private:
+  static constexpr size_t kPage = 4096;
+  static constexpr long long kPinAfter = 16;
+  size_t cap_ = 0;
+  long long fills_ = 0;
+  bool pinned_ = false;
+  long long bytes() const { return (long long)((cap_ + kWords) * sizeof(int)); }
+};
 
 template <typename T>
 class NCC {
@@ -37,7 +96,7 @@ class NCC {
   double t_ncc = 0, t_reduce = 0;
   int num_rows = 0, num_cols = 0, min_num = 0, max_num = 0, errors = 0;
   std::vector<int> histogram;
-  HostVec<int> map;  // pinned: the transfer's own target
+  HostMap map;
 
   ~NCC() {
     for (cudaEvent_t* e : {&e0_, &e1_, &e2_})
@@ -94,13 +153,14 @@ class NCC {
     const bool pooled = B <= 8;  // the fine map is not stored
     if (!d_caus_.alloc_exact(caus.size()) || !d_diff_.alloc_exact(ndiff) ||
         (!pooled && !d_fine_.alloc_exact(fx * fy)) || !d_out_.alloc_exact(nout) || !d_stat_.alloc_exact(3) ||
-        !h_stat_.alloc(3) || !map.alloc(nout))
+        !map.prepare(nout))
       return false;
     IRSB_CKR(cudaMemsetAsync(d_diff_.p, 0, ndiff * sizeof(int), s));
-    h_stat_.p[0] = 0;  // errors, smallest, largest value
-    h_stat_.p[1] = std::numeric_limits<int>::max();
-    h_stat_.p[2] = std::numeric_limits<int>::min();
-    IRSB_CKR(cudaMemcpyAsync(d_stat_.p, h_stat_.p, 3 * sizeof(int), cudaMemcpyHostToDevice, s));
+    int* stat = map.words;
+    stat[0] = 0;  // errors, smallest, largest value
+    stat[1] = std::numeric_limits<int>::max();
+    stat[2] = std::numeric_limits<int>::min();
+    IRSB_CKR(cudaMemcpyAsync(d_stat_.p, stat, 3 * sizeof(int), cudaMemcpyHostToDevice, s));
     IRSB_CKR(cudaMemcpyAsync(d_caus_.p, caus.data(), caus.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
     const NccGeom g{double(center_y.re), double(center_y.im), double(half_length_y.re), double(half_length_y.im),
                     int(fx), int(fy)};
@@ -126,20 +186,25 @@ class NCC {
       IRSB_LAUNCH_CK("ncc_pool");
     }
     IRSB_CKR(cudaEventRecord(e2_, s));
-    IRSB_CKR(cudaMemcpyAsync(h_stat_.p, d_stat_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    const bool small = nout <= kSmallMap;
+    IRSB_CKR(cudaMemcpyAsync(stat, d_stat_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (small) IRSB_CKR(cudaMemcpyAsync(map.p, d_out_.p, nout * sizeof(int), cudaMemcpyDeviceToHost, s));
     IRSB_CKR(cudaStreamSynchronize(s));
     float m01 = 0, m12 = 0;
     IRSB_CKR(cudaEventElapsedTime(&m01, e0_, e1_));
     IRSB_CKR(cudaEventElapsedTime(&m12, e1_, e2_));
     t_ncc = m01 * 1e-3;
     t_reduce = m12 * 1e-3;
-    errors = h_stat_.p[0];
-    min_num = h_stat_.p[1];
-    max_num = h_stat_.p[2];
+    errors = stat[0];
+    min_num = stat[1];
+    max_num = stat[2];
     if (errors) std::cerr << "Error. Caustic crossing takes place outside the desired region.\n";
-    IRSB_CKR(cudaMemcpyAsync(map.p, d_out_.p, nout * sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (!small) IRSB_CKR(cudaMemcpyAsync(map.p, d_out_.p, nout * sizeof(int), cudaMemcpyDeviceToHost, s));
     histogram.clear();
-    if (write_histograms && min_num >= 0) {  // include/ncc.cuh:330-355
+    if (write_histograms && min_num >= 0 && small) {  // include/ncc.cuh:330-355
+      histogram.assign(max_num - min_num + 1, 0);
+      for (long long k = 0; k < nout; k++) histogram[map.p[k] - min_num]++;
+    } else if (write_histograms && min_num >= 0) {
       const int len = max_num - min_num + 1;
       if (!d_hist_.alloc_exact(len)) return false;
       IRSB_CKR(cudaMemsetAsync(d_hist_.p, 0, size_t(len) * sizeof(int), s));
@@ -152,7 +217,7 @@ class NCC {
       histogram.resize(len);
       IRSB_CKR(cudaMemcpyAsync(histogram.data(), d_hist_.p, size_t(len) * sizeof(int), cudaMemcpyDeviceToHost, s));
     }
-    IRSB_CKR(cudaStreamSynchronize(s));
+    if (!small) IRSB_CKR(cudaStreamSynchronize(s));
     if (min_num < 0) {
       std::cerr << "Error. Number of caustic crossings should be >= 0\n";
       return false;
@@ -208,11 +273,15 @@ class NCC {
   }
 
  private:
+  // Up to this many pixels the map comes with the status, in one synchronisation,
+  // and the host counts the histogram; beyond, the device does while the map is
+  // in transfer. Repeated runs (B200, host / device): 8^2 pixels 0.067 / 0.086 ms,
+  // 64^2 0.087 / 0.098, 100^2 0.105 / 0.105, 180^2 0.143 / 0.122.
+  static constexpr long long kSmallMap = 8192;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr, e2_ = nullptr;
   DevVec<double2> d_caus_;
   DevVec<int> d_diff_, d_fine_, d_out_, d_stat_, d_hist_;
-  HostVec<int> h_stat_;
 
   // read_complex_array (include/array_functions.cuh:172-268): int nrows, int
   // ncols, then complex values in T, float or double (by the file size).

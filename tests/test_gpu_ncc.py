@@ -1,6 +1,7 @@
 """NCC on the GPU (lib_ncc.so) against the C restatement (oracle.c orc_ncc,
 pinned against the reference's own kernels in tests/test_ncc_oracle.py):
 integer maps, bit for bit; and the chain CCF -> ccf_caustics.bin -> NCC."""
+import gc
 import os
 import struct
 
@@ -67,6 +68,36 @@ def test_ccf_to_ncc_through_files(tmp_path):
     assert np.array_equal(hist[:, 0], vals) and np.array_equal(hist[:, 1], counts)
     assert "over_sample 2" in open(tmp_path / "ncc_parameter_info.txt").read()
     c.close()
+    n.close()
+
+
+@pytest.mark.parametrize("npix", [1, 90, 91, 300])
+def test_ncc_pins_the_map_of_an_object_that_runs_often(tmp_path, npix):
+    """Page-locked memory takes longer to get than one run gains by it: a new
+    object's map stays pageable and is pinned in place after 16 runs; a size that
+    does not fit starts anew. The map is the same throughout, on both sides of
+    8192 pixels, up to which the host counts the histogram."""
+    from irs_b200 import NCC
+    c = oracle_caustics(5, 8, 40)
+    n = NCC(half_length_y1=4, half_length_y2=4, num_pixels_y1=npix, num_pixels_y2=npix, over_sample=1)
+    n.set_caustics(c)
+    gc.collect()  # objects of other tests hold no memory any more
+    before = n.value("pinned_bytes")
+    ref, _ = po.ncc(c, (0, 0), (4, 4), (npix, npix), 1)
+    for run in range(1, 19):
+        n.run()
+        assert (n.value("pinned_bytes") - before >= 4 * npix * npix) == (run > 16)
+        assert np.array_equal(n.num_caustic_crossings, ref)
+    for size in (npix // 2 + 1, npix + 40):  # fits the memory at hand; does not
+        n.num_pixels_y1 = n.num_pixels_y2 = size
+        n.run()
+        assert np.array_equal(n.num_caustic_crossings, po.ncc(c, (0, 0), (4, 4), (size, size), 1)[0])
+        assert (n.value("pinned_bytes") > before) == (size <= npix)
+    n.outfile_prefix = str(tmp_path) + "/"
+    n.save()
+    hist = np.loadtxt(tmp_path / "ncc_ncc_numpixels.txt", dtype=np.int64, ndmin=2)
+    vals, counts = np.unique(n.num_caustic_crossings, return_counts=True)
+    assert np.array_equal(hist[:, 0], vals) and np.array_equal(hist[:, 1], counts)
     n.close()
 
 
