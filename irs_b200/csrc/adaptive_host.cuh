@@ -450,8 +450,7 @@ class AdaptiveIPM {
     if (!lattice_rects<T>(rtiles_, base.leaves_, base.tree_, base.leaves_.n, sps.base_x, sps.base_y, sps.rhs_x,
                           sps.rhs_y, nxs, nys, jlo, jhi, s))
       return false;
-    IRSB_CKR(cudaStreamSynchronize(s));
-    if (!lattice_table<T>(rtiles_, base.leaves_, base.tree_, s)) return false;
+    if (!tree_status(base.tree_, kTreeOff, s) || !lattice_table<T>(rtiles_, base.leaves_, base.tree_, s)) return false;
     LeafPtrs lp = base.leaf_ptrs();
     lp.rect = rtiles_.rect.p;
     lp.tile_off = rtiles_.tile_off.p;

@@ -689,9 +689,8 @@ class BatchMaker {
   }
 
   bool check(int* st) {
-    int* h = tree_.h_status.p;
-    IRSB_CKR(cudaMemcpyAsync(h, tree_.status.p, kTreeOff * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    IRSB_CKR(cudaStreamSynchronize(stream_));
+    if (!tree_status(tree_, kTreeOff, stream_)) return false;
+    const int* h = tree_.h_status.data();
     if (h[kTreeBarrier]) {
       std::cerr << "Error. The batch's tree build or expansions did not finish.\n";
       return false;

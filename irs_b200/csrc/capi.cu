@@ -187,6 +187,7 @@ double get_value(Obj* self, const char* name) {
   if (n == "t_deposit") return self->t_deposit;
   if (n == "mean_near") return self->mean_near;
   if (n == "launches") return double(self->launches);
+  if (n == "pinned_bytes") return double(irsb::pinned_bytes());
   if (n == "num_lattice_points") return double(self->num_tiles >= 0 ? 1 : 0) *
       (IRSB_IRS ? double(p.num_ray_threads.re) * p.num_ray_threads.im
                 : double(p.num_ray_threads.re + 1) * (p.num_ray_threads.im + 1));

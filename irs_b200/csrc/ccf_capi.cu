@@ -68,6 +68,7 @@ void set_num_iters(Obj* self, int init_iters, int step_iters) {
 double get_value(Obj* self, const char* name) {
   const std::string n = name ? name : "";
   if (n == "max_error") return double(self->max_error);
+  if (n == "pinned_bytes") return double(irsb::pinned_bytes());
   if (n == "t_init_roots") return self->t_init_roots;
   if (n == "t_ccs") return self->t_ccs;
   if (n == "t_caustics") return self->t_caustics;

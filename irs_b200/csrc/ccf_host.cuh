@@ -220,9 +220,7 @@ class CCF {
     stars_out.resize(n);
     IRSB_CKR(cudaMemcpyAsync(stars_out.data(), d_stars_.p, size_t(n) * sizeof(StarRec<T>), cudaMemcpyDeviceToHost,
                              s));
-    if (!fetch_leaf_status(tree_, s)) return false;
-    IRSB_CKR(cudaStreamSynchronize(s));
-    if (!leaves_ok(tree_)) return false;
+    if (!tree_status(tree_, kTreeOff, s) || !leaves_ok(tree_)) return false;
     std::vector<double2> pos(n);  // star positions in tree order, for the sums over all stars
     for (int i = 0; i < n; i++) pos[i] = make_double2(double(stars_out[i].x), double(stars_out[i].y));
     if (!d_spos_.alloc_exact(n)) return false;

@@ -289,8 +289,8 @@ class MapMaker {
     if (!build_tree<T>(tree_, d_stars_.p, n, prm.root_half_length, leaves_.pos, leaves_.node, stream_, rects))
       return false;
     launches += tree_.launches + 4;
-    const unsigned long long* st = tiles_.h_stat.p;
-    mean_near = st[kLatPoints] > 0 ? double(st[kLatNear]) / double(st[kLatPoints]) : 0;
+    const double points = double(lattice_count(tree_, kLatPoints));
+    mean_near = points > 0 ? double(lattice_count(tree_, kLatNear)) / points : 0;
     prm.tree_levels = tree_.levels;
     prm.expansion_order =
         prm.expansion_order_override > 0 ? prm.expansion_order_override : expansion_order_of(prm);
@@ -313,10 +313,8 @@ class MapMaker {
     launches += 4;
     num_tiles = tiles_.total;
     if (!shoot()) return false;
-    if (!fetch_leaf_status(tree_, stream_)) return false;
     IRSB_CKR(cudaEventRecord(ev2_, stream_));
-    IRSB_CKR(cudaEventSynchronize(ev2_));
-    if (!leaves_ok(tree_)) return false;
+    if (!tree_status(tree_, kTreeOff, stream_) || !leaves_ok(tree_)) return false;
     float ms_shoot = 0, ms_all = 0, ms_lat = 0, ms_dep = 0;
     IRSB_CKR(cudaEventElapsedTime(&ms_shoot, ev1_, ev2_));
     IRSB_CKR(cudaEventElapsedTime(&ms_all, ev0_, ev2_));
@@ -553,7 +551,6 @@ class MapMaker {
   DevVec<unsigned long long> d_red_;
   static constexpr int kMaxRanges = 3;
   DevVec<long long> d_mm_;
-  HostVec<long long> h_mm_;
 
   bool init_stream() {
     if (stream_) return true;
@@ -737,8 +734,9 @@ class MapMaker {
   bool value_ranges(const V* const* maps, int nmaps, long long n, V* lo, V* hi) {
     using K = typename OrderedKey<V>::K;
     static_assert(sizeof(K) <= sizeof(long long), "keys fit the buffers");
-    if (!d_mm_.alloc_exact(2 * kMaxRanges) || !h_mm_.alloc(2 * kMaxRanges)) return false;
-    K *dm = reinterpret_cast<K*>(d_mm_.p), *hm = reinterpret_cast<K*>(h_mm_.p);
+    if (!d_mm_.alloc_exact(2 * kMaxRanges)) return false;
+    K* dm = reinterpret_cast<K*>(d_mm_.p);
+    K hm[2 * kMaxRanges];
     for (int i = 0; i < nmaps; i++) {
       hm[2 * i] = std::numeric_limits<K>::max();
       hm[2 * i + 1] = std::numeric_limits<K>::min();

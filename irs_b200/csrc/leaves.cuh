@@ -36,6 +36,8 @@
 #include "smooth.cuh"
 #include "tree.cuh"
 
+#include <cstring>
+
 namespace irsb {
 
 // Tree nodes needed by the descent, and the node -> leaf map. The descent is
@@ -90,14 +92,24 @@ struct LatticeTiles {
   DevVec<long long> tiles;
   DevVec<long long> tile_off;  // [n + 1]
   DevVec<int4> table;          // per tile: leaf, i0, j0, (ni << 16) | nj
-  DevVec<unsigned long long> stat;    // LatticeStat
-  HostVec<unsigned long long> h_stat;  // pinned copy
   long long total = 0;
   ScanScratch scan;
 };
-// Lattice points in leaves, and those weighted with their leaf's near-field
-// star count (the tile total is in `scan.sum`, copied to the third word).
+// Lattice points in leaves, those weighted with their leaf's near-field star
+// count, and the tiles: 64-bit words of the tree's status from kTreeLattice on, so
+// that they come to the host with it.
 enum LatticeStat : int { kLatPoints = 0, kLatNear = 1, kLatTiles = 2, kLatWords = 3 };
+static_assert(kTreeLattice % 2 == 0 && kTreeOff - kTreeLattice == 2 * kLatWords, "room and alignment of the counts");
+template <typename T>
+unsigned long long* lattice_stat(const TreeDev<T>& t) {
+  return reinterpret_cast<unsigned long long*>(t.status.p + kTreeLattice);
+}
+template <typename T>
+unsigned long long lattice_count(const TreeDev<T>& t, LatticeStat k) {
+  unsigned long long v;
+  std::memcpy(&v, t.h_status.data() + kTreeLattice + 2 * k, sizeof(v));
+  return v;
+}
 
 // kTableLanes consecutive lanes per leaf write the table entries of its tiles
 // (row-major over the leaf's rectangle), lane q entries q, q + kTableLanes, ...
@@ -365,19 +377,15 @@ bool build_leaves(LeafSet& L, TreeDev<T>& t, FmmDev& f, const StarRec<T>* stars,
   return true;
 }
 
-// Fetches the tree's status after the expansions and leaf records on stream s;
-// leaves_ok reads it once the stream is synchronised.
-template <typename T>
-bool fetch_leaf_status(TreeDev<T>& t, cudaStream_t s) {
-  return IRSB_CK(cudaMemcpyAsync(t.h_status.p, t.status.p, kTreeOff * sizeof(int), cudaMemcpyDeviceToHost, s));
-}
+// Whether the expansions and leaf records, done by then, went well (from the
+// status on the host, tree_status).
 template <typename T>
 bool leaves_ok(const TreeDev<T>& t) {
-  if (t.h_status.p[kTreeBarrier]) {
+  if (t.h_status[kTreeBarrier]) {
     std::fprintf(stderr, "Error. The expansions did not finish.\n");
     return false;
   }
-  if (t.h_status.p[kTreeNear]) {
+  if (t.h_status[kTreeNear]) {
     std::fprintf(stderr, "Error. A leaf's near field holds more than %d stars.\n", kMaxStarsDirect);
     return false;
   }
@@ -386,38 +394,36 @@ bool leaves_ok(const TreeDev<T>& t) {
 
 // The leaves' rectangles on a lattice and the offsets of their tiles, from the
 // tree as it is on the device (at most cap leaves): no synchronisation. The
-// counts reach W.h_stat when the stream is next synchronised.
+// counts are in the tree's status (LatticeStat).
 template <typename T>
 bool lattice_rects(LatticeTiles& W, const LeafSet& L, TreeDev<T>& t, long long cap, double base_x, double base_y,
                    double rhs_x, double rhs_y, long long nx, long long ny, long long jlo, long long jhi,
                    cudaStream_t s) {
   if (!W.rect.alloc_exact(cap) || !W.tiles.alloc_exact(cap) || !W.tile_off.alloc_exact(cap + 1) ||
-      !W.stat.alloc_exact(kLatWords) || !W.h_stat.alloc(kLatWords) || !scan_reserve(W.scan, cap, s))
+      !scan_reserve(W.scan, cap, s))
     return false;
+  unsigned long long* stat = lattice_stat(t);
   const int* dn = t.status.p + kTreeLeaves;
-  IRSB_CKR(cudaMemsetAsync(W.stat.p, 0, kLatWords * sizeof(unsigned long long), s));
+  IRSB_CKR(cudaMemsetAsync(stat, 0, kLatWords * sizeof(unsigned long long), s));
   const int blocks = std::max(1, std::min(ceil_div(cap, 256), 148 * 8));
   leaf_rects<<<blocks, 256, 0, s>>>(dn, L.node.p, t.lox.p, t.hix.p, t.loy.p, t.hiy.p, t.scnt.p, t.nbr.p, t.n_nbr.p,
                                     base_x, base_y, rhs_x, rhs_y, nx, ny, jlo, jhi, kTileX, kTileY, W.rect.p,
-                                    W.tiles.p, W.stat.p);
+                                    W.tiles.p, stat);
   IRSB_LAUNCH_CK("leaf_rects");
-  if (!exclusive_scan_dev<long long>(W.tiles.p, dn, cap, W.tile_off.p, W.scan, s,
-                                     reinterpret_cast<long long*>(W.stat.p + kLatTiles)))
-    return false;
-  IRSB_CKR(cudaMemcpyAsync(W.h_stat.p, W.stat.p, kLatWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  return true;
+  return exclusive_scan_dev<long long>(W.tiles.p, dn, cap, W.tile_off.p, W.scan, s,
+                                       reinterpret_cast<long long*>(stat + kLatTiles));
 }
 
-// The tile table of the lattice counted by lattice_rects (after the
-// synchronisation).
+// The tile table of the lattice counted by lattice_rects, whose counts the host
+// has (tree_status).
 template <typename T>
 bool lattice_table(LatticeTiles& W, const LeafSet& L, TreeDev<T>& t, cudaStream_t s) {
-  W.total = (long long)W.h_stat.p[kLatTiles];
+  W.total = (long long)lattice_count(t, kLatTiles);
   if (!W.table.alloc_exact(std::max<long long>(W.total, 1))) return false;
   const int blocks = std::max(1, std::min(ceil_div((long long)L.n * kTableLanes, 256), 148 * 8));
   leaf_tile_table<<<blocks, 256, 0, s>>>(L.n, nullptr, W.rect.p, W.tile_off.p,
-                                         reinterpret_cast<const long long*>(W.stat.p + kLatTiles), kTileX, kTileY,
-                                         W.table.p, W.total, t.status.p + kTreeTable);
+                                         reinterpret_cast<const long long*>(lattice_stat(t) + kLatTiles), kTileX,
+                                         kTileY, W.table.p, W.total, t.status.p + kTreeTable);
   IRSB_LAUNCH_CK("leaf_tile_table");
   return true;
 }

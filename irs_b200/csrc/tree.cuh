@@ -53,7 +53,7 @@ struct TreeDev {
   DevVec<int> status;       // TreeStatus, then the level offsets (the FMM reads them there)
   DevVec<unsigned long long> words;  // grid barriers of the build and of the expansions
   DevVec<StarRec<T>> tmp_stars, star_backup;
-  HostVec<int> h_status;    // pinned copy of `status`
+  std::vector<int> h_status;  // copy of `status`
   long long launches = 0;   // kernels the last build launched
 };
 
@@ -90,7 +90,8 @@ enum TreeStatus : int {
   kTreeLeaves = 3,     // leaves
   kTreeNear = 4,       // a leaf's near field overflowed (leaf_build, build_leaves)
   kTreeTable = 5,      // the tile table overflowed (leaf_tile_table)
-  kTreeOff = 8,
+  kTreeLattice = 6,    // LatticeStat: 64-bit words (lattice_rects)
+  kTreeOff = kTreeLattice + 2 * 3,
   kTreeStatusWords = kTreeOff + kMaxLevels + 2,
 };
 // Grid barriers of a build: at most four per level, one for the leaves; then
@@ -643,8 +644,17 @@ template <typename T>
 bool tree_build_reserve(TreeDev<T>& t, int nstars, int cap, cudaStream_t s) {
   return tree_reserve(t, cap, s) && t.split.reserve(cap, s) && t.rank.reserve(cap, s) &&
          t.cta.reserve((3 + 4 * kShareNodes) * 1024, s) && t.status.reserve(kTreeStatusWords, s) &&
-         t.words.reserve(kTreeBarriers + kFmmBarriers, s) && t.tmp_stars.reserve(nstars, s) &&
-         t.h_status.alloc(kTreeStatusWords);
+         t.words.reserve(kTreeBarriers + kFmmBarriers, s) && t.tmp_stars.reserve(nstars, s);
+}
+
+// The first n status words to the host, once the work queued on s is done (the
+// copy goes to pageable memory, so the call waits for it; pinning these few words
+// took 0.5 - 1 ms of every new object's first run).
+template <typename T>
+bool tree_status(TreeDev<T>& t, int n, cudaStream_t s) {
+  t.h_status.resize(kTreeStatusWords);
+  IRSB_CKR(cudaMemcpyAsync(t.h_status.data(), t.status.p, n * sizeof(int), cudaMemcpyDeviceToHost, s));
+  return IRSB_CK(cudaStreamSynchronize(s));
 }
 
 // Builds the tree over `stars` (device, permuted in place into tree order) and
@@ -675,9 +685,8 @@ bool build_tree(TreeDev<T>& t, StarRec<T>* stars, int nstars, T root_hl, DevVec<
       return false;
     t.launches++;
     if (!before_sync(cap)) return false;
-    IRSB_CKR(cudaMemcpyAsync(t.h_status.p, t.status.p, kTreeStatusWords * sizeof(int), cudaMemcpyDeviceToHost, s));
-    IRSB_CKR(cudaStreamSynchronize(s));
-    const int* st = t.h_status.p;
+    if (!tree_status(t, kTreeStatusWords, s)) return false;
+    const int* st = t.h_status.data();
     const int err = st[kTreeErr];
     if (st[kTreeBarrier]) {
       std::fprintf(stderr, "Error. The tree build did not finish.\n");

@@ -246,3 +246,26 @@ def test_deposition_order_covers_every_cell_once(gpu, dbl, ncx, ncy):
     got = float(d_map.double().sum())
     tol = ncx * ncy * 2 * 6 * 2.0 ** -32 + ncx * ncy * 2.0 ** -22
     assert abs(got - ncx * ncy) <= tol
+
+
+def test_new_objects_take_no_pinned_memory_for_their_status(gpu):
+    """Page-locked memory takes about a millisecond to get, more than the whole run
+    of a small object: the first run of critical curves or of an adaptive map
+    takes none, that of a map only what its pixels come back in."""
+    import gc
+
+    def pinned(make):
+        gc.collect()
+        m = make()
+        before = m.value("pinned_bytes")
+        m.run()
+        got = m.value("pinned_bytes") - before
+        m.close()
+        return got
+
+    lens, size = dict(kappa_tot=0.3, shear=0.3, kappa_star=0.27), dict(num_pixels_y1=32, num_pixels_y2=24)
+    assert pinned(lambda: irs_b200.CCF(**lens, num_stars=3, num_phi=8, random_seed=5)) == 0
+    ipm, irs = (dict(kw, **size, write_histograms=1) for kw in (IPM_SMALL, IRS_SMALL))
+    assert pinned(lambda: irs_b200.AdaptiveIPM(**ipm)) == 0
+    assert pinned(lambda: irs_b200.IPM(**ipm)) == 4 * 32 * 24
+    assert pinned(lambda: irs_b200.IRS(**irs)) == 4 * 32 * 24
