@@ -227,6 +227,13 @@ __device__ __forceinline__ double2 refine_point(const AdaGeom& g, const ShootPar
 // each star read from shared memory for one point, and every point of a tile
 // that a leaf boundary crosses found by its own descent: 58 ms for 2.0e9 corners of a
 // 1024^2 map (B200); now 31 ms.
+//
+// GENERIC_SMOOTH: an exact sheet's deviation from the linear form is added in a
+// pass of its own over the group's points, each with the centre of its leaf. It
+// costs far more than the stars (four complex logarithms for a rectangle), and in
+// the rounds, which a dense field has several of per group, every round paid for
+// it with a few lanes at work: a 128^2 map of a rectangular Kroupa field 637 ms
+// (332 with one point per thread, 217 now).
 constexpr int kAdaThreads = 128;
 constexpr int kAdaRows = 8;  // corner rows per warp
 constexpr int kAdaBand = kAdaRows * kAdaThreads / 32;
@@ -246,7 +253,7 @@ __device__ __noinline__ double2 refine_point_call(const AdaGeom& g, const ShootP
 }
 
 template <typename T, bool GENERIC_SMOOTH>
-__global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refine_tiles(const __grid_constant__ AdaGeom g,
+__global__ void __launch_bounds__(kAdaThreads, 4) ada_refine_tiles(const __grid_constant__ AdaGeom g,
                                                                 const __grid_constant__ ShootParams sp,
                                                                 const __grid_constant__ LeafPtrs lp,
                                                                 const __grid_constant__ DescentPtrs<T> dp,
@@ -265,6 +272,7 @@ __global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refin
   const LeafView& L = s_view[w];
   const double4& box = s_box[w];
   const int sh = __ffs(s) - 1, fstep = kAdaMaxLevel >> sh;
+  const double scx = sp.npx / (2.0 * sp.hly_re), scy = sp.npy / (2.0 * sp.hly_im);
   if (lane == 0) s_box[w] = make_double4(1.0, 0.0, 1.0, 0.0);  // nothing staged: empty
   __syncwarp();
   for (long long item = blockIdx.x; item < ada_refine_items(nlist, s); item += gridDim.x) {
@@ -340,19 +348,25 @@ __global__ void __launch_bounds__(kAdaThreads, GENERIC_SMOOTH ? 2 : 4) ada_refin
               const float Sx = sx[r] + cxr[r], Sy = sy[r] + cyr[r];
               const float wr = fmaf(float(L.lin_x), ux, -(Sx + Ar[r]));
               const float wi = fmaf(float(L.lin_y), uy[r], -(Sy - Ai[r]));
-              double px = L.pcx + double(wr) * L.scx;
-              double py = L.pcy + double(wi) * L.scy;
-              if (GENERIC_SMOOTH) {
-                const cplx<double> corner = mk(sp.corner_re, sp.corner_im);
-                const cplx<double> z = mk(L.cx + double(ux), L.cy + double(uy[r]));
-                const cplx<double> a_sm =
-                    alpha_smooth_(z, sp.kstar, sp.rect, corner, sp.approx, sp.taylor_smooth, sp.inv_pi);
-                px += (-a_sm.re - sp.kstar * z.re) * L.scx;
-                py += (-a_sm.im - sp.kstar * z.im) * L.scy;
-              }
-              v = make_double2(px, double(sp.npy) - py);
+              const double px = L.pcx + double(wr) * L.scx, py = L.pcy + double(wi) * L.scy;
+              v = make_double2(px, GENERIC_SMOOTH ? py : double(sp.npy) - py);  // the sheet is added below
             }
             o[(long long)b * w1 + a] = v;
+          }
+        }
+        if constexpr (GENERIC_SMOOTH) {
+          const int own = dp.tile_leaf ? dp.tile_leaf[t] : -1;
+#pragma unroll 1
+          for (int b = r0; b <= rlast; b++) {
+            if (a >= wa || ((a | b) & (s - 1)) == 0 || (a == 0 && coarse_left) || (b == 0 && coarse_low)) continue;
+            const double y = coord_y(b);
+            const int leaf = own >= 0 ? own : descend_leaf(dp, x, y);
+            const double lcx = lp.cx[leaf], lcy = lp.cy[leaf];
+            const cplx<double> z = mk(lcx + double(float(x - lcx)), lcy + double(float(y - lcy)));
+            const cplx<double> a_sm = alpha_smooth_call(z, sp);
+            double2* v = o + (long long)b * w1 + a;  // this lane's own point
+            const double px = v->x + (-a_sm.re - sp.kstar * z.re) * scx, py = v->y + (-a_sm.im - sp.kstar * z.im) * scy;
+            *v = make_double2(px, double(sp.npy) - py);
           }
         }
       }
