@@ -243,7 +243,7 @@ class MapMaker {
     prm = p;
 
     launches = from_stars ? 0 : 1;  // star generation
-    // the logarithmic moment, for the parameter file, while the tree is built
+    // the logarithmic moment, for the parameter file, while the device works
     const auto log_moment = [&] {
       prm.mean_mass2_ln_mass_actual = star_field_log_moment<T>(n, stars_out.data());
       if (from_stars) prm.mean_mass2_ln_mass = prm.mean_mass2_ln_mass_actual;
@@ -267,8 +267,9 @@ class MapMaker {
   // timed with CUDA events (t_pipeline, t_shoot, t_lattice, t_deposit).
   // One host synchronisation before the end: the tree's depth (the expansion
   // order follows from it) and the number of lattice tiles are read together,
-  // after the build and the leaves' rectangles; host_work() runs on the host
-  // meanwhile.
+  // after the build and the leaves' rectangles. host_work() runs on the host once
+  // everything is queued: before that synchronisation, the device waited for it
+  // where it took longer than the tree (1e6 stars, 9.2 ms of device work: 10.2).
   template <typename F>
   bool device_pipeline(F host_work) {
     const int n = prm.num_stars;
@@ -277,14 +278,9 @@ class MapMaker {
     const auto band = band_rows();
     // rays: rows [lo, hi); cells: rows [lo, hi) need corner rows [lo, hi]
     const long long jlo = band.first, jhi = IS_IRS ? band.second : band.second + 1;
-    bool worked = false;
     auto rects = [&](long long cap) {
-      if (!lattice_rects<T>(tiles_, leaves_, tree_, cap, lat.base_x, lat.base_y, lat.rhs_x, lat.rhs_y, lat.nx, lat.ny,
-                            jlo, jhi, stream_))
-        return false;
-      if (!worked) host_work();  // once, also when the build is repeated
-      worked = true;
-      return true;
+      return lattice_rects<T>(tiles_, leaves_, tree_, cap, lat.base_x, lat.base_y, lat.rhs_x, lat.rhs_y, lat.nx, lat.ny,
+                              jlo, jhi, stream_);
     };
     if (!build_tree<T>(tree_, d_stars_.p, n, prm.root_half_length, leaves_.pos, leaves_.node, stream_, rects))
       return false;
@@ -314,6 +310,7 @@ class MapMaker {
     num_tiles = tiles_.total;
     if (!shoot()) return false;
     IRSB_CKR(cudaEventRecord(ev2_, stream_));
+    host_work();
     if (!tree_status(tree_, kTreeOff, stream_) || !leaves_ok(tree_)) return false;
     float ms_shoot = 0, ms_all = 0, ms_lat = 0, ms_dep = 0;
     IRSB_CKR(cudaEventElapsedTime(&ms_shoot, ev1_, ev2_));
