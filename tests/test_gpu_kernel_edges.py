@@ -15,16 +15,22 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 2, 7, 8, 9, 15, 16, 17, 31, 33])
 def test_lattice_bands_equal_whole_lattice(gpu, dbl, rows):
     """A band of few lattice rows (tiles of 1 to 33 rows, cut anywhere) holds the
-    corner positions of the whole lattice, and the maps of the bands that
-    cover it add up to its map."""
+    corner positions of the whole lattice, and the fixed-point maps of the bands
+    that cover it (that one, those before it and after it) add up to its map."""
     cfg = dict(IPM_SMALL, num_pixels_y1=40, num_pixels_y2=24, half_length_y1=1.25, half_length_y2=0.75)
     m = irs_b200.IPM(**cfg, is_double=dbl, expansion_order=10)
     m.run()
-    whole = m.vertices()
-    lo = whole.shape[0] // 2 - rows // 2
-    m.lib.set_band(m.obj, lo, lo + rows)
-    m.run()
-    np.testing.assert_array_equal(m.vertices(), whole[lo:lo + rows + 1])
+    whole, total = m.vertices(), m.fixed_maps()
+    assert total.any()
+    n = whole.shape[0] - 1  # rows of cells
+    lo = n // 2 - rows // 2
+    acc = np.zeros_like(total)
+    for a, b in ((0, lo), (lo, lo + rows), (lo + rows, n)):
+        m.lib.set_band(m.obj, a, b)
+        m.run()
+        np.testing.assert_array_equal(m.vertices(), whole[a:b + 1])
+        acc += m.fixed_maps()
+    np.testing.assert_array_equal(acc, total)
     m.close()
 
 
@@ -222,7 +228,7 @@ def test_deposition_of_awkward_cells(gpu, dbl, kind):
 def test_deposition_order_covers_every_cell_once(gpu, dbl, ncx, ncy):
     """Lattices of fewer cells than a warp, of one chunk per warp, and of more
     chunks than one wave or one grid of warps holds: every cell deposits its
-    area exactly once."""
+    area exactly once, in a pixel of its own."""
     import ctypes
 
     import torch
@@ -233,19 +239,35 @@ def test_deposition_order_covers_every_cell_once(gpu, dbl, ncx, ncy):
     f.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_longlong, T, ctypes.c_int, ctypes.c_int,
                   ctypes.c_void_p, ctypes.c_void_p]
     f.restype = ctypes.c_int
-    npx = npy = 16
-    # cell (i, j) lies inside pixel (i mod 16, j mod 16): both triangles deposit there whole
-    i, j = torch.arange(ncx + 1, device="cuda"), torch.arange(ncy + 1, device="cuda")
-    x = 0.5 + 14.9 * (i.double() / ncx)
-    y = 0.5 + 14.9 * (j.double() / ncy)
-    v = torch.stack([x[None, :].expand(ncy + 1, -1), y[:, None].expand(-1, ncx + 1)], -1).contiguous()
-    d_map = torch.zeros((npy, npx), dtype=tdt, device="cuda")
-    assert f(v.data_ptr(), ncx, ncy, 0.5, npx, npy, d_map.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    # cell (i, j) is pixel (i, j): its two triangles of half a pixel deposit factor each, and
+    # 2 * 0.5 is exact in the map's fixed point
+    i, j = torch.arange(ncx + 1, device="cuda").double(), torch.arange(ncy + 1, device="cuda").double()
+    v = torch.stack([i[None, :].expand(ncy + 1, -1), j[:, None].expand(-1, ncx + 1)], -1).contiguous()
+    d_map = torch.full((ncy, ncx), -1.0, dtype=tdt, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    rows = min(1024, 2 ** 20 // ncx)  # the most that a map of this entry point holds
+    for lo in range(0, ncy, rows):
+        hi = min(ncy, lo + rows)
+        # all cells of the lattice each time; those of other rows lie off the map
+        w = torch.stack([v[..., 0], v[..., 1] - lo], -1).contiguous()
+        assert f(w.data_ptr(), ncx, ncy, 0.5, ncx, hi - lo, d_map[lo:hi].data_ptr(), stream) == 0
     torch.cuda.synchronize()
-    # 2 triangles of factor 0.5 per cell; a triangle loses at most 2^-32 per pixel it touches
-    got = float(d_map.double().sum())
-    tol = ncx * ncy * 2 * 6 * 2.0 ** -32 + ncx * ncy * 2.0 ** -22
-    assert abs(got - ncx * ncy) <= tol
+    assert bool((d_map == 1.0).all())
+
+
+def test_batched_deposition_order_covers_every_cell_once(gpu):
+    """The batched form takes blocks of 8 chunks, 32 of them per 32 x 32-cell tile
+    here, more blocks than a grid has warps: an adaptive map at level 1 holds what the plain form
+    deposits from the same corners, bit for bit."""
+    kw = dict(IPM_SMALL, half_length_y1=64.0, half_length_y2=64.0, num_pixels_y1=2048, num_pixels_y2=2048)
+    a = irs_b200.AdaptiveIPM(**kw, policy="uniform", level=1, audit_fraction=0.0)
+    a.run()
+    assert a.value("cells_base") > 2 ** 5 * 8 * 148 * 256 * 2
+    m = irs_b200.IPM(**kw)
+    m.run()
+    np.testing.assert_array_equal(a.magnifications, m.magnifications)
+    a.close()
+    m.close()
 
 
 def test_new_objects_take_no_pinned_memory_for_their_status(gpu):
