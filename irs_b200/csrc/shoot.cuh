@@ -211,9 +211,12 @@ __device__ __forceinline__ void irs_deposit(double px, double py, int npx, int n
 // 1 / d for a normal d: the hardware's FP64 reciprocal approximation (PTX
 // rcp.approx.ftz.f64, about 2^-20) and one third-order (Halley-type) step
 // r (1 + e + e^2), e = 1 - d r, whose truncation 2^-60 is below the rounding:
-// three FMAs and about an ulp, without the range checks and the slow path of a
-// general division. A zero or subnormal d gives NaN, where 1 / d gives inf;
-// both leave the ray without an image.
+// three FMAs, without the range checks and the slow path of a general division.
+// Over normal d of either sign with a normal 1 / d the error is at most 0.51 ulp
+// (2e7 values; 0.50 for the quotient) and the result differs from the rounded
+// quotient for 3 in 1e4. A zero or subnormal d gives NaN, where 1 / d gives inf;
+// both leave the ray without an image. So does an infinite d (a star farther than
+// 1e154), where 1 / d gives 0; a 1 / d below the normal range gives 0.
 __device__ __forceinline__ double rcp_f64(double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
