@@ -270,10 +270,4 @@ inline bool scan_reserve(ScanScratch& sc, long long n_cap, cudaStream_t s) {
   return sc.totals.reserve(size_t(nb < 1 ? 1 : nb), s) && sc.sum.reserve(1, s);
 }
 
-template <typename T>
-__global__ void fill_kernel(T* p, long long n, T v) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    p[i] = v;
-}
-
 }  // namespace irsb
