@@ -18,10 +18,14 @@
 //   * maps: one fixed-point map per realization, resolved and converted in
 //     two launches.
 // Tree build through deposition is captured once per batch shape and replayed.
-// Each realization's map is bit-identical to a single run of the same inputs at
-// the same expansion order: the per-node, per-leaf, per-point and per-cell
-// arithmetic is the single run's, and the fixed-point deposition does not
-// depend on the order of work.
+// Each realization's map is that of a single run of the same inputs at the same
+// expansion order: the per-leaf, per-point and per-cell arithmetic is the single
+// run's, and the fixed-point deposition does not depend on the order of work. The
+// FP64 expansions may differ in their last bits, since a single run spreads a
+// node's interactions over a CTA on levels of few nodes (kFmmBlockNodes) and the
+// batch over a warp on all; a single-precision coefficient that lies next to a
+// rounding boundary then moves by one unit. None does in the fields of the tests
+// and the benchmark, whose maps are bit-identical.
 #pragma once
 #include "engine.cuh"
 
