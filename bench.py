@@ -848,12 +848,13 @@ def our_arm(args):
         achieved = bytes_ / (dep_ms * 1e-3) / 1e9
         peak = peaks.get("hbm_gbs", 6650.0)
         # DRAM traffic measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum) on the 500^2 case of
-        # the same lens and pixel scale: 519 MB for 29.2 M cells, 17.8 B per cell, scaled to this launch
-        traffic = 17.8 * ncells / 1e9
+        # the same lens and pixel scale: 490 MB for 29.2 M cells, 16.8 B per cell, scaled to this launch
+        traffic = 16.8 * ncells / 1e9
         roof = {"kernel": "ipm_deposit_cells", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "traffic_unit": "GB per launch",
-                "traffic_source": "ncu on the 500^2 case (17.8 B per cell), scaled by cells",
-                "limiter": "instruction issue (ncu, a band of a rectangular lattice: 73 % issue-active, ALU pipe 55 %)",
+                "traffic_source": "ncu on the 500^2 case (16.8 B per cell), scaled by cells",
+                "limiter": "instruction issue (ncu, 500^2 case: 65 % issue-active, ALU pipe 49 %; band of a 4096^2 "
+                           "map: 75 %, 59 %)",
                 "algorithmic": f"16 B x {nverts} corner positions + 8 B x {npix} map words"}
     # the lens-equation kernel against the FP32 FMA roofline, whichever kernel dominates
     lens_tflops = flop_per_vertex * nverts / (lat_ms * 1e-3) / 1e12

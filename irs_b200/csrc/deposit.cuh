@@ -275,12 +275,14 @@ constexpr int kDepositThreads = kDepositWarps * 32;
 // at a time; the warps of such a wave share one stretch of the lattice, striding
 // through it (neighbouring warps on neighbouring units, each warp's units spread
 // over the stretch, which evens out the cells' cost). The stretch's images share
-// a part of the map, whose words stay in L2. With the warps striding over the
-// whole lattice every wave swept it end to end, and its adds missed L2 where the
-// fixed-point map is larger: 1.0e9 cells into 4096^2 pixels (268 MB of map
-// words) took 168 ms, now 81.5 (B200); with consecutive units per warp 92 ms,
-// but 5.3 against 4.9 ms for 8.8e7 cells into 2000^2 pixels. Small CTAs retire
-// as soon as their two warps are done, which keeps the SMs full to the end.
+// a part of the map, so that most adds meet their words in L2 (a middle band of the
+// lattice below takes 15 % of the memory bandwidth, corners included).
+// With the warps striding over the whole lattice every wave swept it end to end,
+// and its adds missed L2 where the fixed-point map is larger: 1.0e9 cells into
+// 4096^2 pixels (268 MB of map words) took 168 ms, now 81.5 (B200; 84 to 85 in
+// other fields, where it was 175); with consecutive units per warp 92 ms, but 5.3
+// against 4.9 ms for 8.8e7 cells into 2000^2 pixels. Small CTAs retire as soon as
+// their two warps are done, which keeps the SMs full to the end.
 struct DepositOrder {
   long long first, stride;  // this warp's first unit and the step to its next
   int count;                // units (those past the last unit are absent)
