@@ -112,16 +112,22 @@ struct CcfDerivs {
   cplx<double> dwdzb, d2wdzb2;
 };
 
-__device__ __forceinline__ CcfDerivs ccf_derivs(const CcfParams& P, const CcfField& f, cplx<double> z) {
+// SERIES: the approximate sheet of a rectangle, with the coefficients of its
+// derivatives' series at hand; else any sheet.
+template <bool SERIES = false>
+__device__ __forceinline__ CcfDerivs ccf_derivs(const CcfParams& P, const CcfField& f, cplx<double> z,
+                                                const SmoothSeries<double>* series = nullptr) {
   const cplx<double> corner = mk(P.corner_re, P.corner_im);
   const double t2 = P.theta2;
   // d alpha_star / d zbar = conj(-theta^2 s2); d2 alpha_star / d zbar2 = conj(2 theta^2 s3)
   const cplx<double> das = cconj(cscale(f.s2, -t2)), d2as = cconj(cscale(f.s3, 2.0 * t2));
   const cplx<double> dal = cconj(cscale(f.a1, t2 / (f.hl * f.hl)));
   const cplx<double> d2al = cconj(cscale(f.a2, t2 / (f.hl * f.hl * f.hl)));
-  const double dsz = d_alpha_smooth_dz_(z, P.kstar, P.rect, corner, P.approx);
-  const cplx<double> dszb = d_alpha_smooth_dzbar_(z, P.kstar, P.rect, corner, P.approx, P.taylor_smooth, P.inv_pi);
-  const cplx<double> d2szb = d2_alpha_smooth_dzbar2_(z, P.kstar, P.rect, corner, P.approx, P.taylor_smooth, P.inv_pi);
+  const int rect = SERIES ? 1 : P.rect, approx = SERIES ? 1 : P.approx;
+  const double dsz = d_alpha_smooth_dz_(z, P.kstar, rect, corner, approx);
+  const cplx<double> dszb = d_alpha_smooth_dzbar_(z, P.kstar, rect, corner, approx, P.taylor_smooth, P.inv_pi, series);
+  const cplx<double> d2szb =
+      d2_alpha_smooth_dzbar2_(z, P.kstar, rect, corner, approx, P.taylor_smooth, P.inv_pi, series);
   CcfDerivs d;
   d.dwdz = 1.0 - P.kappa - dsz;
   d.dwdzb = csub(csub(csub(mk(P.gamma, 0.0), das), dal), dszb);
@@ -238,16 +244,16 @@ __global__ void ccf_phases(CcfParams P, double2* __restrict__ cs) {
 // and over the chain's other roots (strided, so a warp reads 32 consecutive
 // positions at a time) and reduce them in a fixed order. Returns whether the
 // root is final; zn (lane 0) is its new position.
-template <typename T>
+template <typename T, bool SERIES>
 __device__ __forceinline__ bool ccf_update(const CcfParams& P, const LeafPtrs& lp, const DescentPtrs<T>& dp,
                                            const StarRec<T>* __restrict__ stars, const double2* spos,
-                                           const double2* src, int a, double2 cs, double theta, int lane, int& node,
-                                           double2& out) {
+                                           const double2* src, int a, double2 cs, double theta,
+                                           const SmoothSeries<double>* series, int lane, int& node, double2& out) {
   const double2 z2 = src[a];
   const cplx<double> z = mk(z2.x, z2.y);
   out = z2;
   const CcfField f = ccf_field_warp(P, lp, dp, stars, z, lane, node);
-  const CcfDerivs d = ccf_derivs(P, f, z);
+  const CcfDerivs d = ccf_derivs<SERIES>(P, f, z, series);
   const cplx<double> f0 = csub(cconj(d.dwdzb), mk(d.dwdz * cs.x, -d.dwdz * cs.y));  // ccf_f0
   if (ccf_inv_mu_bound(cabs_(f0), d.dwdz) < 1e-9) return true;  // already a root to the precision sought
   const cplx<double> f1 = cconj(d.d2wdzb2);  // d f0 / dz
@@ -289,8 +295,16 @@ __host__ __device__ __forceinline__ long long ccf_spins(const CcfParams& P) {
 // root finding of 137 / 1000 stars took 4.6 / 13.0 ms (B200) besides 3 - 5 ms
 // to capture and instantiate the graphs; as this launch 2.5 / 12.4 ms with every
 // descent, general divisions and four reciprocals in flight, now 2.1 / 7.0 ms.
+//
+// SERIES (the approximate sheet of a rectangle): the coefficients of the sheet's
+// series are formed once per CTA. Formed at every update, a sine, a cosine and two
+// divisions for each of 26 terms in a chain, they held up an update so long that
+// two roots per warp (400 stars, two branches, 40 phi steps) took 4.64 ms against
+// 3.67 in separate launches; now 1.47, and 8.6 -> 3.5 for 1000 stars and four
+// branches. The other sheets keep the general form: without the series' code the
+// compiler's order of the reciprocal sums was slower (1000 stars 3.75, 3.90).
 constexpr int kCcfShared = 4096;  // star positions held in shared memory (64 KB)
-template <typename T>
+template <typename T, bool SERIES>
 __global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs lp, DescentPtrs<T> dp,
                                                           const StarRec<T>* __restrict__ stars,
                                                           const double2* __restrict__ spos,
@@ -299,6 +313,15 @@ __global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs 
                                                           unsigned char* fin, int* nodes, unsigned long long* words,
                                                           int* err, int centres, double2** last) {
   extern __shared__ double2 s_pos[];
+  __shared__ SmoothSeries<double> s_series;
+  if (SERIES) {  // taylor_smooth is odd and at most kMaxTaylorSmooth
+    const double ph = carg(mk(P.corner_re, P.corner_im));
+    for (int k = threadIdx.x + 1; 2 * k < P.taylor_smooth && k < kSeriesTerms; k += kCcfThreads) {
+      s_series.c2[k] = smooth_series_term(ph, 2 * k);
+      s_series.c1[k] = cdivr(s_series.c2[k], double(2 * k));
+    }
+    __syncthreads();
+  }
   const bool shared = P.nstars <= kCcfShared;
   if (shared) {
     for (int i = threadIdx.x; i < P.nstars; i += kCcfThreads) s_pos[i] = spos[i];
@@ -333,8 +356,8 @@ __global__ void __launch_bounds__(kCcfThreads) ccf_follow(CcfParams P, LeafPtrs 
         bool done = true;
         if (state == 0) {
           int node = i == 0 && j <= 1 ? -1 : nodes[q];
-          done = ccf_update<T>(P, lp, dp, stars, pos, src, a, cs[(j == 0 ? 2 * c : ch) * (half + 1) + j], theta, lane,
-                               node, z);
+          done = ccf_update<T, SERIES>(P, lp, dp, stars, pos, src, a, cs[(j == 0 ? 2 * c : ch) * (half + 1) + j], theta,
+                               SERIES ? &s_series : nullptr, lane, node, z);
           if (lane == 0) nodes[q] = node;
         }
         done = __shfl_sync(0xffffffffu, int(done), 0) != 0;

@@ -250,10 +250,11 @@ class CCF {
     // a warp per root, as many CTAs as can be resident together (the grid
     // waits for one another at every update)
     const size_t smem = n <= kCcfShared ? n * sizeof(double2) : 0;
-    IRSB_CKR(cudaFuncSetAttribute(ccf_follow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCcfShared * sizeof(double2))));
+    const auto kernel = rectangular && approx ? ccf_follow<T, true> : ccf_follow<T, false>;
+    IRSB_CKR(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCcfShared * sizeof(double2))));
     auto follow = [&](int centres, int chains, unsigned long long* w) -> bool {
       int grid = 0;
-      if (!cooperative_grid(ccf_follow<T>, kCcfThreads, ceil_div((long long)chains * num_roots, kCcfThreads / 32), &grid,
+      if (!cooperative_grid(kernel, kCcfThreads, ceil_div((long long)chains * num_roots, kCcfThreads / 32), &grid,
                             smem))
         return false;
       CcfParams q = Q;
@@ -266,7 +267,7 @@ class CCF {
       unsigned char* fi = d_fin_.p;
       int* no = d_nodes_.p;
       void* args[] = {&q, &l, &d, &st, &sp, &ph, &i0, &i1, &ro, &s0, &s1, &fi, &no, &w, &err, &centres, &last};
-      return IRSB_CK(cudaLaunchCooperativeKernel((const void*)ccf_follow<T>, dim3(grid), dim3(kCcfThreads), args, smem, s));
+      return IRSB_CK(cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(kCcfThreads), args, smem, s));
     };
     // branch centres (include/ccf.cuh:906-977), then the steps away from them (:979-1037)
     IRSB_CKR(cudaEventRecord(e0_, s));

@@ -8,6 +8,7 @@
 // conj(z)/corner of the exact four-logarithm expression.
 #pragma once
 #include "common.cuh"
+#include "params.hpp"
 
 namespace irsb {
 
@@ -74,8 +75,23 @@ IRSB_HD T d_alpha_smooth_dz_(cplx<T> z, T ks, int rect, cplx<T> c, int approx) {
   return -ks * heaviside_(cabs_(c) - cabs_(z));
 }
 
+// Coefficients of the derivatives' series (approximate sheet of a rectangle),
+// 1 - e^{2 i ph k} for k = 2, 4, ..., ts - 1 and the same over k; entry k / 2.
+constexpr int kSeriesTerms = kMaxTaylorSmooth / 2 + 2;
 template <typename T>
-IRSB_HD cplx<T> d_alpha_smooth_dzbar_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi) {
+struct SmoothSeries {
+  cplx<T> c2[kSeriesTerms], c1[kSeriesTerms];
+};
+template <typename T>
+IRSB_HD cplx<T> smooth_series_term(T ph, int i) {
+  cplx<T> e = cexp_(mk<T>(0, 2 * ph * i));
+  return mk<T>(1 - e.re, -e.im);
+}
+
+// series: those coefficients where the caller holds them (nullptr: formed here)
+template <typename T>
+IRSB_HD cplx<T> d_alpha_smooth_dzbar_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi,
+                                      const SmoothSeries<T>* series = nullptr) {
   cplx<T> d = mk<T>(0, 0);
   if (rect) {
     if (approx) {
@@ -83,8 +99,7 @@ IRSB_HD cplx<T> d_alpha_smooth_dzbar_(cplx<T> z, T ks, int rect, cplx<T> c, int 
       cplx<T> r2 = cmul(r, r);
       T ph = carg(c);
       for (int i = ts - 1; i >= 2; i -= 2) {
-        cplx<T> e = cexp_(mk<T>(0, 2 * ph * i));
-        d = cadd(d, cdivr(mk<T>(1 - e.re, -e.im), T(i)));
+        d = cadd(d, series ? series->c1[i / 2] : cdivr(smooth_series_term(ph, i), T(i)));
         d = cmul(d, r2);
       }
       d = cscale(d, T(2));
@@ -106,7 +121,8 @@ IRSB_HD cplx<T> d_alpha_smooth_dzbar_(cplx<T> z, T ks, int rect, cplx<T> c, int 
 }
 
 template <typename T>
-IRSB_HD cplx<T> d2_alpha_smooth_dzbar2_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi) {
+IRSB_HD cplx<T> d2_alpha_smooth_dzbar2_(cplx<T> z, T ks, int rect, cplx<T> c, int approx, int ts, T inv_pi,
+                                        const SmoothSeries<T>* series = nullptr) {
   cplx<T> d = mk<T>(0, 0);
   cplx<T> zb = cconj(z);
   if (rect) {
@@ -115,8 +131,7 @@ IRSB_HD cplx<T> d2_alpha_smooth_dzbar2_(cplx<T> z, T ks, int rect, cplx<T> c, in
       cplx<T> r2 = cmul(r, r);
       T ph = carg(c);
       for (int i = ts - 1; i >= 2; i -= 2) {
-        cplx<T> e = cexp_(mk<T>(0, 2 * ph * i));
-        d = cadd(d, mk<T>(1 - e.re, -e.im));
+        d = cadd(d, series ? series->c2[i / 2] : smooth_series_term(ph, i));
         d = cmul(d, r2);
       }
       d = cdiv(d, zb);
