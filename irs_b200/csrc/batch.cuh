@@ -694,7 +694,7 @@ class BatchMaker {
 
   bool check(int* st) {
     if (!tree_status(tree_, kTreeOff, stream_)) return false;
-    const int* h = tree_.h_status.data();
+    const int* h = tree_.h_status.p;
     if (h[kTreeBarrier]) {
       std::cerr << "Error. The batch's tree build or expansions did not finish.\n";
       return false;

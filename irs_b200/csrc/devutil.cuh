@@ -3,6 +3,8 @@
 #include "common.cuh"
 
 #include <atomic>
+#include <cstdio>
+#include <cstdlib>
 #include <vector>
 
 namespace irsb {
@@ -95,6 +97,57 @@ struct HostVec {
     pinned_bytes() += (long long)(n * sizeof(T));
     return true;
   }
+};
+
+// Host memory that transfers fill, on pages of its own so that it can be pinned
+// in place. Pinned memory makes a transfer faster but takes long to get
+// (pinned_bytes), so this one starts pageable and is pinned when it has been used
+// pin_after times: the owner sets that to about what getting it costs over what a
+// use gains, so that an object that runs once never pays for it and one that runs
+// often pays about twice at most.
+template <typename T>
+struct HostBuf {
+  T* p = nullptr;
+  HostBuf() = default;
+  HostBuf(const HostBuf&) = delete;
+  HostBuf& operator=(const HostBuf&) = delete;
+  ~HostBuf() { release(); }
+  void release() {
+    if (pinned_) {
+      cudaHostUnregister(p);
+      pinned_bytes() -= (long long)bytes_;
+    }
+    std::free(p);
+    p = nullptr;
+    bytes_ = 0;
+    uses_ = 0;
+    pinned_ = false;
+  }
+  // Room for want values, to be filled once; contents kept only where it suffices.
+  bool prepare(size_t want, long long pin_after) {
+    constexpr size_t kPage = 4096;
+    if (want * sizeof(T) > bytes_) {
+      release();
+      const size_t room = (want * sizeof(T) + kPage - 1) / kPage * kPage;
+      p = static_cast<T*>(std::aligned_alloc(kPage, room));
+      if (!p) {
+        std::fprintf(stderr, "Error. No host memory for %zu bytes.\n", room);
+        return false;
+      }
+      bytes_ = room;
+    } else if (uses_ == pin_after) {
+      pinned_ = cudaHostRegister(p, bytes_, cudaHostRegisterDefault) == cudaSuccess;
+      if (pinned_) pinned_bytes() += (long long)bytes_;
+      else cudaGetLastError();  // stays pageable
+    }
+    uses_++;
+    return true;
+  }
+
+ private:
+  size_t bytes_ = 0;
+  long long uses_ = 0;
+  bool pinned_ = false;
 };
 
 // ---------------------------------------------------------------- grid barrier

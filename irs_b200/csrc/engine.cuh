@@ -548,6 +548,7 @@ class MapMaker {
   DevVec<unsigned long long> d_red_;
   static constexpr int kMaxRanges = 3;
   DevVec<long long> d_mm_;
+  HostBuf<long long> h_mm_;
 
   bool init_stream() {
     if (stream_) return true;
@@ -731,9 +732,8 @@ class MapMaker {
   bool value_ranges(const V* const* maps, int nmaps, long long n, V* lo, V* hi) {
     using K = typename OrderedKey<V>::K;
     static_assert(sizeof(K) <= sizeof(long long), "keys fit the buffers");
-    if (!d_mm_.alloc_exact(2 * kMaxRanges)) return false;
-    K* dm = reinterpret_cast<K*>(d_mm_.p);
-    K hm[2 * kMaxRanges];
+    if (!d_mm_.alloc_exact(2 * kMaxRanges) || !h_mm_.prepare(2 * kMaxRanges, kStatusPinAfter)) return false;
+    K *dm = reinterpret_cast<K*>(d_mm_.p), *hm = reinterpret_cast<K*>(h_mm_.p);
     for (int i = 0; i < nmaps; i++) {
       hm[2 * i] = std::numeric_limits<K>::max();
       hm[2 * i + 1] = std::numeric_limits<K>::min();

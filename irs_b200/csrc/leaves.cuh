@@ -107,7 +107,7 @@ unsigned long long* lattice_stat(const TreeDev<T>& t) {
 template <typename T>
 unsigned long long lattice_count(const TreeDev<T>& t, LatticeStat k) {
   unsigned long long v;
-  std::memcpy(&v, t.h_status.data() + kTreeLattice + 2 * k, sizeof(v));
+  std::memcpy(&v, t.h_status.p + kTreeLattice + 2 * k, sizeof(v));
   return v;
 }
 
@@ -381,11 +381,11 @@ bool build_leaves(LeafSet& L, TreeDev<T>& t, FmmDev& f, const StarRec<T>* stars,
 // status on the host, tree_status).
 template <typename T>
 bool leaves_ok(const TreeDev<T>& t) {
-  if (t.h_status[kTreeBarrier]) {
+  if (t.h_status.p[kTreeBarrier]) {
     std::fprintf(stderr, "Error. The expansions did not finish.\n");
     return false;
   }
-  if (t.h_status[kTreeNear]) {
+  if (t.h_status.p[kTreeNear]) {
     std::fprintf(stderr, "Error. A leaf's near field holds more than %d stars.\n", kMaxStarsDirect);
     return false;
   }

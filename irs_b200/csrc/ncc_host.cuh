@@ -8,7 +8,6 @@
 #include "post.cuh"
 
 #include <algorithm>
-#include <cstdlib>
 #include <filesystem>
 #include <fstream>
 #include <iostream>
@@ -16,64 +15,6 @@
 #include <vector>
 
 namespace irsb {
-
-// Host memory of the map and of a few words of status behind it, on pages of
-// its own so that it can be pinned in place. Pinned memory makes the transfers
-// faster but takes long to get, also for a few bytes (B200, first run of a new
-// object, pinned against pageable: 100^2 pixels 2.4 / 0.53 ms, 1000^2 7.9 / 4.5;
-// repeated runs 0.10 / 0.11 and 0.63 / 0.90). Pinning memory that is there takes
-// 0.33 ms (100^2) and 2 - 4 ms (1000^2), what about 10 to 30 runs gain by it. So
-// it is pinned when it has been filled kPinAfter times: an object that runs once
-// never pays for it, one that runs often about twice at most.
-struct HostMap {
-  static constexpr int kWords = 3;
-  int *p = nullptr, *words = nullptr;
-  size_t n = 0;
-  HostMap() = default;
-  HostMap(const HostMap&) = delete;
-  HostMap& operator=(const HostMap&) = delete;
-  ~HostMap() { release(); }
-  void release() {
-    if (pinned_) {
-      cudaHostUnregister(p);
-      pinned_bytes() -= bytes();
-    }
-    std::free(p);
-    p = words = nullptr;
-    n = cap_ = 0;
-    fills_ = 0;
-    pinned_ = false;
-  }
-  // Room for want values, to be filled once; contents kept only where it suffices.
-  bool prepare(size_t want) {
-    if (want > cap_) {
-      release();
-      const size_t room = ((want + kWords) * sizeof(int) + kPage - 1) / kPage * kPage;
-      p = static_cast<int*>(std::aligned_alloc(kPage, room));
-      if (!p) {
-        std::cerr << "Error. No host memory for the map.\n";
-        return false;
-      }
-      cap_ = room / sizeof(int) - kWords;
-      words = p + cap_;
-    } else if (fills_ == kPinAfter) {
-      pinned_ = cudaHostRegister(p, size_t(bytes()), cudaHostRegisterDefault) == cudaSuccess;
-      if (pinned_) pinned_bytes() += bytes();
-      else cudaGetLastError();  // stays pageable
-    }
-    fills_++;
-    n = want;
-    return true;
-  }
-
- private:
-  static constexpr size_t kPage = 4096;
-  static constexpr long long kPinAfter = 16;
-  size_t cap_ = 0;
-  long long fills_ = 0;
-  bool pinned_ = false;
-  long long bytes() const { return (long long)((cap_ + kWords) * sizeof(int)); }
-};
 
 template <typename T>
 class NCC {
@@ -96,7 +37,8 @@ class NCC {
   double t_ncc = 0, t_reduce = 0;
   int num_rows = 0, num_cols = 0, min_num = 0, max_num = 0, errors = 0;
   std::vector<int> histogram;
-  HostMap map;
+  HostBuf<int> map;  // the map, then three words of status
+  long long map_size = 0;  // values of the map
 
   ~NCC() {
     for (cudaEvent_t* e : {&e0_, &e1_, &e2_})
@@ -153,10 +95,11 @@ class NCC {
     const bool pooled = B <= 8;  // the fine map is not stored
     if (!d_caus_.alloc_exact(caus.size()) || !d_diff_.alloc_exact(ndiff) ||
         (!pooled && !d_fine_.alloc_exact(fx * fy)) || !d_out_.alloc_exact(nout) || !d_stat_.alloc_exact(3) ||
-        !map.prepare(nout))
+        !map.prepare(nout + 3, kPinAfter))
       return false;
+    map_size = nout;
     IRSB_CKR(cudaMemsetAsync(d_diff_.p, 0, ndiff * sizeof(int), s));
-    int* stat = map.words;
+    int* stat = map.p + nout;
     stat[0] = 0;  // errors, smallest, largest value
     stat[1] = std::numeric_limits<int>::max();
     stat[2] = std::numeric_limits<int>::min();
@@ -265,7 +208,7 @@ class NCC {
       const int nr = num_pixels_y.im, nc = num_pixels_y.re;
       m.write(reinterpret_cast<const char*>(&nr), sizeof(int));
       m.write(reinterpret_cast<const char*>(&nc), sizeof(int));
-      m.write(reinterpret_cast<const char*>(map.p), map.n * sizeof(int));
+      m.write(reinterpret_cast<const char*>(map.p), map_size * sizeof(int));
       if (!m) return false;
     }
     if (verbose >= 1) std::cout << "Done writing NCC files with prefix " << outfile_prefix << "\n";
@@ -278,6 +221,11 @@ class NCC {
   // in transfer. Repeated runs (B200, host / device): 8^2 pixels 0.067 / 0.086 ms,
   // 64^2 0.087 / 0.098, 100^2 0.105 / 0.105, 180^2 0.143 / 0.122.
   static constexpr long long kSmallMap = 8192;
+  // Runs of the map's memory before it is pinned (HostBuf). First run of a new
+  // object, pinned against pageable (B200): 100^2 pixels 2.4 / 0.53 ms, 1000^2
+  // 7.9 / 4.9; repeated runs 0.10 / 0.11 and 0.63 / 0.90. Pinning in place takes
+  // 0.33 ms (100^2) and 2 - 4 ms (1000^2), what about 10 to 30 runs gain by it.
+  static constexpr long long kPinAfter = 16;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr, e2_ = nullptr;
   DevVec<double2> d_caus_;

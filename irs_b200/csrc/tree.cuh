@@ -53,7 +53,7 @@ struct TreeDev {
   DevVec<int> status;       // TreeStatus, then the level offsets (the FMM reads them there)
   DevVec<unsigned long long> words;  // grid barriers of the build and of the expansions
   DevVec<StarRec<T>> tmp_stars, star_backup;
-  std::vector<int> h_status;  // copy of `status`
+  HostBuf<int> h_status;      // copy of `status`
   long long launches = 0;   // kernels the last build launched
 };
 
@@ -647,13 +647,14 @@ bool tree_build_reserve(TreeDev<T>& t, int nstars, int cap, cudaStream_t s) {
          t.words.reserve(kTreeBarriers + kFmmBarriers, s) && t.tmp_stars.reserve(nstars, s);
 }
 
-// The first n status words to the host, once the work queued on s is done (the
-// copy goes to pageable memory, so the call waits for it; pinning these few words
-// took 0.5 - 1 ms of every new object's first run).
+// The first n status words to the host, once the work queued on s is done. Pinning
+// these words took 0.5 - 1 ms of every new object's first run; it gains 2 us of each
+// of a run's two copies (HostBuf).
+constexpr long long kStatusPinAfter = 128;
 template <typename T>
 bool tree_status(TreeDev<T>& t, int n, cudaStream_t s) {
-  t.h_status.resize(kTreeStatusWords);
-  IRSB_CKR(cudaMemcpyAsync(t.h_status.data(), t.status.p, n * sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (!t.h_status.prepare(kTreeStatusWords, kStatusPinAfter)) return false;
+  IRSB_CKR(cudaMemcpyAsync(t.h_status.p, t.status.p, n * sizeof(int), cudaMemcpyDeviceToHost, s));
   return IRSB_CK(cudaStreamSynchronize(s));
 }
 
@@ -686,7 +687,7 @@ bool build_tree(TreeDev<T>& t, StarRec<T>* stars, int nstars, T root_hl, DevVec<
     t.launches++;
     if (!before_sync(cap)) return false;
     if (!tree_status(t, kTreeStatusWords, s)) return false;
-    const int* st = t.h_status.data();
+    const int* st = t.h_status.p;
     const int err = st[kTreeErr];
     if (st[kTreeBarrier]) {
       std::fprintf(stderr, "Error. The tree build did not finish.\n");

@@ -291,3 +291,20 @@ def test_new_objects_take_no_pinned_memory_for_their_status(gpu):
     assert pinned(lambda: irs_b200.AdaptiveIPM(**ipm)) == 0
     assert pinned(lambda: irs_b200.IPM(**ipm)) == 4 * 32 * 24
     assert pinned(lambda: irs_b200.IRS(**irs)) == 4 * 32 * 24
+
+
+def test_status_words_of_an_object_that_runs_often_are_pinned(gpu):
+    """They are fetched twice a run and pinned, one page, after 128 fetches; the
+    map stays the same."""
+    import gc
+    gc.collect()
+    m = irs_b200.IPM(**dict(IPM_SMALL, num_pixels_y1=32, num_pixels_y2=24))
+    m.run()
+    first, held = m.magnifications.copy(), m.value("pinned_bytes")
+    for _ in range(63):
+        m.run()
+    assert m.value("pinned_bytes") == held
+    m.run()
+    assert m.value("pinned_bytes") == held + 4096
+    np.testing.assert_array_equal(m.magnifications, first)
+    m.close()
